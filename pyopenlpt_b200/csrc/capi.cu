@@ -152,6 +152,7 @@ OtfView otf_view(olpt_ctx* ctx) {
     v.bmin[k] = ctx->otf.bmin[k];
     v.bmax[k] = ctx->otf.bmax[k];
     v.d[k] = ctx->otf.d[k];
+    v.inv_d[k] = 1.0 / v.d[k];
   }
   v.table = ctx->otf_table.as<double>();
   v.alpha_zero = ctx->otf.alpha_zero;
@@ -454,8 +455,14 @@ olpt_status_t olpt_otf_upload(olpt_ctx* ctx, int nx, int ny, int nz, const doubl
       std::memcpy(&bits, alpha + i, sizeof(bits));
       if (bits != 0) o.alpha_zero = 0;
     }
+    // the device table holds a node's four values side by side (OtfView::table)
+    const size_t nodes = (size_t)ctx->n_cam * o.n_grid;
+    std::vector<double> inter(4 * nodes);
+    for (size_t q = 0; q < 4; ++q)
+      for (size_t i = 0; i < nodes; ++i) inter[4 * i + q] = abca[q * nodes + i];
     ctx->otf_table.ensure(bytes, ctx->stream);
-    OLPT_CUDA(cudaMemcpyAsync(ctx->otf_table.p, abca, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    OLPT_CUDA(cudaMemcpyAsync(ctx->otf_table.p, inter.data(), bytes, cudaMemcpyHostToDevice,
+                              ctx->stream));
     OLPT_CUDA(cudaStreamSynchronize(ctx->stream));
   });
 }

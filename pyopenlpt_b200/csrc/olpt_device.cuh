@@ -47,11 +47,13 @@ struct Line3 {
 
 // ---------------------------------------------------------------- pinhole
 // Camera::distort (Camera.cpp:913-966), returns pixel coordinates.
-__device__ __forceinline__ void cam_distort(const CamDev& c, double x, double y, double& pu,
+// Cam: CamDev, or another holder of the same members.
+template <class Cam>
+__device__ __forceinline__ void cam_distort(const Cam& c, double x, double y, double& pu,
                                             double& pv) {
   double xd, yd;
   if (c.is_distorted) {
-    const double* k = c.dist;
+    const auto& k = c.dist;
     double r2 = x * x + y * y;
     double r4 = r2 * r2;
     double r6 = r4 * r2;
@@ -77,7 +79,8 @@ __device__ __forceinline__ void cam_distort(const CamDev& c, double x, double y,
 }
 
 // Camera::worldToUndistImg + distort (Camera.cpp:648-690, 913-966).
-__device__ __forceinline__ void pinhole_project(const CamDev& c, double X, double Y, double Z,
+template <class Cam>
+__device__ __forceinline__ void pinhole_project(const Cam& c, double X, double Y, double Z,
                                                 double& u, double& v) {
   // Matrix<double>::operator* accumulates from 0 in column order (Matrix.hpp:392-406),
   // then operator+ adds T elementwise.
@@ -344,7 +347,7 @@ __device__ __forceinline__ void los_to_line2d(const CamDev& c, const Line3& L, d
 // ---------------------------------------------------------------- triangulation
 // myMATH::internal::gaussForward/gaussBackward (myMATH.h:183-289) for n = 3,
 // returning inverse(A) (gaussInverse, myMATH.h:291-301).
-__device__ __forceinline__ void gauss_inverse3(const double A[9], double R[9]) {
+__host__ __device__ __forceinline__ void gauss_inverse3(const double A[9], double R[9]) {
   // Rows move physically instead of through an index permutation (same operations on
   // the same values, so the same result), which keeps every array in registers.
   double r[3][3], mr[3];

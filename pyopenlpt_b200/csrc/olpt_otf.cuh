@@ -9,7 +9,10 @@ namespace olpt {
 struct OtfView {
   int nx, ny, nz, n_grid, n_cam;
   double bmin[3], bmax[3], d[3];
-  const double* table;  // [4][n_cam][n_grid]
+  double inv_d[3];  // 1 / d
+  // [n_cam][n_grid][4]: a, b, c, alpha of a node side by side, so that the two nodes of a
+  // cell along z are one run of 64 bytes
+  const double* table;
   // every alpha entry is +0.0: the interpolated angle is then +0.0 and its cosine and
   // sine are exactly 1 and +0 (the reference's values), so they are not evaluated
   int alpha_zero;
@@ -35,33 +38,45 @@ __device__ __forceinline__ void otf_param(const OtfView& o, int cam, double X, d
   int id[3];
   for (int k = 0; k < 3; ++k) {
     p[k] = fmin(fmax(P[k], o.bmin[k]), o.bmax[k]);
-    int i = (int)floor((p[k] - o.bmin[k]) / o.d[k]);
+    const double off = p[k] - o.bmin[k];
+    // the cell floor(off / d): off * (1 / d) is within a few ulp of the quotient, so only a
+    // product next to an integer needs the division
+    double q = off * o.inv_d[k];
+    if (!(fabs(q - rint(q)) > 1e-9 * (1.0 + fabs(q)))) q = off / o.d[k];
+    int i = (int)floor(q);
     i = i < 0 ? 0 : i;
     i = i > n[k] - 2 ? n[k] - 2 : i;
     id[k] = i;
-    const double delta = (o.bmax[k] - o.bmin[k]) / (n[k] - 1);
-    lo[k] = o.bmin[k] + delta * i;
-    hi[k] = o.bmin[k] + delta * (i + 1);
+    lo[k] = o.bmin[k] + o.d[k] * i;  // d = (bmax - bmin) / (n - 1): the nodes' spacing
+    hi[k] = o.bmin[k] + o.d[k] * (i + 1);
   }
   double t[3];
   for (int k = 0; k < 3; ++k) {
     double v = (p[k] - lo[k]) / (hi[k] - lo[k]);
     t[k] = fmax(0.0, fmin(1.0, v));
   }
+  // corners in the order of otf_lerp8 (OTF.cpp:312-317)
   const int nyz = o.ny * o.nz;
-  const int x0 = id[0], y0 = id[1], z0 = id[2];
-  const int g[8] = {x0 * nyz + y0 * o.nz + z0,             x0 * nyz + nyz + y0 * o.nz + z0,
-                    x0 * nyz + nyz + y0 * o.nz + z0 + 1,   x0 * nyz + y0 * o.nz + z0 + 1,
-                    x0 * nyz + (y0 + 1) * o.nz + z0,       x0 * nyz + nyz + (y0 + 1) * o.nz + z0,
-                    x0 * nyz + nyz + (y0 + 1) * o.nz + z0 + 1, x0 * nyz + (y0 + 1) * o.nz + z0 + 1};
-  double res[4];
-  const int nq = o.alpha_zero ? 3 : 4;
-  for (int q = 0; q < nq; ++q) {
-    const double* tab = o.table + ((size_t)q * o.n_cam + cam) * o.n_grid;
-    double v[8];
-    for (int k = 0; k < 8; ++k) v[k] = tab[g[k]];
-    res[q] = otf_lerp8(v, t[0], t[1], t[2]);
+  const double* base =
+      o.table + 4 * ((int64_t)cam * o.n_grid + (id[0] * nyz + id[1] * o.nz + id[2]));
+  double c[4][8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    // c000, c100, c101, c001, c010, c110, c111, c011
+    constexpr int X[8] = {0, 1, 1, 0, 0, 1, 1, 0}, Y[8] = {0, 0, 0, 0, 1, 1, 1, 1},
+                  Z[8] = {0, 0, 1, 1, 0, 0, 1, 1};
+    const double2* n2 =
+        reinterpret_cast<const double2*>(base + 4 * (X[k] * nyz + Y[k] * o.nz + Z[k]));
+    const double2 ab = n2[0], ca = n2[1];
+    c[0][k] = ab.x;
+    c[1][k] = ab.y;
+    c[2][k] = ca.x;
+    c[3][k] = ca.y;
   }
+  double res[4];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) res[q] = otf_lerp8(c[q], t[0], t[1], t[2]);
+  if (!o.alpha_zero) res[3] = otf_lerp8(c[3], t[0], t[1], t[2]);
   out[0] = res[0];
   out[1] = res[1];
   out[2] = res[2];

@@ -37,7 +37,10 @@ struct ShakeView {
   int n_tiles;
   PlaneView orig[OLPT_MAX_CAM];  // current images (u8/u16/f32/f64)
   PlaneView res[OLPT_MAX_CAM];   // residual planes (Real)
-  size_t smem_per_warp, off_dd, off_otf, off_uv;
+  int n_poly;            // most terms of a polynomial camera with exponents 0..3
+  double fit3[2][3];     // linear and quadratic rows of the three-point parabola fit
+  // shared memory of the shake kernel: the cameras' table, then the objects' arrays
+  size_t cam_bytes, obj_stride, off_dd, off_uv, off_roi, off_ey, off_otf, off_win, off_pw;
 };
 
 }  // namespace olpt
