@@ -148,11 +148,8 @@ struct ShakeWork {
 
 // Device workspace of stereo matching (grown on demand, reused across frames).
 struct StereoWork {
-  DevBuf cell_start[OLPT_MAX_CAM], cell_cursor[OLPT_MAX_CAM], cell_items[OLPT_MAX_CAM];
-  DevBuf cell_of[OLPT_MAX_CAM], los[OLPT_MAX_CAM];
-  DevBuf l2d[OLPT_MAX_CAM * OLPT_MAX_CAM];
-  DevBuf cxy[OLPT_MAX_CAM], cbp[OLPT_MAX_CAM * OLPT_MAX_CAM];
-  DevBuf l2d_ptrs, cbp_ptrs, active_d, counters, scan_tmp;
+  DevBuf cell_start, cell_cnt, cell_of, pid, xy, fxy, los, l2d, fl;
+  DevBuf counters, scan_tmp;
   DevBuf path_a, path_b, term, pairs;
   DevBuf cand_ids, cand_e, cand_x;
   // near-tolerance decision log: records (olpt_near_record) and a 64-bit counter of
@@ -164,19 +161,8 @@ struct StereoWork {
   void release(cudaStream_t s) {
     near_rec.release(s);
     near_count.release(s);
-    for (int c = 0; c < OLPT_MAX_CAM; ++c) {
-      cell_start[c].release(s);
-      cell_cursor[c].release(s);
-      cell_items[c].release(s);
-      cell_of[c].release(s);
-      los[c].release(s);
-    }
-    for (auto& b : l2d) b.release(s);
-    for (auto& b : cxy) b.release(s);
-    for (auto& b : cbp) b.release(s);
-    l2d_ptrs.release(s);
-    cbp_ptrs.release(s);
-    active_d.release(s);
+    for (DevBuf* b : {&cell_start, &cell_cnt, &cell_of, &pid, &xy, &fxy, &los, &l2d, &fl, &scan_tmp})
+      b->release(s);
     counters.release(s);
     path_a.release(s);
     path_b.release(s);

@@ -78,16 +78,24 @@ __global__ void scan_add_kernel(int* out, int n, const int* sums, int n_tiles) {
 }  // namespace
 
 void exclusive_scan(const int* in, int n, int* out, DevBuf& tmp, cudaStream_t s) {
-  const int n_tiles = (n + kScanTile - 1) / kScanTile;
-  OLPT_REQUIRE(n_tiles <= kScanTile, OLPT_ERR_UNSUPPORTED, "scan longer than 16M entries");
-  tmp.ensure((n_tiles + 1) * sizeof(int), s);
-  if (n > 0) {
-    scan_tiles_kernel<<<OLPT_G(n_tiles), kScanThreads, 0, s>>>(in, n, out, tmp.as<int>());
-    scan_sums_kernel<<<OLPT_G(1), 1024, 0, s>>>(tmp.as<int>(), n_tiles);
-    scan_add_kernel<<<OLPT_G((n + 255) / 256), 256, 0, s>>>(out, n, tmp.as<int>(), n_tiles);
-  } else {
+  if (n <= 0) {
     OLPT_CUDA(cudaMemsetAsync(out, 0, sizeof(int), s));
+    return;
   }
+  const int n_tiles = (n + kScanTile - 1) / kScanTile;
+  const int n_super = (n_tiles + kScanTile - 1) / kScanTile;  // tiles of tile sums
+  tmp.ensure((size_t)(n_tiles + n_super + 2) * sizeof(int), s);
+  int* sums = tmp.as<int>();
+  scan_tiles_kernel<<<OLPT_G(n_tiles), kScanThreads, 0, s>>>(in, n, out, sums);
+  if (n_super == 1) {
+    scan_sums_kernel<<<OLPT_G(1), 1024, 0, s>>>(sums, n_tiles);
+  } else {
+    int* super = sums + n_tiles + 1;
+    scan_tiles_kernel<<<OLPT_G(n_super), kScanThreads, 0, s>>>(sums, n_tiles, sums, super);
+    scan_sums_kernel<<<OLPT_G(1), 1024, 0, s>>>(super, n_super);
+    scan_add_kernel<<<OLPT_G((n_tiles + 255) / 256), 256, 0, s>>>(sums, n_tiles, super, n_super);
+  }
+  scan_add_kernel<<<OLPT_G((n + 255) / 256), 256, 0, s>>>(out, n, sums, n_tiles);
   OLPT_CUDA(cudaGetLastError());
 }
 

@@ -6,18 +6,24 @@
 // triangulation gate (:1083-1141), camera selection (:1307-1411), check (:504-609).
 //
 // B200 mapping.
-//  * Grid: a counting sort per camera (histogram -> scan -> scatter -> per-cell
-//    ascending pid order), i.e. the reference's bucket lists as CSR arrays.
+//  * Grid: one counting sort over the detections of all cameras (histogram -> scan ->
+//    scatter), into cells of idmap_cell_px rows by a fraction of that in columns.  The
+//    detections are renumbered by it: position G holds the coordinates, the line of sight
+//    and the image lines on every camera of one detection, and a run of cells of one row is
+//    a run of positions.  The paths carry positions; the candidates get the detections' ids
+//    back at the end.
 //  * Every detection's line of sight and its image line on every other camera are
 //    computed once (same FP64 functions the reference calls on the fly, so the
 //    values are bit-identical) and reused by every path that touches the point.
 //  * The depth-first search over build cameras is expanded breadth-first: level k
 //    holds all partial paths with k chosen cameras and the target camera of their
-//    next choice.  One warp expands one path: lanes take rows of cells, replicate the
-//    reference's per-row span arithmetic exactly, visit the cells and apply the exact
-//    point-line test, back-projection test and quick triangulation gate.  Children
-//    are appended with atomics; the final candidate list is sorted by ids on the
-//    host, so append order never shows.
+//    next choice.  enum_kernel finds the detections of the target camera inside the
+//    path's strips, tri_kernel applies the back-projection test and the triangulation
+//    gate to them.  Children are appended with atomics; the final candidate list is
+//    sorted by ids, so append order never shows.
+//  * 2D tests are decided in FP32 where the distance is clear of the tolerance by more
+//    than FP32 can err, and by the reference's FP64 expressions elsewhere: the accepted set
+//    is the FP64 one.
 //  * The whole set of candidates (ids, e_check) is therefore identical to the
 //    reference's.  Decisions that pass through acos/sin (only when the minimum
 //    parallax is below 6 degrees) can differ by one ulp; those are the only
@@ -38,21 +44,25 @@ namespace olpt {
 struct SmView {
   int n_cam, m, n_active;
   int active[OLPT_MAX_CAM];
-  int cell;
-  int rows[OLPT_MAX_CAM], cols[OLPT_MAX_CAM];
+  int cell, sub;            // grid: rows of `cell` px, `sub` columns per `cell` px
+  int rows[OLPT_MAX_CAM], cols[OLPT_MAX_CAM];  // in units of `cell`
+  int cell_off[OLPT_MAX_CAM];                  // first cell of the camera in cstart
+  int raw_off[OLPT_MAX_CAM + 1];               // detections of the cameras before it
   double Wd[OLPT_MAX_CAM], Hd[OLPT_MAX_CAM];
-  const int* cell_start[OLPT_MAX_CAM];
-  const int* cell_items[OLPT_MAX_CAM];
-  const double* x[OLPT_MAX_CAM];
+  const double* x[OLPT_MAX_CAM];               // the detections as found
   const double* y[OLPT_MAX_CAM];
-  int64_t n[OLPT_MAX_CAM];
-  const double* los[OLPT_MAX_CAM];                  // n x 6
-  const double* l2d[OLPT_MAX_CAM][OLPT_MAX_CAM];    // [c][t]: n[c] x 6 (pt, unit, U)
-  // cell-ordered copies of camera t's detections (position q of cell_items[t]):
-  // their coordinates, and the first four values of their image lines on camera c
-  const double2* cxy[OLPT_MAX_CAM];
-  const double* cbp[OLPT_MAX_CAM][OLPT_MAX_CAM];    // [t][c]: n[t] x 4
+  // by position G (camera c holds raw_off[c] .. raw_off[c + 1] - 1; detections outside the
+  // image come last in their camera's range, in a cell of their own that no row reaches)
+  const int* cstart;     // first position of every cell
+  const int* pid;        // detection id in its camera's list
+  const double2* xy;
+  const float2* fxy;
+  const double* los;     // x 6: line of sight
+  const double* l2d;     // x n_cam x 6: image line on camera t (pt, unit, normalized unit)
+  const float4* fl;      // x n_cam: (n, d) of that line, |n . p + d| = distance of p from it
   double tol2d, tol3d;
+  float eps;             // FP32 error bound of a distance, without the part of |d|
+  double tq[OLPT_MAX_CAM + 1];  // quick-gate tolerance of k lines without its angle factor
   double limit[6];
   // near-tolerance log (off when near_band == 0): 2D tests whose distance lies within
   // near_band px of tol2d are appended to near_rec
@@ -74,7 +84,7 @@ struct Path {
 // and the next camera.  16 bytes for N = 2 (the 30 M first-level children of a 2048^2
 // frame) instead of the 48 of a full Path.
 template <int N>
-struct alignas(16) PathN {
+struct alignas(16) PathN {  // camera i in bits 4 i .. 4 i + 3 of cams
   int ids[N];
   unsigned cams;
   int target;
@@ -86,100 +96,271 @@ namespace {
 inline int nblk(int64_t n, int t = 256) { return (int)((n + t - 1) / t); }
 
 // ---------------------------------------------------------------- grid
-__global__ void cell_hist_kernel(const double* x, const double* y, int64_t n, int cell, int rows,
-                                 int cols, int* cell_of, int* counts) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  // IDMap::rebuild (StereoMatch.cpp:1423-1437)
-  int cx = (int)floor(x[i] / (double)cell);
-  int cy = (int)floor(y[i] / (double)cell);
-  if (cx < 0 || cy < 0 || cx >= cols || cy >= rows) {
-    cell_of[i] = -1;
-    return;
-  }
-  int c = cy * cols + cx;
-  cell_of[i] = c;
-  atomicAdd(&counts[c], 1);
+__device__ __forceinline__ int cam_of(const SmView& v, int g) {
+  int c = 0;
+#pragma unroll
+  for (int k = 1; k < OLPT_MAX_CAM; ++k)
+    if (k < v.n_cam && g >= v.raw_off[k]) c = k;
+  return c;
 }
 
-__global__ void cell_scatter_kernel(const int* cell_of, int64_t n, const int* start, int* cursor,
-                                    int* items) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// Cell of every detection (IDMap::rebuild's cell, StereoMatch.cpp:1423-1437, cut into `sub`
+// columns) and the cells' counts.
+__global__ void bin_kernel(const __grid_constant__ SmView v, int n, int* key, int* counts) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int c = cell_of[i];
-  if (c < 0) return;
-  int pos = start[c] + atomicAdd(&cursor[c], 1);
-  items[pos] = (int)i;
+  const int c = cam_of(v, i), k = i - v.raw_off[c];
+  const double x = v.x[c][k], y = v.y[c][k];
+  const int cx = (int)floor(x / (double)v.cell), cy = (int)floor(y / (double)v.cell);
+  int cell = v.rows[c] * v.cols[c] * v.sub;  // outside the image
+  if (!(cx < 0 || cy < 0 || cx >= v.cols[c] || cy >= v.rows[c])) {
+    const int f = (int)floor((x - (double)cx * v.cell) * v.sub / (double)v.cell);
+    cell = (cy * v.cols[c] + cx) * v.sub + min(max(f, 0), v.sub - 1);
+  }
+  cell += v.cell_off[c];
+  key[i] = cell;
+  atomicAdd(&counts[cell], 1);
 }
 
-// ascending pid order inside every cell (the reference pushes pids in order)
-__global__ void cell_sort_kernel(const int* start, int n_cells, int* items) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n_cells) return;
-  int b = start[c], e = start[c + 1];
-  for (int i = b + 1; i < e; ++i) {
-    int v = items[i];
-    int j = i - 1;
-    while (j >= b && items[j] > v) {
-      items[j + 1] = items[j];
-      --j;
-    }
-    items[j + 1] = v;
-  }
+// Positions: the order inside a cell is arbitrary (no result depends on it).
+__global__ void place_kernel(const __grid_constant__ SmView v, int n, const int* key, int* counts,
+                             int* pid, double2* xy, float2* fxy) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int c = cam_of(v, i), k = i - v.raw_off[c];
+  const int g = v.cstart[key[i]] + atomicSub(&counts[key[i]], 1) - 1;
+  const double x = v.x[c][k], y = v.y[c][k];
+  pid[g] = k;
+  xy[g] = make_double2(x, y);
+  fxy[g] = make_float2((float)x, (float)y);
 }
 
 // ---------------------------------------------------------------- per-detection lines
-__global__ void lines_kernel(const CamDev* cams, int c, const double* x, const double* y, int64_t n,
-                             int n_cam, const int* active, double* los, double* const* l2d) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  Line3 L;
-  cam_los(cams[c], x[i], y[i], L);
-  for (int k = 0; k < 3; ++k) {
-    los[6 * i + k] = L.p[k];
-    los[6 * i + 3 + k] = L.u[k];
+// A polynomial camera with exponents 0..3 as a block's threads evaluate it: the terms'
+// coefficients and, per term, the positions of its three factors in the thread's power list
+// 1, x, x^2, x^3, 1, y, .. (one byte each), in shared memory.  The powers of a thread's point
+// lie in shared memory too, one column a thread: indexed by the (uniform) positions they cost
+// one load each, where an indexed local array went through memory.
+constexpr int kLineThreads = 128;
+struct PolyTab {
+  double coef[6][OLPT_MAX_POLY];     // u, v, du/d0, du/d1, dv/d0, dv/d1
+  uint32_t fac[6][OLPT_MAX_POLY];
+  int same;                          // u and v share their monomials
+  double pw[12][kLineThreads];
+};
+
+__device__ void load_poly(PolyTab& T, const CamDev& m) {
+  const int n = m.n_coeff;
+  if (threadIdx.x == 0) T.same = 1;
+  __syncthreads();
+  for (int i = threadIdx.x; i < 6 * n; i += blockDim.x) {
+    const int q = i / n, k = i - q * n;
+    const double* t = q == 0   ? m.ucoef + 4 * k
+                      : q == 1 ? m.vcoef + 4 * k
+                      : q == 2 ? m.ducoef + 4 * k
+                      : q == 3 ? m.ducoef + 4 * (k + n)
+                      : q == 4 ? m.dvcoef + 4 * k
+                               : m.dvcoef + 4 * (k + n);
+    T.coef[q][k] = t[0];
+    uint32_t f = 0;
+    for (int j = 0; j < 3; ++j) f |= (uint32_t)(4 * j + (int)t[1 + j]) << (8 * j);
+    T.fac[q][k] = f;
   }
-  for (int t = 0; t < n_cam; ++t) {
-    if (t == c || !active[t]) continue;
-    double o[4];
-    los_to_line2d(cams[t], L, o);
-    double* d = l2d[t] + 6 * i;
-    d[0] = o[0];
-    d[1] = o[1];
-    d[2] = o[2];
-    d[3] = o[3];
-    // IDMap::normalized (StereoMatch.cpp:1441-1451)
-    const double n2 = o[2] * o[2] + o[3] * o[3];
-    if (n2 <= 1e-24) {
-      d[4] = 1.0;
-      d[5] = 0.0;
-    } else {
-      const double inv = 1.0 / sqrt(n2);
-      d[4] = o[2] * inv;
-      d[5] = o[3] * inv;
-    }
+  __syncthreads();
+  for (int k = threadIdx.x; k < n; k += blockDim.x)
+    if (T.fac[0][k] != T.fac[1][k] || T.fac[2][k] != T.fac[4][k] || T.fac[3][k] != T.fac[5][k])
+      T.same = 0;
+  __syncthreads();
+}
+
+__device__ __forceinline__ void set_powers(PolyTab& T, const double P[3]) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    T.pw[4 * j][threadIdx.x] = 1.0;
+    T.pw[4 * j + 1][threadIdx.x] = P[j];
+    T.pw[4 * j + 2][threadIdx.x] = poly_pow(P[j], 2.0);
+    T.pw[4 * j + 3][threadIdx.x] = poly_pow(P[j], 3.0);
   }
 }
 
-// Cell-ordered copies of camera t's detections for the enumeration's inner loop:
-// coordinates, and for every other active camera c the point and direction of the
-// detection's image line on c.
-__global__ void cell_pack_kernel(const int* items, int64_t n, const double* x, const double* y,
-                                 double2* cxy, double* const* bp_out, const double* const* l2d,
-                                 int n_cam, int t) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int pid = items[q];
-  cxy[q] = make_double2(x[pid], y[pid]);
-  for (int c = 0; c < n_cam; ++c) {
-    double* o = bp_out[c];
-    if (c == t || !o) continue;
-    const double* L = l2d[c] + 6 * (int64_t)pid;
-    o[4 * q] = L[0];
-    o[4 * q + 1] = L[1];
-    o[4 * q + 2] = L[2];
-    o[4 * q + 3] = L[3];
+// one term of polynomial q: coefficient times its three factors, in poly_project's order
+__device__ __forceinline__ double term(const PolyTab& T, int q, int i) {
+  const uint32_t f = T.fac[q][i];
+  const int x = threadIdx.x;
+  return T.coef[q][i] * T.pw[f & 255u][x] * T.pw[(f >> 8) & 255u][x] * T.pw[f >> 16][x];
+}
+// terms of two polynomials with the same monomial
+__device__ __forceinline__ void term2(const PolyTab& T, int q, int r, int i, double& a, double& b) {
+  const uint32_t f = T.fac[q][i];
+  const int x = threadIdx.x;
+  const double f0 = T.pw[f & 255u][x], f1 = T.pw[(f >> 8) & 255u][x], f2 = T.pw[f >> 16][x];
+  a = T.coef[q][i] * f0 * f1 * f2;
+  b = T.coef[r][i] * f0 * f1 * f2;
+}
+
+// poly_project at the point whose powers are set
+__device__ __forceinline__ void project_set(const PolyTab& T, int n, double& u, double& v) {
+  double su = 0, sv = 0;
+  for (int i = 0; i < n; ++i) {
+    double a, b;
+    if (T.same) {
+      term2(T, 0, 1, i, a, b);
+    } else {
+      a = term(T, 0, i);
+      b = term(T, 1, i);
+    }
+    su += a;
+    sv += b;
   }
+  u = su;
+  v = sv;
+}
+
+// poly_img_to_world on the table: the same operations in the same order
+__device__ void newton_tab(PolyTab& T, const CamDev& m, double pu, double pv, double plane,
+                           double P[3]) {
+  P[0] = P[1] = P[2] = 0.5;
+  const int rp = m.ref_plane, n = m.n_coeff;
+  if (rp == 1) P[0] = plane;
+  if (rp == 2) P[1] = plane;
+  if (rp == 3) P[2] = plane;
+  double err = 1.7976931348623157e308;
+  int iter = 0;
+  const bool same = T.same != 0;
+  while (err > 1e-5 && iter < 50) {
+    set_powers(T, P);
+    double j00 = 0, j01 = 0, j10 = 0, j11 = 0, tu = 0, tv = 0;
+    for (int i = 0; i < n; ++i) {
+      double a, b, c, d, e, f;
+      if (same) {
+        term2(T, 2, 4, i, a, c);
+        term2(T, 3, 5, i, b, d);
+        term2(T, 0, 1, i, e, f);
+      } else {
+        a = term(T, 2, i);
+        b = term(T, 3, i);
+        c = term(T, 4, i);
+        d = term(T, 5, i);
+        e = term(T, 0, i);
+        f = term(T, 1, i);
+      }
+      j00 += a;
+      j01 += b;
+      j10 += c;
+      j11 += d;
+      tu += e;
+      tv += f;
+    }
+    double det = j00 * j11 - j01 * j10;
+    if (fabs(det) < 1e-8) det = 1e-8;
+    const double i00 = j11 / det, i01 = -j01 / det, i10 = -j10 / det, i11 = j00 / det;
+    const double du = pu - tu, dv = pv - tv;
+    const double dx = i00 * du + i01 * dv;
+    const double dy = i10 * du + i11 * dv;
+    if (rp == 1) {
+      P[1] += dx;
+      P[2] += dy;
+    } else if (rp == 2) {
+      P[0] += dx;
+      P[2] += dy;
+    } else {
+      P[0] += dx;
+      P[1] += dy;
+    }
+    err = sqrt(du * du + dv * dv);
+    iter++;
+  }
+}
+
+// Lines of sight: blockIdx.y = camera, two lanes per detection (a polynomial camera inverts
+// two planes, one each).
+__global__ void __launch_bounds__(kLineThreads) los_kernel(const __grid_constant__ SmView v,
+                                                           const CamDev* cams, double* los) {
+  __shared__ PolyTab T;
+  const int c = blockIdx.y;
+  const int n = v.raw_off[c + 1] - v.raw_off[c];
+  if ((int64_t)blockIdx.x * (kLineThreads / 2) >= n) return;
+  const CamDev& m = cams[c];
+  const bool poly = m.type == CAM_POLYNOMIAL && m.pow3;
+  if (poly) load_poly(T, m);
+  const int k = blockIdx.x * (kLineThreads / 2) + (threadIdx.x >> 1), half = threadIdx.x & 1;
+  const bool ok = k < n;
+  const int g = v.raw_off[c] + (ok ? k : n - 1);
+  const double2 p = v.xy[g];
+  Line3 L;
+  if (poly) {
+    double P[3], Q[3];
+    newton_tab(T, m, p.x, p.y, m.plane[half], P);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) Q[d] = __shfl_xor_sync(0xffffffffu, P[d], 1);
+    if (half) return;
+    L.p[0] = P[0];
+    L.p[1] = P[1];
+    L.p[2] = P[2];
+    unit_vector3(P, Q, L.u);
+  } else {
+    if (half) return;
+    cam_los(m, p.x, p.y, L);
+  }
+  if (!ok) return;
+  double* o = los + 6 * (int64_t)g;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    o[d] = L.p[d];
+    o[3 + d] = L.u[d];
+  }
+}
+
+// Image lines of every detection on camera t = blockIdx.y.
+__global__ void __launch_bounds__(kLineThreads) lines_kernel(const __grid_constant__ SmView v,
+                                                             const CamDev* cams, double* l2d,
+                                                             float4* fl) {
+  __shared__ PolyTab T;
+  const int t = blockIdx.y;
+  if (!v.active[t]) return;
+  const CamDev& m = cams[t];
+  const bool poly = m.type == CAM_POLYNOMIAL && m.pow3;
+  if (poly) load_poly(T, m);
+  const int g = blockIdx.x * kLineThreads + threadIdx.x;
+  if (g >= v.raw_off[v.n_cam] || (g >= v.raw_off[t] && g < v.raw_off[t + 1])) return;
+  const double* S = v.los + 6 * (int64_t)g;
+  Line3 L;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    L.p[d] = S[d];
+    L.u[d] = S[3 + d];
+  }
+  double o[4];
+  if (poly) {  // los_to_line2d
+    double ax, ay, bx, by;
+    set_powers(T, L.p);
+    project_set(T, m.n_coeff, ax, ay);
+    const double B[3] = {L.p[0] + L.u[0], L.p[1] + L.u[1], L.p[2] + L.u[2]};
+    set_powers(T, B);
+    project_set(T, m.n_coeff, bx, by);
+    const double dx = bx - ax, dy = by - ay;
+    const double n = sqrt(dx * dx + dy * dy);
+    o[0] = ax;
+    o[1] = ay;
+    o[2] = dx / n;
+    o[3] = dy / n;
+  } else {
+    los_to_line2d(m, L, o);
+  }
+  double U0 = 1.0, U1 = 0.0;
+  // IDMap::normalized (StereoMatch.cpp:1441-1451)
+  const double n2 = o[2] * o[2] + o[3] * o[3];
+  if (!(n2 <= 1e-24)) {
+    const double inv = 1.0 / sqrt(n2);
+    U0 = o[2] * inv;
+    U1 = o[3] * inv;
+  }
+  const int64_t e = (int64_t)g * v.n_cam + t;
+  double2* d = reinterpret_cast<double2*>(l2d + 6 * e);
+  d[0] = make_double2(o[0], o[1]);
+  d[1] = make_double2(o[2], o[3]);
+  d[2] = make_double2(U0, U1);
+  fl[e] = make_float4((float)-U1, (float)U0, (float)(U1 * o[0] - U0 * o[1]), 0.0f);
 }
 
 __device__ __forceinline__ void load_line3(const double* p, Line3& L) {
@@ -238,13 +419,13 @@ __device__ double seg_len(const double* L, double W, double H) {
 // seed level: one path per reference detection with its second build camera
 __global__ void seed_kernel(const __grid_constant__ SmView v, int ref, PathN<1>* out, int* out_count,
                             int cap) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= v.n[ref]) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + v.raw_off[ref];
+  if (i >= v.raw_off[ref + 1]) return;
   int best = -1;
   double best_len = __longlong_as_double(0x7ff0000000000000LL);
   for (int cam = 0; cam < v.n_cam; ++cam) {
     if (!v.active[cam] || cam == ref) continue;
-    const double L = seg_len(v.l2d[ref][cam] + 6 * i, v.Wd[cam], v.Hd[cam]);
+    const double L = seg_len(v.l2d + 6 * ((int64_t)i * v.n_cam + cam), v.Wd[cam], v.Hd[cam]);
     if (L < best_len - 1e-9) {
       best_len = L;
       best = cam;
@@ -254,7 +435,7 @@ __global__ void seed_kernel(const __grid_constant__ SmView v, int ref, PathN<1>*
   int slot = atomicAdd(out_count, 1);
   if (slot >= cap) return;
   PathN<1> p;
-  p.ids[0] = (int)i;
+  p.ids[0] = i;
   p.cams = (unsigned)ref;
   p.target = best;
   out[slot] = p;
@@ -321,11 +502,13 @@ __device__ __forceinline__ double clamped_dot(const double a[3], const double b[
 // the smallest pairwise parallax lies inside (6, 174) degrees.
 constexpr double kCos6 = 0.99452189536827329;
 
-// A path and one of its candidates on the target camera that passed the 2D tests.
+// A path and the position of one of its candidates on the target camera: inside all strips,
+// or (kEdge) so close to a strip's border that FP64 has to decide.
 struct Pair {
   int path;
-  int pid;
+  unsigned g;
 };
+constexpr unsigned kEdge = 1u << 31;
 
 // Slot in an append buffer for every active lane, one atomic per warp.
 __device__ __forceinline__ int append_slot(int* counter) {
@@ -355,476 +538,559 @@ __device__ __noinline__ void near_append(const SmView& v, int kind, int k, int c
   v.near_rec[slot] = r;
 }
 
-// Expand one level, first half: each path has K chosen cameras; its candidates on
-// the target camera are enumerated over rows of cells and kept when they pass the
-// strip test (IDMap::visitPointsInRowSpans) and the back-projection test.  WARP: one
-// warp per path, lanes take rows (the single long strip of K = 1); otherwise one
-// thread per path (K >= 2, where the strips intersect in a few rows).
-template <int K, bool WARP>
-__global__ void __launch_bounds__(256, K == 1 ? 4 : 2) enum_kernel(const __grid_constant__ SmView v, const void* in_v, int n_in,
-                                                   Pair* pairs, int* pair_count, int pair_cap) {
-  const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int pidx = WARP ? (gtid >> 5) : gtid;
-  const int r0 = WARP ? (threadIdx.x & 31) : 0;
-  // thread-per-path levels keep every lane of a warp to the end (the items of the
-  // warp's paths are shared out over all lanes); a lane without a path has no rows
-  const bool live = pidx < n_in;
-  if (WARP && !live) return;
-  const PathN<K>* in = static_cast<const PathN<K>*>(in_v);
-  PathN<K> P{};
-  if (live) P = in[pidx];
+// The strip tests (IDMap::visitPointsInRowSpans) and back-projection tests
+// (checkBackProjection, StereoMatch.cpp:1206-1227) of position g on camera t against a
+// path's chosen points, in the reference's FP64 expressions; LOG: near-tolerance tests are
+// recorded.
+template <int K, bool LOG>
+__device__ __noinline__ bool exact_2d(const SmView& v, const PathN<K>& P, int g) {
   const int t = P.target;
-  // image lines of the chosen points on the target camera
-  double lp[K][2], lU[K][2];
-  double cpt[K][2];
-#pragma unroll
-  for (int i = 0; i < K; ++i) {
-    lp[i][0] = lp[i][1] = lU[i][0] = cpt[i][0] = cpt[i][1] = 0.0;
-    lU[i][1] = 1.0;
-    if (!live) continue;
-    const int c = P.cam(i);
-    const double* L = v.l2d[c][t] + 6 * (int64_t)P.ids[i];
-    lp[i][0] = L[0];
-    lp[i][1] = L[1];
-    lU[i][0] = L[4];
-    lU[i][1] = L[5];
-    cpt[i][0] = v.x[c][P.ids[i]];
-    cpt[i][1] = v.y[c][P.ids[i]];
-  }
-  const int rows = v.rows[t], cols = v.cols[t];
-  const double cellp = (double)v.cell;
-  const double hw = 0.5 * v.cell, hh = 0.5 * v.cell;
-  const double tol_grow = v.tol2d + 1e-6;
   const double tol2 = v.tol2d * v.tol2d;
-  const int* cstart = v.cell_start[t];
-  const int* citems = v.cell_items[t];
-  const double2* cxy = v.cxy[t];
-  const double* cbp[K];
-#pragma unroll
-  for (int i = 0; i < K; ++i) cbp[i] = live ? v.cbp[t][P.cam(i)] : nullptr;
+  const double2 q = v.xy[g];
+  bool ok = true;
+  for (int i = 0; i < K; ++i) {
+    const double* L = v.l2d + 6 * ((int64_t)P.ids[i] * v.n_cam + t);
+    const double dx = q.x - L[0], dy = q.y - L[1];
+    const double z = dy * L[4] - dx * L[5];
+    ok = ok && !(z * z > tol2);
+    if (LOG) {
+      const double m = fabs(z) - v.tol2d;
+      if (fabs(m) < v.near_band)
+        near_append(v, 0, K, t, v.pid[g], P.cam(i), v.pid[P.ids[i]], m);
+    }
+  }
+  for (int i = 0; i < K && ok; ++i) {
+    const double* L = v.l2d + 6 * ((int64_t)g * v.n_cam + P.cam(i));
+    const double2 c = v.xy[P.ids[i]];
+    const double d0 = c.x - L[0], d1 = c.y - L[1];
+    const double z = d1 * L[2] - d0 * L[3];
+    ok = !(z * z > tol2);
+    if (LOG) {
+      const double m = fabs(z) - v.tol2d;
+      if (fabs(m) < v.near_band)
+        near_append(v, 1, K, t, v.pid[g], P.cam(i), v.pid[P.ids[i]], m);
+    }
+  }
+  return ok;
+}
 
-  // Rows that can hold a non-empty span: with two or more strips, the cell-centre rows
-  // inside the y-extent of the first two strips' intersection parallelogram (plus one
-  // row each side).  Rows outside it have an empty exact span, so skipping them leaves
-  // the visited set unchanged.
-  int row_lo = 0, row_hi = live ? rows - 1 : -1;
-  if (K >= 2 && live) {
-    const double n00 = -lU[0][1], n01 = lU[0][0], n10 = -lU[1][1], n11 = lU[1][0];
-    const double d0 = -(n00 * lp[0][0] + n01 * lp[0][1]);
-    const double d1 = -(n10 * lp[1][0] + n11 * lp[1][1]);
-    const double T0 = tol_grow + fabs(n00) * hw + fabs(n01) * hh;
-    const double T1 = tol_grow + fabs(n10) * hw + fabs(n11) * hh;
-    const double det = n00 * n11 - n01 * n10;
+// The search over the reference's cells, with every test in FP64: the cell ranges of
+// IDMap::computeStripIntersection as a superset (row by row, cell centres within the strips
+// widened by a cell's extent and 0.01 px).  For the near-tolerance log, which records the
+// tests of exactly these visits, and for paths with an image line that is not finite.  Rows
+// row0, row0 + step, ...
+template <int K, bool LOG>
+__device__ __noinline__ void visit_cells(const SmView& v, const PathN<K>& P, int pidx, int row0,
+                                         int step, Pair* pairs, int* pair_count, int pair_cap) {
+  const int t = P.target;
+  const int rows = v.rows[t], cols = v.cols[t];
+  const double hw = 0.5 * v.cell, tol_grow = v.tol2d + 1e-6;
+  double n0[K], n1[K], dd[K], T[K];
+  for (int i = 0; i < K; ++i) {
+    const double* L = v.l2d + 6 * ((int64_t)P.ids[i] * v.n_cam + t);
+    n0[i] = -L[5];
+    n1[i] = L[4];
+    dd[i] = -(n0[i] * L[0] + n1[i] * L[1]);
+    T[i] = tol_grow + fabs(n0[i]) * hw + fabs(n1[i]) * hw;
+  }
+  int row_lo = 0, row_hi = rows - 1;
+  if (K >= 2) {
+    // cell-centre rows inside the y-extent of the first two strips' parallelogram
+    const double det = n0[0] * n1[K > 1 ? 1 : 0] - n1[0] * n0[K > 1 ? 1 : 0];
     if (fabs(det) > 1e-9) {
       double ymin = 1e300, ymax = -1e300;
-#pragma unroll
       for (int s0 = -1; s0 <= 1; s0 += 2)
-#pragma unroll
         for (int s1 = -1; s1 <= 1; s1 += 2) {
-          const double y = (n00 * (s1 * T1 - d1) - n10 * (s0 * T0 - d0)) / det;
+          const int b = K > 1 ? 1 : 0;
+          const double y = (n0[0] * (s1 * T[b] - dd[b]) - n0[b] * (s0 * T[0] - dd[0])) / det;
           ymin = fmin(ymin, y);
           ymax = fmax(ymax, y);
         }
       if (isfinite(ymin) && isfinite(ymax)) {
-        const double lo = floor(ymin / cellp - 0.5) - 1.0, hi = ceil(ymax / cellp - 0.5) + 1.0;
+        const double lo = floor(ymin / v.cell - 0.5) - 1.0, hi = ceil(ymax / v.cell - 0.5) + 1.0;
         row_lo = (int)fmax(0.0, fmin((double)(rows - 1), lo));
         row_hi = (int)fmax(-1.0, fmin((double)(rows - 1), hi));
       }
     }
   }
-
-  // IDMap::computeStripIntersection, one row: a cell range [xmin, xmax] (empty when
-  // xmin > xmax) that contains the reference's.  The range only selects the items that
-  // the exact FP64 tests below then decide, and every item that passes them lies in a
-  // cell of the reference's range, so any superset of that range gives the same
-  // accepted set.  It is evaluated in FP32 with the strip widened by 0.01 px and the
-  // cell bounds widened by 1e-3 cells (FP32 errors here stay below 1e-3 px), and the
-  // division by n0 folded into one reciprocal per strip.
-  float sn0[K], sn1[K], sd[K], sT[K], sinv[K];
-  bool shz[K];
-#pragma unroll
-  for (int i = 0; i < K; ++i) {
-    const double n0 = -lU[i][1], n1 = lU[i][0];
-    sn0[i] = (float)n0;
-    sn1[i] = (float)n1;
-    sd[i] = (float)(-(n0 * lp[i][0] + n1 * lp[i][1]));
-    sT[i] = (float)(tol_grow + fabs(n0) * hw + fabs(n1) * hh) + 0.01f;
-    shz[i] = fabs(n0) < 1e-12;
-    sinv[i] = shz[i] ? 0.0f : 1.0f / (float)n0;
-  }
-  const float cellf = (float)cellp, to_index_f = 1.0f / cellf;
-  auto row_span = [&](int cy, int& xmin, int& xmax) {
-    xmin = 0;
-    xmax = cols - 1;
-    const float y_c = ((float)cy + 0.5f) * cellf;
-#pragma unroll
+  const float cellf = (float)v.cell, to_index = 1.0f / cellf;
+  for (int cy = row_lo + row0; cy <= row_hi; cy += step) {
+    int xmin = 0, xmax = cols - 1;
+    const float yc = ((float)cy + 0.5f) * cellf;
     for (int i = 0; i < K; ++i) {
-      const float C = fmaf(sn1[i], y_c, sd[i]);
-      int a = 0, b = cols - 1;
-      if (shz[i]) {
-        if (fabsf(C) > sT[i]) {
+      const float C = fmaf((float)n1[i], yc, (float)dd[i]), Tf = (float)T[i] + 0.01f;
+      if (fabs(n0[i]) < 1e-12) {
+        if (fabsf(C) > Tf) {
           xmin = 1;
           xmax = 0;
         }
       } else {
-        float xl = (-sT[i] - C) * sinv[i];
-        float xr = (sT[i] - C) * sinv[i];
+        const float inv = 1.0f / (float)n0[i];
+        float xl = (-Tf - C) * inv, xr = (Tf - C) * inv;
         if (xl > xr) {
           const float s_ = xl;
           xl = xr;
           xr = s_;
         }
-        a = (int)ceilf(xl * to_index_f - 0.5f - 1e-3f);
-        b = (int)floorf(xr * to_index_f - 0.5f + 1e-3f);
-        a = a > 0 ? a : 0;
-        b = b < cols - 1 ? b : cols - 1;
-      }
-      xmin = xmin > a ? xmin : a;
-      xmax = xmax < b ? xmax : b;
-    }
-  };
-  // IDMap::visitPointsInRowSpans precise test and checkBackProjection of the item at
-  // cell-ordered position q; true when the pair passes both
-  auto item_ok = [&](int q) -> bool {
-    const double2 xy = cxy[q];
-    bool ok = true;
-    // IDMap::visitPointsInRowSpans precise test
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      const double dx = xy.x - lp[i][0], dy = xy.y - lp[i][1];
-      const double z = dy * lU[i][0] - dx * lU[i][1];
-      ok = ok && !(z * z > tol2);
-      if (v.near_band > 0.0) {
-        const double m = fabs(z) - v.tol2d;
-        if (fabs(m) < v.near_band)
-          near_append(v, 0, K, t, citems[q], P.cam(i), P.ids[i], m);
+        const int a = (int)ceilf(xl * to_index - 0.5f - 1e-3f);
+        const int b = (int)floorf(xr * to_index - 0.5f + 1e-3f);
+        xmin = max(xmin, max(a, 0));
+        xmax = min(xmax, min(b, cols - 1));
       }
     }
-    if (!ok) return false;
-    // checkBackProjection (StereoMatch.cpp:1206-1227)
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      if (!ok) break;
-      const double2 a = reinterpret_cast<const double2*>(cbp[i])[2 * q];
-      const double2 b = reinterpret_cast<const double2*>(cbp[i])[2 * q + 1];
-      const double d0 = cpt[i][0] - a.x, d1 = cpt[i][1] - a.y;
-      const double z = d1 * b.x - d0 * b.y;
-      ok = !(z * z > tol2);
-      if (v.near_band > 0.0) {
-        const double m = fabs(z) - v.tol2d;
-        if (fabs(m) < v.near_band)
-          near_append(v, 1, K, t, citems[q], P.cam(i), P.ids[i], m);
-      }
-    }
-    return ok;
-  };
-
-  if constexpr (WARP) {
-    // one warp per path: 32 rows at a time (lane = row), then the rows' item ranges
-    // flattened over the lanes (consecutive items of a row are adjacent in memory, so
-    // the loads coalesce and no lane idles on a short row)
-    for (int base = row_lo; base <= row_hi; base += 32) {
-      const int cy = base + r0;
-      int q0 = 0, cnt = 0;
-      if (cy <= row_hi) {
-        int xmin, xmax;
-        row_span(cy, xmin, xmax);
-        if (xmin <= xmax) {
-          q0 = cstart[cy * cols + xmin];
-          cnt = cstart[cy * cols + xmax + 1] - q0;
-        }
-      }
-      int incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t_ = __shfl_up_sync(0xffffffffu, incl, o);
-        if (r0 >= o) incl += t_;
-      }
-      const int excl = incl - cnt;
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      for (int k0 = 0; k0 < total; k0 += 32) {
-        const int k = k0 + r0;
-        // the row holding item k: the largest lane r with excl[r] <= k
-        int r = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-          const int e = __shfl_sync(0xffffffffu, excl, r + step);
-          if (e <= k) r += step;
-        }
-        const int qr = __shfl_sync(0xffffffffu, q0, r);
-        const int er = __shfl_sync(0xffffffffu, excl, r);
-        if (k >= total) continue;
-        const int q = qr + (k - er);
-        if (!item_ok(q)) continue;
+    if (xmin > xmax) continue;
+    const int base = v.cell_off[t] + cy * cols * v.sub;
+    const int q1 = v.cstart[base + (xmax + 1) * v.sub];
+    for (int q = v.cstart[base + xmin * v.sub]; q < q1; ++q)
+      if (exact_2d<K, LOG>(v, P, q)) {
         const int slot = append_slot(pair_count);
-        if (slot < pair_cap) pairs[slot] = Pair{pidx, citems[q]};
+        if (slot < pair_cap) pairs[slot] = Pair{pidx, (unsigned)q | kEdge};
       }
-    }
-  } else {
-    // K >= 2, one path per lane: row j of every lane's path at a time, the 32 rows'
-    // item ranges flattened over the warp; an item is tested against its owner lane's
-    // lines and points (fetched by shuffles), so no lane waits on another's long row
-    const int lane = threadIdx.x & 31;
-    const int nrow = row_hi >= row_lo ? row_hi - row_lo + 1 : 0;
-    const int maxrow = __reduce_max_sync(0xffffffffu, nrow);
-    for (int j = 0; j < maxrow; ++j) {
-      int q0 = 0, cnt = 0;
-      if (j < nrow) {
-        const int cy = row_lo + j;
-        int xmin, xmax;
-        row_span(cy, xmin, xmax);
-        if (xmin <= xmax) {
-          q0 = cstart[cy * cols + xmin];
-          cnt = cstart[cy * cols + xmax + 1] - q0;
-        }
-      }
-      int incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t_ = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t_;
-      }
-      const int excl = incl - cnt;
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      for (int k0 = 0; k0 < total; k0 += 32) {
-        const int k = k0 + lane;
-        int r = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-          const int e = __shfl_sync(0xffffffffu, excl, r + step);
-          if (e <= k) r += step;
-        }
-        const int qr = __shfl_sync(0xffffffffu, q0, r);
-        const int er = __shfl_sync(0xffffffffu, excl, r);
-        const int ot = __shfl_sync(0xffffffffu, t, r);
-        const int opidx = __shfl_sync(0xffffffffu, pidx, r);
-        double Lp[K][2], LU[K][2], Cp[K][2];
-        const double* Cb[K];
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-          Lp[i][0] = __shfl_sync(0xffffffffu, lp[i][0], r);
-          Lp[i][1] = __shfl_sync(0xffffffffu, lp[i][1], r);
-          LU[i][0] = __shfl_sync(0xffffffffu, lU[i][0], r);
-          LU[i][1] = __shfl_sync(0xffffffffu, lU[i][1], r);
-          Cp[i][0] = __shfl_sync(0xffffffffu, cpt[i][0], r);
-          Cp[i][1] = __shfl_sync(0xffffffffu, cpt[i][1], r);
-          Cb[i] = reinterpret_cast<const double*>(__shfl_sync(
-              0xffffffffu, reinterpret_cast<unsigned long long>(cbp[i]), r));
-        }
-        if (k >= total) continue;
-        const int q = qr + (k - er);
-        const double2 xy = v.cxy[ot][q];
-        bool ok = true;
-        // IDMap::visitPointsInRowSpans precise test
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-          const double dx = xy.x - Lp[i][0], dy = xy.y - Lp[i][1];
-          const double z = dy * LU[i][0] - dx * LU[i][1];
-          ok = ok && !(z * z > tol2);
-          if (v.near_band > 0.0) {
-            const double m = fabs(z) - v.tol2d;
-            if (fabs(m) < v.near_band)
-              near_append(v, 0, K, ot, v.cell_items[ot][q], in[opidx].cam(i), in[opidx].ids[i], m);
-          }
-        }
-        if (!ok) continue;
-        // checkBackProjection (StereoMatch.cpp:1206-1227)
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-          if (!ok) break;
-          const double2 a = reinterpret_cast<const double2*>(Cb[i])[2 * q];
-          const double2 b = reinterpret_cast<const double2*>(Cb[i])[2 * q + 1];
-          const double d0 = Cp[i][0] - a.x, d1 = Cp[i][1] - a.y;
-          const double z = d1 * b.x - d0 * b.y;
-          ok = !(z * z > tol2);
-          if (v.near_band > 0.0) {
-            const double m = fabs(z) - v.tol2d;
-            if (fabs(m) < v.near_band)
-              near_append(v, 1, K, ot, v.cell_items[ot][q], in[opidx].cam(i), in[opidx].ids[i], m);
-          }
-        }
-        if (!ok) continue;
-        const int slot = append_slot(pair_count);
-        if (slot < pair_cap) pairs[slot] = Pair{opidx, v.cell_items[ot][q]};
-      }
-    }
   }
 }
 
-// Expand one level, second half: one thread per (path, candidate) pair.  The quick
-// triangulation gate (computeMinParallaxDeg, calTriangulateTol,
-// TriangulationCheckWithTol: StereoMatch.cpp:1072-1141) on the path's lines plus the
-// candidate's, then the child path (terminal, or with its next target camera).
+// visit_cells for every path: a warp per path at level 1, else a thread.
 template <int K>
-__global__ void __launch_bounds__(256, 2) tri_kernel(const __grid_constant__ SmView v, const void* in_v,
-                                                     const Pair* pairs, int n_pairs, void* out_v,
-                                                     int* out_count, int out_cap, Path* term,
-                                                     int* term_count, int term_cap) {
-  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gi >= n_pairs) return;
-  const Pair pr = pairs[gi];
-  const PathN<K> P = static_cast<const PathN<K>*>(in_v)[pr.path];
-  const int t = P.target;
-  const int pid = pr.pid;
-  double cp[K][3], cu[K][3];  // chosen lines of sight (build order)
-#pragma unroll
-  for (int i = 0; i < K; ++i) {
-    const double* S = v.los[P.cam(i)] + 6 * (int64_t)P.ids[i];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      cp[i][q] = S[q];
-      cu[i][q] = S[3 + q];
-    }
-  }
-  // Normal equations of the chosen lines, summed in build order: the candidate's
-  // term is added last, which is the reference's summation order
-  // (myMATH::triangulation sums lines in list order, myMATH.cpp:376-391).
-  double Mc[9], bc[3];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) Mc[q] = 0.0;
-  bc[0] = bc[1] = bc[2] = 0.0;
-#pragma unroll
-  for (int i = 0; i < K; ++i) {
-    double tt[9];
-    normal_terms(cu[i], tt);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-      bc[r] = bc[r] + (tt[3 * r] * cp[i][0] + tt[3 * r + 1] * cp[i][1] + tt[3 * r + 2] * cp[i][2]);
-#pragma unroll
-    for (int q = 0; q < 9; ++q) Mc[q] = Mc[q] + tt[q];
-  }
-  // largest pairwise dot (smallest parallax) among the chosen lines
-  double maxdot_c = -2.0;
-#pragma unroll
-  for (int i = 0; i < K; ++i)
-#pragma unroll
-    for (int j = i + 1; j < K; ++j) maxdot_c = fmax(maxdot_c, clamped_dot(cu[i], cu[j]));
+__global__ void __launch_bounds__(256) enum_log_kernel(const __grid_constant__ SmView v,
+                                                       const void* in_v, int n_in, Pair* pairs,
+                                                       int* pair_count, int pair_cap) {
+  constexpr int L = K == 1 ? 32 : 1;
+  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+  const int pidx = gt / L;
+  if (pidx >= n_in) return;
+  visit_cells<K, true>(v, static_cast<const PathN<K>*>(in_v)[pidx], pidx, gt % L, L, pairs,
+                       pair_count, pair_cap);
+}
 
-  {
-    {
+// Expand one level, first half: the detections of the target camera inside the strips of a
+// path's K chosen points.  Any search region that holds every point within tol2d of all lines
+// gives the same set, because the tests decide; here it is, for each row of cells, the x range
+// that the strips (widened by the FP32 error bound) cover over the row's height.  A lane takes
+// four rows at a time (K >= 2: one path a lane, whose strips meet in a few rows; K = 1: one
+// path a warp, its rows over the lanes), looks up their runs of positions together and walks
+// them.  FP32 decides each distance; pairs whose distance is within the bound of the tolerance
+// are marked for FP64.  Accepted pairs collect in shared memory, and one atomic serves a
+// buffer of them.
+constexpr int kPairBuf = 160;  // entries a warp; flushed above 128
+
+template <int K>
+__global__ void __launch_bounds__(256, K <= 2 ? 4 : 3) enum_kernel(
+    const __grid_constant__ SmView v, const void* in_v, int n_in, Pair* pairs, int* pair_count,
+    int pair_cap) {
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int kRowStep = K == 1 ? 32 : 1;
+  __shared__ Pair buf_s[8][kPairBuf];
+  const int lane = threadIdx.x & 31;
+  Pair* buf = buf_s[threadIdx.x >> 5];
+  const PathN<K>* in = static_cast<const PathN<K>*>(in_v);
+  const float tol = (float)v.tol2d;
+  int fill = 0;
+  auto flush = [&] {
+    int base = 0;
+    if (lane == 0) base = atomicAdd(pair_count, fill);
+    base = __shfl_sync(kFull, base, 0);
+    __syncwarp();
+    for (int i = lane; i < fill; i += 32)
+      if (base + i < pair_cap) pairs[base + i] = buf[i];
+    __syncwarp();
+    fill = 0;
+  };
+  const int warps = gridDim.x * 8, w0 = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int n_chunk = K == 1 ? n_in : (n_in + 31) / 32;
+  for (int ch = w0; ch < n_chunk; ch += warps) {
+    const int pidx = K == 1 ? ch : ch * 32 + lane;
+    const bool live = pidx < n_in;
+    const PathN<K> P = in[live ? pidx : n_in - 1];
+    const int t = P.target;
+    float nx[K], ny[K], d[K], T[K], inv[K], r[K];
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const float4 L = v.fl[(int64_t)P.ids[i] * v.n_cam + t];
+      nx[i] = L.x;
+      ny[i] = L.y;
+      d[i] = L.z;
+      finite = finite && fabsf(L.x) + fabsf(L.y) + fabsf(L.z) < 1e30f;
+      T[i] = tol + v.eps + 5e-7f * fabsf(L.z);
+      inv[i] = fabsf(L.x) < 1e-6f ? 0.0f : 1.0f / L.x;
+      r[i] = T[i] * fabsf(inv[i]);
+    }
+    const int rows = v.rows[t], colsf = v.cols[t] * v.sub;
+    const float cellf = (float)v.cell, to_col = (float)v.sub / cellf;
+    const float xmax = (float)v.cols[t] * cellf, pad = 0.005f + 1e-6f * xmax;
+    int row_lo = 0, row_hi = live ? rows - 1 : -1;
+    if (!finite) {
+      if (live)
+        visit_cells<K, false>(v, P, pidx, K == 1 ? lane : 0, kRowStep, pairs, pair_count, pair_cap);
+      row_hi = -1;
+    } else {
+      // rows that the strips reach: the line's segment over the image's width (K = 1), the
+      // y-extent of the first two strips' parallelogram
+      float ymin = -1e30f, ymax = 1e30f;
+      if (K == 1) {
+        if (fabsf(ny[0]) >= 1e-6f) {
+          const float in_ = 1.0f / ny[0];
+          const float ya = -d[0] * in_, yb = -(d[0] + nx[0] * xmax) * in_;
+          const float e = T[0] * fabsf(in_) + 0.05f + 1e-6f * (fabsf(ya) + fabsf(yb));
+          ymin = fminf(ya, yb) - e;
+          ymax = fmaxf(ya, yb) + e;
+        }
+      } else {
+        constexpr int b = K > 1 ? 1 : 0;
+        const float det = nx[0] * ny[b] - ny[0] * nx[b];
+        if (fabsf(det) > 1e-4f) {
+          const float id = 1.0f / det;
+          const float c = (nx[b] * d[0] - nx[0] * d[b]) * id;
+          const float e = (fabsf(nx[0]) * T[b] + fabsf(nx[b]) * T[0]) * fabsf(id) +
+                          2.0f * v.eps * fabsf(id) + 0.01f;
+          ymin = c - e;
+          ymax = c + e;
+        }
+      }
+      const float lo = floorf(ymin / cellf - 1e-3f), hi = floorf(ymax / cellf + 1e-3f);
+      row_lo = (int)fminf(fmaxf(lo, 0.0f), (float)rows);
+      row_hi = live ? (int)fmaxf(fminf(hi, (float)(rows - 1)), -1.0f) : -1;
+    }
+    const int base = v.cell_off[t];
+    const int n_row = max(0, row_hi - row_lo + 1);
+    const int n_max = __reduce_max_sync(kFull, n_row);
+    for (int j0 = 0; j0 < n_max; j0 += 4 * kRowStep) {
+      int q0[4], end[4], total = 0;
       {
-        // extend the path; quick triangulation gate (computeMinParallaxDeg,
-        // calTriangulateTol, TriangulationCheckWithTol: StereoMatch.cpp:1072-1141)
-        double qp[3], qu[3];
-        {
-          const double* S = v.los[t] + 6 * (int64_t)pid;
-          qp[0] = S[0];
-          qp[1] = S[1];
-          qp[2] = S[2];
-          qu[0] = S[3];
-          qu[1] = S[4];
-          qu[2] = S[5];
-        }
-        constexpr int k1 = K + 1;
-        double maxdot = maxdot_c;
+        int a[4], b[4];
 #pragma unroll
-        for (int i = 0; i < K; ++i) maxdot = fmax(maxdot, clamped_dot(cu[i], qu));
-        double tq;
-        if (maxdot <= kCos6 - 1e-9 && maxdot >= -kCos6 + 1e-9) {
-          // min parallax in (6 + 5e-7, 174 - 5e-7) deg: the angle factor is exactly 1
-          tq = v.tol3d * sqrt(double(v.m > 2 ? v.m : 2) / double(k1)) * 1.0;
-        } else {
-          // near the 6-degree knee or beyond: the reference's acos/sin path
-          double min_deg = 180.0;
+        for (int s = 0; s < 4; ++s) {
+          const int j = j0 + (K == 1 ? s * 32 + lane : s);
+          a[s] = b[s] = 0;
+          if (j < n_row) {
+            const int cy = row_lo + j;
+            const float y0 = (float)cy * cellf, y1 = y0 + cellf;
+            float xl = 0.0f, xr = xmax;
 #pragma unroll
-          for (int i = 0; i < k1; ++i)
-#pragma unroll
-            for (int j = i + 1; j < k1; ++j)
-              min_deg = fmin(min_deg, pair_deg(i < K ? cu[i] : qu, j < K ? cu[j] : qu));
-          tq = quick_tol_from_deg(min_deg, k1, v.m, v.tol3d);
-        }
-        double M[9], b[3];
-        {
-          double tt[9];
-          normal_terms(qu, tt);
-#pragma unroll
-          for (int r = 0; r < 3; ++r)
-            b[r] = bc[r] + (tt[3 * r] * qp[0] + tt[3 * r + 1] * qp[1] + tt[3 * r + 2] * qp[2]);
-#pragma unroll
-          for (int q2 = 0; q2 < 9; ++q2) M[q2] = Mc[q2] + tt[q2];
-        }
-        double Mi[9], X[3];
-        gauss_inverse3(M, Mi);
-#pragma unroll
-        for (int r = 0; r < 3; ++r) X[r] = Mi[3 * r] * b[0] + Mi[3 * r + 1] * b[1] + Mi[3 * r + 2] * b[2];
-        double e = 0.0;
-        bool thrown = false;
-#pragma unroll
-        for (int i = 0; i < k1; ++i) {
-          const double* pp = (i < K) ? cp[i] : qp;
-          const double* uu = (i < K) ? cu[i] : qu;
-          thrown |= !line_error_term(X, pp, uu, e);
-        }
-        if (thrown) return;  // the reference's triangulation throws; the check fails
-        const double err = sqrt(e / k1);
-        if (!(err <= tq)) return;
-        PathN<K + 1> ch;
-#pragma unroll
-        for (int i = 0; i < K; ++i) ch.ids[i] = P.ids[i];
-        ch.ids[K] = pid;
-        ch.cams = P.cams | ((unsigned)t << (4 * K));
-        if (k1 == v.m) {
-          Path full;
-#pragma unroll
-          for (int i = 0; i < OLPT_MAX_CAM; ++i) {
-            full.ids[i] = 0;
-            full.cams[i] = 0;
-          }
-#pragma unroll
-          for (int i = 0; i < K + 1; ++i) {
-            full.ids[i] = ch.ids[i];
-            full.cams[i] = (signed char)ch.cam(i);
-          }
-          full.k = k1;
-          full.target = -1;
-          const int slot = append_slot(term_count);
-          if (slot < term_cap) term[slot] = full;
-          return;
-        }
-        if (k1 >= OLPT_MAX_CAM) return;
-        // StereoMatch::selectNextCameraByMaxPairAngle (StereoMatch.cpp:1375-1411)
-        int best = -1;
-        double best_score = -1.0;
-        for (int cam = 0; cam < v.n_cam; ++cam) {
-          if (!v.active[cam]) continue;
-          bool used = false;
-#pragma unroll
-          for (int i = 0; i < K + 1; ++i) used |= (ch.cam(i) == cam);
-          if (used) continue;
-          double ux[K + 1], uy[K + 1];
-#pragma unroll
-          for (int i = 0; i < K + 1; ++i) {
-            const double* L = v.l2d[ch.cam(i)][cam] + 6 * (int64_t)ch.ids[i];
-            ux[i] = L[2];
-            uy[i] = L[3];
-          }
-          double score = 0.0;
-          if (k1 >= 2) {
-#pragma unroll
-            for (int i = 0; i < K + 1; ++i) {
-#pragma unroll
-              for (int j = i + 1; j < K + 1; ++j) {
-                const double s = fabs(ux[i] * uy[j] - uy[i] * ux[j]);
-                if (s > score) score = s;
-                if (score >= 1.0 - 1e-12) break;
-              }
-              if (score >= 1.0 - 1e-12) break;
+            for (int i = 0; i < K; ++i) {
+              if (inv[i] == 0.0f) continue;
+              const float ca = -fmaf(ny[i], y0, d[i]) * inv[i];
+              const float cb = -fmaf(ny[i], y1, d[i]) * inv[i];
+              xl = fmaxf(xl, fminf(ca, cb) - r[i] - pad);
+              xr = fminf(xr, fmaxf(ca, cb) + r[i] + pad);
+            }
+            const int fa = max(0, (int)floorf(xl * to_col - 0.01f));
+            const int fb = min(colsf - 1, (int)floorf(xr * to_col + 0.01f));
+            if (xl <= xr && fa <= fb) {
+              a[s] = v.cstart[base + cy * colsf + fa];
+              b[s] = v.cstart[base + cy * colsf + fb + 1];
             }
           }
-          if (score > best_score) {
-            best_score = score;
-            best = cam;
+        }
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          q0[s] = a[s] - total;
+          total += b[s] - a[s];
+          end[s] = total;
+        }
+      }
+      const int most = __reduce_max_sync(kFull, total);
+      for (int j = 0; j < most; ++j) {
+        const int q = j + (j < end[0] ? q0[0] : j < end[1] ? q0[1] : j < end[2] ? q0[2] : q0[3]);
+        bool ok = j < total, edge = false;
+        if (ok) {
+          const float2 p = v.fxy[q];
+#pragma unroll
+          for (int i = 0; i < K; ++i) {
+            const float z = fabsf(fmaf(nx[i], p.x, fmaf(ny[i], p.y, d[i])));
+            ok = ok && !(z > T[i]);
+            edge = edge || !(z < 2.0f * tol - T[i]);
           }
         }
-        if (best < 0) return;
-        ch.target = best;
-        const int slot = append_slot(out_count);
-        if (slot < out_cap) static_cast<PathN<K + 1>*>(out_v)[slot] = ch;
+        const unsigned m = __ballot_sync(kFull, ok);
+        if (m) {
+          if (ok)
+            buf[fill + __popc(m & ((1u << lane) - 1u))] =
+                Pair{pidx, (unsigned)q | (edge ? kEdge : 0u)};
+          fill += __popc(m);
+          if (fill > kPairBuf - 32) flush();
+        }
       }
     }
   }
+  if (fill) flush();
 }
 
+// Lines of sight of a path's chosen points and of a candidate (last).
+template <int K>
+struct Rays {
+  double p[K + 1][3], u[K + 1][3];
+};
+
+// calTriangulateTol (StereoMatch.cpp:1103-1126) where the smallest parallax is near or below
+// the 6-degree knee: the reference's acos / sin path.
+template <int K>
+__device__ __noinline__ double knee_tol(const SmView& v, const Rays<K>& r) {
+  double min_deg = 180.0;
+  for (int i = 0; i <= K; ++i)
+    for (int j = i + 1; j <= K; ++j) min_deg = fmin(min_deg, pair_deg(r.u[i], r.u[j]));
+  return quick_tol_from_deg(min_deg, K + 1, v.m, v.tol3d);
+}
+
+// TriangulationCheckWithTol (StereoMatch.cpp:1127-1141) with myMATH::triangulation's own
+// operations: the lines summed in build order, the candidate last (myMATH.cpp:376-418).
+template <int K>
+__device__ __noinline__ bool gate_exact(const Rays<K>& r, double tq) {
+  double M[9], b[3];
+  for (int q = 0; q < 9; ++q) M[q] = 0.0;
+  b[0] = b[1] = b[2] = 0.0;
+  for (int i = 0; i <= K; ++i) {
+    double tt[9];
+    normal_terms(r.u[i], tt);
+    for (int q = 0; q < 3; ++q)
+      b[q] = b[q] + (tt[3 * q] * r.p[i][0] + tt[3 * q + 1] * r.p[i][1] + tt[3 * q + 2] * r.p[i][2]);
+    for (int q = 0; q < 9; ++q) M[q] = M[q] + tt[q];
+  }
+  double Mi[9], X[3];
+  gauss_inverse3(M, Mi);
+  for (int q = 0; q < 3; ++q) X[q] = Mi[3 * q] * b[0] + Mi[3 * q + 1] * b[1] + Mi[3 * q + 2] * b[2];
+  double e = 0.0;
+  bool thrown = false;
+  for (int i = 0; i <= K; ++i) thrown |= !line_error_term(X, r.p[i], r.u[i], e);
+  if (thrown) return false;  // the reference's triangulation throws; the check fails
+  return sqrt(e / (K + 1)) <= tq;
+}
+
+__device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
+  return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+}
+
+// The triangulation gate.  The sum E of the squared distances of the least-squares point to
+// the lines is formed from the point o of line 0 nearest line 1: with v_i the perpendicular
+// from o to line i, M = sum(I - u u^T) and b = sum v_i, E = sum |v_i|^2 - b M^-1 b.  The v_i
+// are as small as the distances themselves, so nothing cancels, and it takes two divisions
+// where the reference's elimination and square roots take 17 and 2 k.  The reference's own e
+// is within a few ulp of |X - p|^2 per line of E; a value farther than a wide multiple of that
+// from the limit decides as the reference does, any other goes through its operations, as do
+// nearly parallel lines and points so far away that its distance could turn out negative
+// enough to throw.
+template <int K>
+__device__ __forceinline__ bool gate(const SmView& v, const Rays<K>& r) {
+  constexpr int k1 = K + 1;
+  double maxdot = -2.0;
+#pragma unroll
+  for (int i = 0; i < k1; ++i)
+#pragma unroll
+    for (int j = i + 1; j < k1; ++j) maxdot = fmax(maxdot, clamped_dot(r.u[i], r.u[j]));
+  // min parallax in (6 + 5e-7, 174 - 5e-7) deg: the angle factor is exactly 1
+  const double tq =
+      maxdot <= kCos6 - 1e-9 && maxdot >= -kCos6 + 1e-9 ? v.tq[k1] : knee_tol<K>(v, r);
+  const double w[3] = {r.p[1][0] - r.p[0][0], r.p[1][1] - r.p[0][1], r.p[1][2] - r.p[0][2]};
+  const double c = dot3(r.u[0], r.u[1]), s2 = 1.0 - c * c;
+  const double t0 = (dot3(w, r.u[0]) - dot3(w, r.u[1]) * c) / s2;
+  double o[3], R2 = t0 * t0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) o[d] = r.p[0][d] + t0 * r.u[0][d];
+  double E, det = 1.0;
+  if (K == 1) {
+    const double q[3] = {r.p[1][0] - o[0], r.p[1][1] - o[1], r.p[1][2] - o[2]};
+    const double a = dot3(q, r.u[1]);
+    const double x[3] = {q[0] - a * r.u[1][0], q[1] - a * r.u[1][1], q[2] - a * r.u[1][2]};
+    R2 = fmax(R2, dot3(q, q));
+    E = 0.5 * dot3(x, x);  // the point halfway between the lines
+  } else {
+    double b[3] = {0, 0, 0}, S = 0.0;
+    double mxx = k1, myy = k1, mzz = k1, mxy = 0, mxz = 0, myz = 0;
+#pragma unroll
+    for (int i = 0; i < k1; ++i) {
+      const double* u = r.u[i];
+      mxx -= u[0] * u[0];
+      myy -= u[1] * u[1];
+      mzz -= u[2] * u[2];
+      mxy -= u[0] * u[1];
+      mxz -= u[0] * u[2];
+      myz -= u[1] * u[2];
+      if (i == 0) continue;  // o lies on line 0
+      const double q[3] = {r.p[i][0] - o[0], r.p[i][1] - o[1], r.p[i][2] - o[2]};
+      const double a = dot3(q, u);
+      R2 = fmax(R2, dot3(q, q));
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double x = q[d] - a * u[d];
+        b[d] += x;
+        S += x * x;
+      }
+    }
+    const double cxx = myy * mzz - myz * myz, cxy = mxz * myz - mxy * mzz,
+                 cxz = mxy * myz - mxz * myy;
+    const double cyy = mxx * mzz - mxz * mxz, cyz = mxy * mxz - mxx * myz,
+                 czz = mxx * myy - mxy * mxy;
+    det = mxx * cxx + mxy * cxy + mxz * cxz;
+    const double bMb = b[0] * (cxx * b[0] + 2.0 * (cxy * b[1] + cxz * b[2])) +
+                       b[1] * (cyy * b[1] + 2.0 * cyz * b[2]) + czz * b[2] * b[2];
+    E = S - bMb / det;
+  }
+  const double lim = k1 * (tq * tq);
+  // R2 <= 4e6: the reference's squared distances are above -1e-8 (8 ulp of R2)
+  const bool safe = s2 > 1e-3 && det > 1e-3 && R2 <= 4e6;
+  const double band = 1e-6 * lim + k1 * 1e-14 * R2 + 1e-9 * E;
+  if (safe && E > lim + band) return false;
+  if (safe && E < lim - band) return true;
+  return gate_exact<K>(r, tq);
+}
+
+// StereoMatch::selectNextCameraByMaxPairAngle (StereoMatch.cpp:1375-1411) in FP64.
+template <int N>
+__device__ __noinline__ int next_camera_exact(const SmView& v, const PathN<N>& ch) {
+  int best = -1;
+  double best_score = -1.0;
+  for (int cam = 0; cam < v.n_cam; ++cam) {
+    if (!v.active[cam]) continue;
+    bool used = false;
+    for (int i = 0; i < N; ++i) used |= (ch.cam(i) == cam);
+    if (used) continue;
+    double ux[N], uy[N];
+    for (int i = 0; i < N; ++i) {
+      const double* L = v.l2d + 6 * ((int64_t)ch.ids[i] * v.n_cam + cam);
+      ux[i] = L[2];
+      uy[i] = L[3];
+    }
+    double score = 0.0;
+    for (int i = 0; i < N; ++i) {
+      for (int j = i + 1; j < N; ++j) {
+        const double s = fabs(ux[i] * uy[j] - uy[i] * ux[j]);
+        if (s > score) score = s;
+        if (score >= 1.0 - 1e-12) break;
+      }
+      if (score >= 1.0 - 1e-12) break;
+    }
+    if (score > best_score) {
+      best_score = score;
+      best = cam;
+    }
+  }
+  return best;
+}
+
+// The same from the FP32 lines (their normals span the same angles): the largest score wins
+// when it is clear of the others by far more than FP32 can err.
+template <int N>
+__device__ __forceinline__ int next_camera(const SmView& v, const PathN<N>& ch) {
+  int best = -1, left = 0;
+  float top = -1.0f, second = -1.0f;
+  for (int cam = 0; cam < v.n_cam; ++cam) {
+    bool used = !v.active[cam];
+#pragma unroll
+    for (int i = 0; i < N; ++i) used |= (ch.cam(i) == cam);
+    if (used) continue;
+    ++left;
+    float2 n[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      n[i] = *reinterpret_cast<const float2*>(v.fl + (int64_t)ch.ids[i] * v.n_cam + cam);
+    float score = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = i + 1; j < N; ++j)
+        score = fmaxf(score, fabsf(n[i].x * n[j].y - n[i].y * n[j].x));
+    if (score > top) {
+      second = top;
+      top = score;
+      best = cam;
+    } else if (score > second) {
+      second = score;
+    }
+  }
+  if (left <= 1 || top - second > 1e-5f) return best;
+  return next_camera_exact<N>(v, ch);
+}
+
+// Expand one level, second half: one thread per (path, candidate) pair.  The
+// back-projection test (in FP32 where it is clear, else all 2D tests in FP64), the quick
+// triangulation gate (computeMinParallaxDeg, calTriangulateTol, TriangulationCheckWithTol:
+// StereoMatch.cpp:1072-1141), then the child path (terminal, or with its next target camera).
+// Bound by the gathers of the candidates' lines (about 150 B each).
+template <int K>
+__global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
+    const __grid_constant__ SmView v, const void* in_v, const Pair* pairs, int n_pairs,
+    void* out_v, int* out_count, int out_cap, Path* term, int* term_count, int term_cap) {
+  __shared__ int s_cnt[8], s_base;
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool last = K + 1 == v.m;
+  PathN<K + 1> ch;
+  bool ok = gi < n_pairs;
+  if (ok) {
+    const Pair pr = pairs[gi];
+    const PathN<K> P = static_cast<const PathN<K>*>(in_v)[pr.path];
+    const int g = (int)(pr.g & ~kEdge);
+    bool edge = (pr.g & kEdge) != 0;
+    const float tol = (float)v.tol2d;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const float4 L = v.fl[(int64_t)g * v.n_cam + P.cam(i)];
+      const float2 p = v.fxy[P.ids[i]];
+      const float z = fabsf(fmaf(L.x, p.x, fmaf(L.y, p.y, L.z)));
+      const float e = v.eps + 5e-7f * fabsf(L.z);
+      ok = ok && !(z > tol + e);
+      edge = edge || !(z < tol - e);
+    }
+    if (ok && edge) ok = exact_2d<K, false>(v, P, g);
+    if (ok) {
+      Rays<K> r;
+#pragma unroll
+      for (int i = 0; i <= K; ++i) {
+        const double2* S =
+            reinterpret_cast<const double2*>(v.los + 6 * (int64_t)(i < K ? P.ids[i < K ? i : 0] : g));
+        const double2 a = S[0], b = S[1], c = S[2];
+        r.p[i][0] = a.x;
+        r.p[i][1] = a.y;
+        r.p[i][2] = b.x;
+        r.u[i][0] = b.y;
+        r.u[i][1] = c.x;
+        r.u[i][2] = c.y;
+      }
+      ok = gate<K>(v, r);
+    }
+    if (ok) {
+#pragma unroll
+      for (int i = 0; i < K; ++i) ch.ids[i] = P.ids[i];
+      ch.ids[K] = g;
+      ch.cams = P.cams | ((unsigned)P.target << (4 * K));
+      ch.target = -1;
+      if (!last) {
+        ch.target = K + 1 < OLPT_MAX_CAM ? next_camera<K + 1>(v, ch) : -1;
+        ok = ch.target >= 0;
+      }
+    }
+  }
+  // one atomic a block
+  const unsigned m = __ballot_sync(0xffffffffu, ok);
+  if (lane == 0) s_cnt[warp] = __popc(m);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int t = 0;
+    for (int w = 0; w < 8; ++w) {
+      const int k = s_cnt[w];
+      s_cnt[w] = t;
+      t += k;
+    }
+    s_base = t ? atomicAdd(last ? term_count : out_count, t) : 0;
+  }
+  __syncthreads();
+  if (!ok) return;
+  const int slot = s_base + s_cnt[warp] + __popc(m & ((1u << lane) - 1u));
+  if (!last) {
+    if (slot < out_cap) static_cast<PathN<K + 1>*>(out_v)[slot] = ch;
+    return;
+  }
+  if (slot >= term_cap) return;
+  Path full;
+#pragma unroll
+  for (int i = 0; i < OLPT_MAX_CAM; ++i) {
+    full.ids[i] = i <= K ? ch.ids[i <= K ? i : 0] : 0;
+    full.cams[i] = i <= K ? (signed char)ch.cam(i) : 0;
+  }
+  full.k = K + 1;
+  full.target = -1;
+  term[slot] = full;
+}
 
 // StereoMatch::checkMatch, case "every active camera was used to build"
 // (StereoMatch.cpp:520-540): triangulate in camera order, gate on tol_3d and limit.
@@ -841,7 +1107,7 @@ __global__ void check_kernel(const __grid_constant__ SmView v, const Path* term,
   int n = 0;
   for (int c = 0; c < v.n_cam; ++c) {
     if (ids[c] < 0) continue;
-    load_line3(v.los[c] + 6 * (int64_t)ids[c], Ls[n]);
+    load_line3(v.los + 6 * (int64_t)ids[c], Ls[n]);
     Lp[n] = &Ls[n];
     ++n;
   }
@@ -853,7 +1119,8 @@ __global__ void check_kernel(const __grid_constant__ SmView v, const Path* term,
     return;
   int slot = atomicAdd(cand_count, 1);
   if (slot >= cap) return;
-  for (int c = 0; c < v.n_cam; ++c) cand_ids[(int64_t)slot * v.n_cam + c] = ids[c];
+  for (int c = 0; c < v.n_cam; ++c)
+    cand_ids[(int64_t)slot * v.n_cam + c] = ids[c] < 0 ? -1 : v.pid[ids[c]];
   cand_e[slot] = err;
   cand_x[3 * slot] = X[0];
   cand_x[3 * slot + 1] = X[1];
@@ -957,100 +1224,74 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
   }
   res.ref_cam = ref;
 
-  // grids and lines
+  // grid over the detections of all cameras
+  int64_t total = 0;
+  float max_side = 0.0f;
+  int64_t cells = 0;
   for (int c = 0; c < n_cam; ++c) {
     const CamDev& cm = ctx->cams_h[c];
-    const int64_t n = v.active[c] ? ctx->det_counts_h[c] : 0;
-    v.n[c] = n;
+    v.raw_off[c] = (int)total;
+    total += v.active[c] ? ctx->det_counts_h[c] : 0;
     v.x[c] = ctx->dets[c].x.as<double>();
     v.y[c] = ctx->dets[c].y.as<double>();
     v.Wd[c] = (double)cm.n_col;
     v.Hd[c] = (double)cm.n_row;
-    const int rows = std::max(1, cm.n_row / v.cell + (cm.n_row % v.cell ? 1 : 0));
-    const int cols = std::max(1, cm.n_col / v.cell + (cm.n_col % v.cell ? 1 : 0));
-    v.rows[c] = rows;
-    v.cols[c] = cols;
-    if (!v.active[c]) continue;
-    const int ncell = rows * cols;
-    W.cell_start[c].ensure((ncell + 1) * sizeof(int), s);
-    W.cell_cursor[c].ensure(ncell * sizeof(int), s);
-    W.cell_items[c].ensure((n + 1) * sizeof(int), s);
-    W.cell_of[c].ensure((n + 1) * sizeof(int), s);
-    W.los[c].ensure((n + 1) * 6 * sizeof(double), s);
-    OLPT_CUDA(cudaMemsetAsync(W.cell_cursor[c].p, 0, ncell * sizeof(int), s));
-    if (n > 0) {
-      cell_hist_kernel<<<OLPT_G(nblk(n)), 256, 0, s>>>(v.x[c], v.y[c], n, v.cell, rows, cols,
-                                                W.cell_of[c].as<int>(), W.cell_cursor[c].as<int>());
-    }
-    exclusive_scan(W.cell_cursor[c].as<int>(), ncell, W.cell_start[c].as<int>(), W.scan_tmp, s);
-    OLPT_CUDA(cudaMemsetAsync(W.cell_cursor[c].p, 0, ncell * sizeof(int), s));
-    if (n > 0) {
-      cell_scatter_kernel<<<OLPT_G(nblk(n)), 256, 0, s>>>(W.cell_of[c].as<int>(), n, W.cell_start[c].as<int>(),
-                                                   W.cell_cursor[c].as<int>(), W.cell_items[c].as<int>());
-      cell_sort_kernel<<<OLPT_G(nblk(ncell)), 256, 0, s>>>(W.cell_start[c].as<int>(), ncell,
-                                                    W.cell_items[c].as<int>());
-    }
-    OLPT_CUDA(cudaGetLastError());
-    v.cell_start[c] = W.cell_start[c].as<int>();
-    v.cell_items[c] = W.cell_items[c].as<int>();
-    v.los[c] = W.los[c].as<double>();
+    v.rows[c] = std::max(1, cm.n_row / v.cell + (cm.n_row % v.cell ? 1 : 0));
+    v.cols[c] = std::max(1, cm.n_col / v.cell + (cm.n_col % v.cell ? 1 : 0));
+    max_side = std::max(max_side, (float)(v.rows[c] + v.cols[c]) * v.cell);
+    cells += (int64_t)v.rows[c] * v.cols[c];
   }
-  // image lines of every detection on every other active camera
-  {
-    W.l2d_ptrs.ensure(OLPT_MAX_CAM * OLPT_MAX_CAM * sizeof(double*), s);
-    W.active_d.ensure(OLPT_MAX_CAM * sizeof(int), s);
-    std::vector<double*> ptrs(OLPT_MAX_CAM * OLPT_MAX_CAM, nullptr);
-    for (int c = 0; c < n_cam; ++c) {
-      if (!v.active[c]) continue;
-      for (int t = 0; t < n_cam; ++t) {
-        if (t == c || !v.active[t]) continue;
-        DevBuf& b = W.l2d[c * OLPT_MAX_CAM + t];
-        b.ensure((v.n[c] + 1) * 6 * sizeof(double), s);
-        ptrs[c * OLPT_MAX_CAM + t] = b.as<double>();
-        v.l2d[c][t] = b.as<double>();
-      }
-    }
-    OLPT_CUDA(cudaMemcpyAsync(W.l2d_ptrs.p, ptrs.data(), ptrs.size() * sizeof(double*),
-                              cudaMemcpyHostToDevice, s));
-    OLPT_CUDA(cudaMemcpyAsync(W.active_d.p, v.active, OLPT_MAX_CAM * sizeof(int),
-                              cudaMemcpyHostToDevice, s));
-    for (int c = 0; c < n_cam; ++c) {
-      if (!v.active[c] || v.n[c] == 0) continue;
-      lines_kernel<<<OLPT_G(nblk(v.n[c], 128)), 128, 0, s>>>(
-          ctx->cams_d.as<CamDev>(), c, v.x[c], v.y[c], v.n[c], n_cam, W.active_d.as<int>(),
-          W.los[c].as<double>(), W.l2d_ptrs.as<double*>() + c * OLPT_MAX_CAM);
-      OLPT_CUDA(cudaGetLastError());
-    }
-    // cell-ordered copies for the enumeration
-    W.cbp_ptrs.ensure(2 * OLPT_MAX_CAM * OLPT_MAX_CAM * sizeof(double*), s);
-    std::vector<double*> bp(2 * OLPT_MAX_CAM * OLPT_MAX_CAM, nullptr);
-    for (int t = 0; t < n_cam; ++t) {
-      if (!v.active[t]) continue;
-      W.cxy[t].ensure((v.n[t] + 1) * sizeof(double2), s);
-      v.cxy[t] = W.cxy[t].as<double2>();
-      for (int c = 0; c < n_cam; ++c) {
-        if (c == t || !v.active[c]) continue;
-        DevBuf& b = W.cbp[t * OLPT_MAX_CAM + c];
-        b.ensure((v.n[t] + 1) * 4 * sizeof(double), s);
-        bp[t * OLPT_MAX_CAM + c] = b.as<double>();
-        v.cbp[t][c] = b.as<double>();
-      }
-      for (int c = 0; c < n_cam; ++c)
-        bp[OLPT_MAX_CAM * OLPT_MAX_CAM + t * OLPT_MAX_CAM + c] = ptrs[t * OLPT_MAX_CAM + c];
-    }
-    OLPT_CUDA(cudaMemcpyAsync(W.cbp_ptrs.p, bp.data(), bp.size() * sizeof(double*),
-                              cudaMemcpyHostToDevice, s));
-    for (int t = 0; t < n_cam; ++t) {
-      if (!v.active[t] || v.n[t] == 0) continue;
-      double* const* outs = W.cbp_ptrs.as<double*>() + t * OLPT_MAX_CAM;
-      const double* const* lines =
-          W.cbp_ptrs.as<const double*>() + OLPT_MAX_CAM * OLPT_MAX_CAM + t * OLPT_MAX_CAM;
-      cell_pack_kernel<<<OLPT_G(nblk(v.n[t])), 256, 0, s>>>(
-          W.cell_items[t].as<int>(), v.n[t], v.x[t], v.y[t], W.cxy[t].as<double2>(), outs, lines,
-          n_cam, t);
-      OLPT_CUDA(cudaGetLastError());
-    }
+  OLPT_REQUIRE(total < (1ll << 30), OLPT_ERR_UNSUPPORTED, "stereo: too many detections");
+  v.raw_off[n_cam] = (int)total;
+  v.eps = 1e-6f * max_side;
+  // calTriangulateTol (StereoMatch.cpp:1103-1126) with an angle factor of 1
+  for (int k = 2; k <= OLPT_MAX_CAM; ++k)
+    v.tq[k] = v.tol3d * std::sqrt(double(v.m > 2 ? v.m : 2) / double(k)) * 1.0;
+  // columns of a pixel where the cells stay within a few million entries (a run of cells then
+  // covers little more than its x range: 1.7 times fewer positions to test at 0.06
+  // detections/px than with square cells of 4 px), else wider
+  v.sub = v.cell;
+  while (v.sub > 1 && cells * v.sub > (8ll << 20)) v.sub /= 2;
+  int64_t n_cells = 0;
+  for (int c = 0; c < n_cam; ++c) {
+    v.cell_off[c] = (int)n_cells;
+    if (v.active[c]) n_cells += (int64_t)v.rows[c] * v.cols[c] * v.sub + 1;
   }
+  OLPT_REQUIRE(n_cells < (1ll << 30), OLPT_ERR_UNSUPPORTED, "stereo: too many grid cells");
+  const int n = (int)total;
+  W.cell_start.ensure((size_t)(n_cells + 1) * sizeof(int), s);
+  W.cell_cnt.ensure((size_t)(n_cells + 1) * sizeof(int), s);
+  W.cell_of.ensure((size_t)(n + 1) * sizeof(int), s);
+  W.pid.ensure((size_t)(n + 1) * sizeof(int), s);
+  W.xy.ensure((size_t)(n + 1) * sizeof(double2), s);
+  W.fxy.ensure((size_t)(n + 1) * sizeof(float2), s);
+  W.los.ensure((size_t)(n + 1) * 6 * sizeof(double), s);
+  W.l2d.ensure((size_t)(n + 1) * n_cam * 6 * sizeof(double), s);
+  W.fl.ensure((size_t)(n + 1) * n_cam * sizeof(float4), s);
+  v.cstart = W.cell_start.as<int>();
+  v.pid = W.pid.as<int>();
+  v.xy = W.xy.as<double2>();
+  v.fxy = W.fxy.as<float2>();
+  v.los = W.los.as<double>();
+  v.l2d = W.l2d.as<double>();
+  v.fl = W.fl.as<float4>();
+  OLPT_CUDA(cudaMemsetAsync(W.cell_cnt.p, 0, (size_t)n_cells * sizeof(int), s));
+  if (n > 0)
+    bin_kernel<<<OLPT_G(nblk(n)), 256, 0, s>>>(v, n, W.cell_of.as<int>(), W.cell_cnt.as<int>());
+  exclusive_scan(W.cell_cnt.as<int>(), (int)n_cells, W.cell_start.as<int>(), W.scan_tmp, s);
+  if (n > 0) {
+    place_kernel<<<OLPT_G(nblk(n)), 256, 0, s>>>(v, n, W.cell_of.as<int>(), W.cell_cnt.as<int>(),
+                                                 W.pid.as<int>(), W.xy.as<double2>(),
+                                                 W.fxy.as<float2>());
+    int64_t most = 0;
+    for (int c = 0; c < n_cam; ++c)
+      most = std::max<int64_t>(most, v.raw_off[c + 1] - v.raw_off[c]);
+    los_kernel<<<OLPT_G(dim3(nblk(most, kLineThreads / 2), n_cam)), kLineThreads, 0, s>>>(
+        v, ctx->cams_d.as<CamDev>(), W.los.as<double>());
+    lines_kernel<<<OLPT_G(dim3(nblk(n, kLineThreads), n_cam)), kLineThreads, 0, s>>>(
+        v, ctx->cams_d.as<CamDev>(), W.l2d.as<double>(), W.fl.as<float4>());
+  }
+  OLPT_CUDA(cudaGetLastError());
 
   // breadth-first expansion of the build DFS
   W.counters.ensure(8 * sizeof(int), s);
@@ -1061,9 +1302,21 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
     OLPT_CUDA(cudaStreamSynchronize(s));
     return h;
   };
-  int64_t n_ref = v.n[ref];
+  const int64_t n_ref = v.raw_off[ref + 1] - v.raw_off[ref];
   int cap_a = (int)std::max<int64_t>(n_ref, 1024);
-  W.path_a.ensure(cap_a * sizeof(Path), s);
+  // bytes of a partial path of k points
+  auto rec = [](int k) -> size_t {
+    switch (k) {
+      case 1: return sizeof(PathN<1>);
+      case 2: return sizeof(PathN<2>);
+      case 3: return sizeof(PathN<3>);
+      case 4: return sizeof(PathN<4>);
+      case 5: return sizeof(PathN<5>);
+      case 6: return sizeof(PathN<6>);
+      default: return sizeof(PathN<8>);
+    }
+  };
+  W.path_a.ensure(cap_a * rec(1), s);
   OLPT_CUDA(cudaMemsetAsync(cnt, 0, 8 * sizeof(int), s));
   if (n_ref > 0)
     seed_kernel<<<OLPT_G(nblk(n_ref)), 256, 0, s>>>(v, ref, W.path_a.as<PathN<1>>(), cnt, cap_a);
@@ -1085,19 +1338,22 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
       W.pairs.ensure((size_t)pair_cap * sizeof(Pair), s);
       OLPT_CUDA(cudaMemsetAsync(cnt + 4, 0, sizeof(int), s));
       const int pid = ctx->prof.begin(PROF_STEREO, s);
-      auto kern = enum_kernel<1, true>;
+      const bool log = v.near_band > 0.0;
+      auto kern = log ? enum_log_kernel<1> : enum_kernel<1>;
       switch (level) {
-        case 1: kern = enum_kernel<1, true>; break;
-        case 2: kern = enum_kernel<2, false>; break;
-        case 3: kern = enum_kernel<3, false>; break;
-        case 4: kern = enum_kernel<4, false>; break;
-        case 5: kern = enum_kernel<5, false>; break;
-        case 6: kern = enum_kernel<6, false>; break;
-        default: kern = enum_kernel<7, false>; break;
+        case 1: break;
+        case 2: kern = log ? enum_log_kernel<2> : enum_kernel<2>; break;
+        case 3: kern = log ? enum_log_kernel<3> : enum_kernel<3>; break;
+        case 4: kern = log ? enum_log_kernel<4> : enum_kernel<4>; break;
+        case 5: kern = log ? enum_log_kernel<5> : enum_kernel<5>; break;
+        case 6: kern = log ? enum_log_kernel<6> : enum_kernel<6>; break;
+        default: kern = log ? enum_log_kernel<7> : enum_kernel<7>; break;
       }
       const int64_t work = level == 1 ? (int64_t)n_in * 32 : (int64_t)n_in;
-      kern<<<OLPT_G(nblk(work)), 256, 0, s>>>(v, in_buf->p, n_in, W.pairs.as<Pair>(), cnt + 4,
-                                                pair_cap);
+      // enum_kernel: at most eight chunks a warp slot, so that a warp's buffer fills
+      const int64_t blocks = log ? nblk(work) : std::min<int64_t>(nblk(work), 148 * 32);
+      kern<<<OLPT_G((int)blocks), 256, 0, s>>>(v, in_buf->p, n_in, W.pairs.as<Pair>(), cnt + 4,
+                                               pair_cap);
       ctx->prof.end(PROF_STEREO, pid, s, 0.0);
       OLPT_CUDA(cudaGetLastError());
       n_pairs = read_count(4);
@@ -1108,10 +1364,11 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
       break;
     }
     // quick triangulation gate and the children
-    out_cap = (int)std::max<int64_t>(out_cap, (int64_t)(out_buf->bytes / sizeof(Path)) - 1);
+    out_cap = (int)std::max<int64_t>(
+        out_cap, std::min<int64_t>(INT32_MAX, (int64_t)(out_buf->bytes / rec(level + 1)) - 1));
     term_cap = (int)std::max<int64_t>(term_cap, (int64_t)(W.term.bytes / sizeof(Path)) - 1);
     for (;;) {
-      out_buf->ensure((size_t)out_cap * sizeof(Path), s);
+      if (level + 1 < v.m) out_buf->ensure((size_t)out_cap * rec(level + 1), s);
       W.term.ensure((size_t)term_cap * sizeof(Path), s);
       // counters: [1] = children, [2] = terminals (terminals accumulate across levels)
       OLPT_CUDA(cudaMemsetAsync(cnt + 1, 0, sizeof(int), s));
