@@ -111,11 +111,10 @@ struct Dets {
 };
 
 // CSR (start[n_buckets + 1], items[n]) from per-item bucket keys (key < 0: dropped);
-// built by count -> exclusive scan -> scatter -> per-bucket ascending order (scan.cu).
+// built by count -> exclusive scan -> scatter (scan.cu); items of a bucket in any order.
 struct Csr {
   DevBuf start, items, cursor, tmp;
-  // sort_buckets: ascending item order inside each bucket (only where order matters)
-  void build(const int* key, int n, int n_buckets, cudaStream_t s, bool sort_buckets = false);
+  void build(const int* key, int n, int n_buckets, cudaStream_t s);
   void release(cudaStream_t s) {
     start.release(s);
     items.release(s);
@@ -186,20 +185,21 @@ struct PruneView {
 struct PruneWork {
   DevBuf key, val, key2, val2, hist, scan_tmp;
   DevBuf ids_s, e_s, X_s;
-  DevBuf fl, slot_key, fcnt, slot_pct, slot_used, pct, flag;
-  DevBuf f_pct, f_both, pos_pct, pos_both, pcls, ecls, newc, excl, cstart;
+  DevBuf fl, slot_key, fcnt, slot_pct, slot_used, pct;
+  DevBuf counts;  // PruneCount words (prune.cu)
+  DevBuf pcls, ecls, cstart, tiles, mixed;
   DevBuf g_pts, g_cnt, g_pct, g_e, pool_e, pool_i;
-  DevBuf gkey, gstate, gfirst, gowner, sel, spos, scnt, mixed;
-  Csr points, gpoints;
-  HostBuf pin;  // pinned staging of the greedy's input
+  DevBuf gstate, gfirst, gowner, sel, spos, scnt;
+  Csr points;
+  int n_sel = 0;  // kept candidates of the last device prune
+  HostBuf pin;    // pinned staging of the sequential greedy's input
   void release(cudaStream_t s) {
     for (DevBuf* b : {&key, &val, &key2, &val2, &hist, &scan_tmp, &ids_s, &e_s, &X_s, &fl,
-                      &slot_key, &fcnt, &slot_pct, &slot_used, &pct, &flag, &f_pct, &f_both,
-                      &pos_pct, &pos_both, &pcls, &ecls, &newc, &excl, &cstart, &g_pts, &g_cnt,
-                      &g_pct, &g_e, &pool_e, &pool_i, &gkey, &gstate, &gfirst, &gowner, &sel, &spos, &scnt, &mixed})
+                      &slot_key, &fcnt, &slot_pct, &slot_used, &pct, &counts, &pcls, &ecls,
+                      &cstart, &tiles, &mixed, &g_pts, &g_cnt, &g_pct, &g_e, &pool_e, &pool_i,
+                      &gstate, &gfirst, &gowner, &sel, &spos, &scnt})
       b->release(s);
     points.release(s);
-    gpoints.release(s);
   }
 };
 

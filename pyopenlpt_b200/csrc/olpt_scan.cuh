@@ -1,6 +1,6 @@
 // Device-wide exclusive prefix sum of int32 counts and a CSR builder
-// (count -> scan -> scatter -> per-bucket ascending order), shared by the stereo
-// cell grid, the shake tile bins and the 3D hash grid.  Implementation: scan.cu.
+// (count -> scan -> scatter; the order inside a bucket is arbitrary), shared by the
+// stereo grid and prune, the shake tile bins and the 3D hash grids.  Implementation: scan.cu.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -1138,10 +1138,15 @@ bool prune_select_device(olpt_ctx* ctx, const PruneView& pv, int M, int n_cam,
                          int64_t total_points, char* selected) {
   cudaStream_t s = ctx->stream;
   PruneWork& P = ctx->prune;
-  int G = 0;
-  if (!prune_order_device(P, pv, M, n_cam, total_points, &G, s)) return false;
-  P.sel.ensure((size_t)M + 16, s);
-  if (greedy_device(P, M, G, n_cam, total_points, P.sel.as<uint8_t>(), s)) {
+  prune_device(P, pv, M, n_cam, total_points, s);
+  int cnt[PC_N];
+  OLPT_CUDA(cudaMemcpyAsync(cnt, P.counts.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+  OLPT_CUDA(cudaMemcpyAsync(&P.n_sel, P.spos.as<int>() + M, sizeof(int), cudaMemcpyDeviceToHost,
+                            s));
+  OLPT_CUDA(cudaStreamSynchronize(s));
+  if (cnt[PC_FLAG]) return false;
+  const int G = cnt[PC_BOTH];
+  if (!cnt[PC_REPLACE]) {
     if (selected && M > 0) {
       OLPT_CUDA(cudaMemcpyAsync(selected, P.sel.p, (size_t)M, cudaMemcpyDeviceToHost, s));
       OLPT_CUDA(cudaStreamSynchronize(s));
@@ -1177,6 +1182,9 @@ bool prune_select_device(olpt_ctx* ctx, const PruneView& pv, int M, int n_cam,
     OLPT_CUDA(cudaStreamSynchronize(s));
   }
   if (selected) std::copy(flags.begin(), flags.end(), selected);
+  count_selected(P, M, s);
+  P.n_sel = 0;
+  for (int i = 0; i < G; ++i) P.n_sel += sel[i] ? 1 : 0;
   return true;
 }
 
@@ -1469,11 +1477,6 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
   prune_candidates(res, counts, active);
 }
 
-__global__ void sel_count_kernel(const uint8_t* sel, int M, int* f) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < M) f[i] = sel[i] ? 1 : 0;
-}
-
 __global__ void sel_gather_kernel(const uint8_t* sel, const int* pos, int M, const double* X,
                                   double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1513,15 +1516,7 @@ int64_t stereo_objects(olpt_ctx* ctx, const StereoResult& r) {
   if (r.on_device) {
     PruneWork& P = ctx->prune;
     const int M = (int)r.M;
-    P.spos.ensure((size_t)(M + 1) * sizeof(int), s);
-    P.scnt.ensure((size_t)(M + 1) * sizeof(int), s);
-    if (M > 0)
-      sel_count_kernel<<<OLPT_G(nblk(M)), 256, 0, s>>>(P.sel.as<uint8_t>(), M, P.scnt.as<int>());
-    exclusive_scan(P.scnt.as<int>(), M, P.spos.as<int>(), P.scan_tmp, s);
-    int total = 0;
-    OLPT_CUDA(cudaMemcpyAsync(&total, P.spos.as<int>() + M, sizeof(int), cudaMemcpyDeviceToHost, s));
-    OLPT_CUDA(cudaStreamSynchronize(s));
-    n = total;
+    n = P.n_sel;
     ctx->obj.ensure(std::max<int64_t>(n, 1), ctx->n_cam, s);
     ctx->obj.n = n;
     if (n > 0)
