@@ -1378,13 +1378,20 @@ olpt_status_t olpt_mlp_forward(olpt_ctx* ctx, int64_t n, const float* x, float* 
       OLPT_CUDA(cudaMemcpyAsync(W.xin.p, x, (size_t)n * ctx->mlp.dims.in * 4, cudaMemcpyHostToDevice, s));
       dx = W.xin.as<float>();
     }
-    W.x.ensure((size_t)n * ctx->mlp.dims.in_pad * 2, s);
-    W.o.ensure((size_t)n * kMlpOut * 4, s);
-    mlp_input_device(ctx, dx, n, W.x.as<__nv_bfloat16>());
-    mlp_infer_device(ctx, W.x.as<__nv_bfloat16>(), n, W.o.as<float>());
-    OLPT_CUDA(cudaMemcpyAsync(out, W.o.p, (size_t)n * kMlpOut * 4,
-                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
-    OLPT_CUDA(cudaStreamSynchronize(s));
+    // rows are written while others are read: a result over the input goes through a buffer
+    const float *x1 = x + n * ctx->mlp.dims.in, *o1 = out + n * kMlpOut;
+    const bool direct = on_device && (out >= x1 || o1 <= x);
+    float* o = out;
+    if (!direct) {
+      W.o.ensure((size_t)n * kMlpOut * 4, s);
+      o = W.o.as<float>();
+    }
+    mlp_infer_device(ctx, dx, nullptr, n, o);
+    if (!direct) {
+      OLPT_CUDA(cudaMemcpyAsync(out, o, (size_t)n * kMlpOut * 4,
+                                on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
+      OLPT_CUDA(cudaStreamSynchronize(s));
+    }
   });
 }
 

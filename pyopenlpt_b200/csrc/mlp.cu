@@ -316,7 +316,7 @@ __global__ void features_kernel(const CamDev* cams, OtfView otf, const double* x
 }
 
 // ---------------------------------------------------------------- host helpers
-void ensure_batch(olpt_ctx* ctx, int64_t n, bool training) {
+void ensure_batch(olpt_ctx* ctx, int64_t n) {
   MlpWork& W = ctx->mlp;
   const MlpDims& D = W.dims;
   cudaStream_t s = ctx->stream;
@@ -329,7 +329,6 @@ void ensure_batch(olpt_ctx* ctx, int64_t n, bool training) {
   W.h3.ensure(hb * 2, s);
   W.o.ensure((size_t)m * kMlpOut * 4, s);
   W.err.ensure(16, s);
-  if (!training) return;
   W.xin.ensure((size_t)m * D.in * 4, s);
   W.tgt.ensure((size_t)m * kMlpOut * 4, s);
   W.xt.ensure((size_t)D.in_pad * lt * 2, s);
@@ -378,9 +377,9 @@ int check_err(olpt_ctx* ctx) {
   return e;
 }
 
-// forward of the three hidden layers; with training, also the f32 pre-activations
-// and the transposed activations for the weight gradients
-void forward(olpt_ctx* ctx, int64_t n, bool training) {
+// forward of a training batch: the three hidden layers with their f32 pre-activations and
+// the transposed activations for the weight gradients (inference: mlp_fused.cu)
+void forward(olpt_ctx* ctx, int64_t n) {
   MlpWork& W = ctx->mlp;
   const MlpDims& D = W.dims;
   cudaStream_t s = ctx->stream;
@@ -392,21 +391,17 @@ void forward(olpt_ctx* ctx, int64_t n, bool training) {
   e1.gelu = true;
   e1.out_bf16 = W.h1.as<__nv_bfloat16>();
   e1.ld_bf16 = kMlpHid;
-  if (training) {
-    e1.out_f32 = W.z1.as<float>();
-    e1.ld_f32 = kMlpHid;
-    e1.out_bf16_t = W.h1t.as<__nv_bfloat16>();
-    e1.ld_t = lt;
-  }
+  e1.out_f32 = W.z1.as<float>();
+  e1.ld_f32 = kMlpHid;
+  e1.out_bf16_t = W.h1t.as<__nv_bfloat16>();
+  e1.ld_t = lt;
   gemm_bf16(W.x.as<__nv_bfloat16>(), D.in_pad, W.wb1.as<__nv_bfloat16>(), D.in_pad, (int)n,
             kMlpHid, D.in_pad, e1, 1, err, s);
   GemmEpilogue e2 = e1;
   e2.bias = M + D.off_b2;
   e2.out_bf16 = W.h2.as<__nv_bfloat16>();
-  if (training) {
-    e2.out_f32 = W.z2.as<float>();
-    e2.out_bf16_t = W.h2t.as<__nv_bfloat16>();
-  }
+  e2.out_f32 = W.z2.as<float>();
+  e2.out_bf16_t = W.h2t.as<__nv_bfloat16>();
   gemm_bf16(W.h1.as<__nv_bfloat16>(), kMlpHid, W.wb2.as<__nv_bfloat16>(), kMlpHid, (int)n, kMlpHid,
             kMlpHid, e2, 1, err, s);
   GemmEpilogue e3;
@@ -414,10 +409,8 @@ void forward(olpt_ctx* ctx, int64_t n, bool training) {
   e3.gelu = true;
   e3.out_bf16 = W.h3.as<__nv_bfloat16>();
   e3.ld_bf16 = kMlpHid;
-  if (training) {
-    e3.out_f32 = W.z3.as<float>();
-    e3.ld_f32 = kMlpHid;
-  }
+  e3.out_f32 = W.z3.as<float>();
+  e3.ld_f32 = kMlpHid;
   gemm_bf16(W.h2.as<__nv_bfloat16>(), kMlpHid, W.wb3.as<__nv_bfloat16>(), kMlpHid, (int)n, kMlpHid,
             kMlpHid, e3, 1, err, s);
   head_fwd_kernel<<<OLPT_G(nblk(n * 32)), 256, 0, s>>>(W.h3.as<__nv_bfloat16>(), n, M + D.off_w4,
@@ -556,26 +549,14 @@ void gelu_inplace_device(float* p, int64_t n, cudaStream_t s) {
   OLPT_CUDA(cudaGetLastError());
 }
 
-void mlp_input_device(olpt_ctx* ctx, const float* x_f32, int64_t n, __nv_bfloat16* x) {
-  if (n == 0) return;
-  const MlpDims& D = ctx->mlp.dims;
-  input_kernel<<<OLPT_G(nblk(n * D.in_pad)), 256, 0, ctx->stream>>>(x_f32, n, D.in, D.in_pad, x);
-  OLPT_CUDA(cudaGetLastError());
-}
-
-void mlp_infer_device(olpt_ctx* ctx, const __nv_bfloat16* x, int64_t n, float* o) {
+void mlp_infer_device(olpt_ctx* ctx, const float* x_f32, const __nv_bfloat16* x, int64_t n,
+                      float* o) {
   MlpWork& W = ctx->mlp;
   OLPT_REQUIRE(W.ready, OLPT_ERR_INVALID_ARG, "network not initialised");
   if (n == 0) return;
-  cudaStream_t s = ctx->stream;
-  ensure_batch(ctx, n, false);
-  OLPT_CUDA(cudaMemsetAsync(W.err.p, 0, 16, s));
-  if (x != W.x.as<__nv_bfloat16>())
-    OLPT_CUDA(cudaMemcpyAsync(W.x.p, x, (size_t)n * W.dims.in_pad * 2, cudaMemcpyDeviceToDevice,
-                              s));
-  forward(ctx, n, false);
-  if (o != W.o.as<float>())
-    OLPT_CUDA(cudaMemcpyAsync(o, W.o.p, (size_t)n * kMlpOut * 4, cudaMemcpyDeviceToDevice, s));
+  W.err.ensure(16, ctx->stream);
+  OLPT_CUDA(cudaMemsetAsync(W.err.p, 0, 16, ctx->stream));
+  mlp_fused_forward(ctx, x_f32, x, n, o);
   check_err(ctx);
 }
 
@@ -590,7 +571,7 @@ double mlp_train_device(olpt_ctx* ctx, const float* x_f32, const float* tgt, int
                         double ghost_weight, bool update) {
   OLPT_REQUIRE(ctx->mlp.ready, OLPT_ERR_INVALID_ARG, "network not initialised");
   OLPT_REQUIRE(n > 0, OLPT_ERR_INVALID_ARG, "empty batch");
-  ensure_batch(ctx, n, true);
+  ensure_batch(ctx, n);
   OLPT_CUDA(cudaMemsetAsync(ctx->mlp.err.p, 0, 16, ctx->stream));
   const double* d_loss = train_enqueue(ctx, x_f32, tgt, n, lr, ghost_weight, update);
   double loss = 0.0;
@@ -607,7 +588,7 @@ const double* train_enqueue(olpt_ctx* ctx, const float* x_f32, const float* tgt,
   OLPT_REQUIRE(n > 0, OLPT_ERR_INVALID_ARG, "empty batch");
   cudaStream_t s = ctx->stream;
   const MlpDims& D = W.dims;
-  ensure_batch(ctx, n, true);
+  ensure_batch(ctx, n);
   const int64_t lt = round8(n);
   input_kernel<<<OLPT_G(nblk(n * D.in_pad)), 256, 0, s>>>(x_f32, n, D.in, D.in_pad,
                                                           W.x.as<__nv_bfloat16>());
@@ -616,7 +597,7 @@ const double* train_enqueue(olpt_ctx* ctx, const float* x_f32, const float* tgt,
     transpose_kernel<<<OLPT_G(g), dim3(32, 8), 0, s>>>(W.x.as<__nv_bfloat16>(), n, D.in_pad,
                                                        D.in_pad, W.xt.as<__nv_bfloat16>(), lt);
   }
-  forward(ctx, n, true);
+  forward(ctx, n);
   float* G = W.grad.as<float>();
   const float* M = W.master.as<float>();
   // loss and head
@@ -698,7 +679,7 @@ void mlp_train_many(olpt_ctx* ctx, const float* x, const float* t, int64_t n, in
   W.tgt.ensure((size_t)batch * kMlpOut * 4, s);
   // the steps are enqueued back to back; the losses stay on the device until the end
   W.loss_hist.ensure((size_t)(steps + 1) * sizeof(double), s);
-  ensure_batch(ctx, batch, true);
+  ensure_batch(ctx, batch);
   OLPT_CUDA(cudaMemsetAsync(W.err.p, 0, 16, s));
   for (int it = 0; it < steps; ++it) {
     const double a = lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(M_PI * it / (double)steps)));

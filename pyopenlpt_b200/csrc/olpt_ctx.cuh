@@ -358,14 +358,17 @@ void mlp_get_params(olpt_ctx* ctx, float* host);
 // them (FP32 or FP64 planes per sp.precision); x: n x dims.in_pad bf16 (device),
 // f32 (optional, device): n x dims.in
 void mlp_features_device(olpt_ctx* ctx, const ShakeParams& sp, __nv_bfloat16* x, float* f32);
-// f32 rows of dims.in (device) -> bf16 rows of dims.in_pad
-void mlp_input_device(olpt_ctx* ctx, const float* x_f32, int64_t n, __nv_bfloat16* x);
 void gelu_inplace_device(float* p, int64_t n, cudaStream_t s);
 // residual planes of the current images with every object projected (the first step
 // of a shake iteration)
 void residual_all_device(olpt_ctx* ctx, const ShakeParams& sp);
-// o (device, n x 4) = network(x)
-void mlp_infer_device(olpt_ctx* ctx, const __nv_bfloat16* x, int64_t n, float* o);
+// o (device, n x 4) = network(x), for f32 rows of dims.in or bf16 rows of dims.in_pad (device;
+// the other one null); waits for the result
+void mlp_infer_device(olpt_ctx* ctx, const float* x_f32, const __nv_bfloat16* x, int64_t n,
+                      float* o);
+// the same enqueued in one kernel (mlp_fused.cu); MlpWork::err reports a timed-out wait
+void mlp_fused_forward(olpt_ctx* ctx, const float* x_f32, const __nv_bfloat16* x, int64_t n,
+                       float* o);
 // one training batch: loss (mean), gradients into MlpWork::grad, Adam update when lr > 0
 double mlp_train_device(olpt_ctx* ctx, const float* x_f32, const float* tgt, int64_t n, double lr,
                         double ghost_weight, bool update);

@@ -1499,7 +1499,7 @@ static void learned_impl(olpt_ctx* ctx, const ShakeParams& sp) {
     M.x.ensure((size_t)n * M.dims.in_pad * 2, s);
     mlp_features_device(ctx, sp, M.x.as<__nv_bfloat16>(), nullptr);
     M.o.ensure((size_t)n * kMlpOut * 4, s);
-    mlp_infer_device(ctx, M.x.as<__nv_bfloat16>(), n, M.o.as<float>());
+    mlp_infer_device(ctx, nullptr, M.x.as<__nv_bfloat16>(), n, M.o.as<float>());
     // 2. correction, and the network's ghosts leave before any shaking
     M.keep.ensure((size_t)(n + 1) * sizeof(int), s);
     M.pos.ensure((size_t)(n + 1) * sizeof(int), s);
