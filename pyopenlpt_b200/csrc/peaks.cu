@@ -43,6 +43,7 @@ namespace olpt {
 namespace {
 
 constexpr int kPeakThreads = 256;
+constexpr int kBandChunks = 512;  // two-pass detector: 16-byte chunks a band
 
 struct PeakCam {
   const unsigned char* img;
@@ -61,10 +62,27 @@ struct PeakArgs {
   int n_cam;
   PeakCam cam[OLPT_MAX_CAM];
   double min_int;
+  int min_level;      // integer images: v < min_level  <=>  (double)v < min_int
   const double* lut;  // integer images only
   int* band_counts;
   const int64_t* band_offsets;
 };
+
+// levels are 0 .. 65535: NaN or <= 0 rejects none, above 65535 rejects all
+int min_level_of(double min_int) {
+  return !(min_int > 0.0) ? 0 : min_int > 65535.0 ? 65536 : (int)std::ceil(min_int);
+}
+
+// Threshold test of one pixel: (double)v < min_int, for integer levels as the integer
+// compare v < min_level (the same outcome for every level and every min_int).
+template <typename T>
+__device__ __forceinline__ bool below(T v, double min_int, int min_level) {
+  if constexpr (std::is_integral<T>::value) {
+    return (int)v < min_level;
+  } else {
+    return (double)v < min_int;
+  }
+}
 
 template <typename T>
 struct Ln;
@@ -121,18 +139,29 @@ __device__ __forceinline__ bool fit3(double l1, double l2, double l3, int p, dou
   return true;
 }
 
-// Evaluate one chunk; returns a bitmask of detections (bit j = pixel c0 + j) and
-// fills xs/ys for them when EMIT.
-template <typename T, int N, bool EMIT>
-__device__ __forceinline__ unsigned eval_chunk(const PeakCam& c, const PeakArgs& a, int r, int c0,
-                                               double (&xs)[N], double (&ys)[N]) {
+// The two fits of the detection at (r, col).
+template <typename T>
+__device__ __forceinline__ bool fit_at(const PeakCam& c, const double* lut, int r, int col,
+                                       double& x, double& y) {
+  const T* row = reinterpret_cast<const T*>(c.img + (int64_t)r * c.pitch);
+  const T* up = reinterpret_cast<const T*>(c.img + (int64_t)(r - 1) * c.pitch);
+  const T* dn = reinterpret_cast<const T*>(c.img + (int64_t)(r + 1) * c.pitch);
+  const double l = Ln<T>::f(__ldg(row + col - 1), lut), m = Ln<T>::f(__ldg(row + col), lut),
+               h = Ln<T>::f(__ldg(row + col + 1), lut), u = Ln<T>::f(__ldg(up + col), lut),
+               d = Ln<T>::f(__ldg(dn + col), lut);
+  return fit3(l, m, h, col, x) && fit3(u, m, d, r, y);
+}
+
+// Evaluate one chunk; returns a bitmask of detections (bit j = pixel c0 + j).
+template <typename T, int N>
+__device__ __forceinline__ unsigned eval_chunk(const PeakCam& c, const PeakArgs& a, int r, int c0) {
   if (r < 1 || r > c.H - 2) return 0u;
   T cen[N];
   load_chunk<T, N>(c, r, c0, cen);
   // quick reject: nothing in the chunk reaches the threshold
   bool any = false;
 #pragma unroll
-  for (int j = 0; j < N; ++j) any |= !((double)cen[j] < a.min_int);
+  for (int j = 0; j < N; ++j) any |= !below<T>(cen[j], a.min_int, a.min_level);
   if (!any) return 0u;
   T up[N], dn[N];
   load_chunk<T, N>(c, r - 1, c0, up);
@@ -140,26 +169,27 @@ __device__ __forceinline__ unsigned eval_chunk(const PeakCam& c, const PeakArgs&
   const T* row = reinterpret_cast<const T*>(c.img + (int64_t)r * c.pitch);
   const T left = (c0 > 0) ? __ldg(row + c0 - 1) : T(0);
   const T right = (c0 + N < c.W) ? __ldg(row + c0 + N) : T(0);
-  unsigned mask = 0u;
+  unsigned cand = 0u;
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     const int col = c0 + j;
     if (col < 1 || col > c.W - 2) continue;
     const T v = cen[j];
-    if ((double)v < a.min_int) continue;
+    if (below<T>(v, a.min_int, a.min_level)) continue;
     const T l = (j > 0) ? cen[j - 1] : left;
     const T rr = (j < N - 1) ? cen[j + 1] : right;
     // isLocalMax tie rule: up/left reject if strictly greater, down/right if >=.
     if (up[j] > v || l > v || dn[j] >= v || rr >= v) continue;
-    const double lc = Ln<T>::f(v, a.lut);
-    double xc, yc;
-    if (!fit3(Ln<T>::f(l, a.lut), lc, Ln<T>::f(rr, a.lut), col, xc)) continue;
-    if (!fit3(Ln<T>::f(up[j], a.lut), lc, Ln<T>::f(dn[j], a.lut), r, yc)) continue;
-    if (EMIT) {
-      xs[j] = xc;
-      ys[j] = yc;
-    }
-    mask |= 1u << j;
+    cand |= 1u << j;
+  }
+  // integer levels: a local maximum always has a finite centre (see mask_staged)
+  if constexpr (std::is_integral<T>::value) return cand;
+  unsigned mask = 0u;
+  while (cand) {
+    const int j = __ffs(cand) - 1;
+    cand &= cand - 1;
+    double x, y;
+    if (fit_at<T>(c, a.lut, r, c0 + j, x, y)) mask |= 1u << j;
   }
   return mask;
 }
@@ -171,6 +201,11 @@ __device__ __forceinline__ int find_cam(const PeakArgs& a, int blk) {
   return cam;
 }
 
+// One band: COUNT leaves its number of detections; EMIT lists them in raster order in shared
+// memory (256 chunks at a time), fits them one per thread and stores coalesced.  Bands of 512
+// chunks: 2048^2 u16 makes 1,024 blocks where bands of 2,048 made 256, fewer than two a SM,
+// and the fits ran on the few lanes of a warp that held a detection, for each of the chunk's
+// pixels in turn (400,000 spots: 84 us a call before, 27 us with these bands).
 template <typename T, bool EMIT>
 __global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
   constexpr int N = 16 / sizeof(T);
@@ -184,21 +219,19 @@ __global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
   const int total = rows * cpr;
 
   __shared__ int warp_sums[kPeakThreads / 32];
-  __shared__ int s_base;
-  int64_t base = 0;
-  if (EMIT) base = a.band_offsets[blockIdx.x];
-  int running = 0;
-  int count = 0;
+  // 4-neighbour maxima: at most half the pixels of 256 chunks
+  __shared__ uint32_t list[EMIT ? kPeakThreads * N / 2 : 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int64_t base = EMIT ? a.band_offsets[blockIdx.x] : 0;
+  int count = 0;
   for (int start = 0; start < total; start += kPeakThreads) {
     const int i = start + threadIdx.x;
-    double xs[N], ys[N];
     unsigned mask = 0u;
-    int r = 0, c0 = 0;
+    int lr = 0, c0 = 0;
     if (i < total) {
-      r = r0 + i / cpr;
-      c0 = (i % cpr) * N;
-      mask = eval_chunk<T, N, EMIT>(c, a, r, c0, xs, ys);
+      lr = i / cpr;
+      c0 = (i - lr * cpr) * N;
+      mask = eval_chunk<T, N>(c, a, r0 + lr, c0);
     }
     const int n = __popc(mask);
     if (!EMIT) {
@@ -214,35 +247,33 @@ __global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
     }
     if (lane == 31) warp_sums[wid] = incl;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int acc = 0;
-      for (int w = 0; w < kPeakThreads / 32; ++w) {
-        int t = warp_sums[w];
-        warp_sums[w] = acc;
-        acc += t;
-      }
-      s_base = acc;
+    int before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kPeakThreads / 32; ++w) {
+      before += w < wid ? warp_sums[w] : 0;
+      all += warp_sums[w];
+    }
+    int pos = before + incl - n;
+    while (mask) {
+      const int j = __ffs(mask) - 1;
+      mask &= mask - 1;
+      list[pos++] = (uint32_t)(lr * cpr * N + c0 + j);  // pixel of the band, rows padded
     }
     __syncthreads();
-    int pos = running + warp_sums[wid] + incl - n;
-    if (mask) {
-      for (int j = 0; j < N; ++j) {
-        if (mask & (1u << j)) {
-          const int64_t o = base + pos;
-          c.x[o] = xs[j];
-          c.y[o] = ys[j];
-          c.rc[o] = make_int2(r, c0 + j);
-          ++pos;
-        }
-      }
+    for (int k = threadIdx.x; k < all; k += kPeakThreads) {
+      const int p = (int)list[k], lrow = p / (cpr * N);
+      const int r = r0 + lrow, col = p - lrow * cpr * N;
+      double x, y;
+      fit_at<T>(c, a.lut, r, col, x, y);
+      c.x[base + k] = x;
+      c.y[base + k] = y;
+      c.rc[base + k] = make_int2(r, col);
     }
-    running += s_base;
+    base += all;
     __syncthreads();
   }
   if (!EMIT) {
-    // block reduction of count
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) count += __shfl_down_sync(0xffffffffu, count, o);
+    count = __reduce_add_sync(0xffffffffu, count);
     if (lane == 0) warp_sums[wid] = count;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -254,41 +285,38 @@ __global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
 }
 
 // Per-camera exclusive scan of band counts -> band offsets, and totals.
-__global__ void band_scan_kernel(const PeakArgs a, int64_t* band_offsets, int64_t* totals) {
+__global__ void __launch_bounds__(1024) band_scan_kernel(const PeakArgs a, int64_t* band_offsets,
+                                                         int64_t* totals) {
   const int cam = blockIdx.x;
   if (cam >= a.n_cam) return;
   const PeakCam& c = a.cam[cam];
-  __shared__ int64_t s_run, s_total;
   __shared__ int64_t warp_sums[32];
-  if (threadIdx.x == 0) s_run = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int s = 0; s < c.n_bands; s += blockDim.x) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int64_t run = 0;
+  for (int s = 0; s < c.n_bands; s += 1024) {
     const int b = s + threadIdx.x;
-    int64_t v = (b < c.n_bands && c.active) ? a.band_counts[c.band_base + b] : 0;
+    const int64_t v = (b < c.n_bands && c.active) ? a.band_counts[c.band_base + b] : 0;
     int64_t incl = v;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       int64_t t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
     if (lane == 31) warp_sums[wid] = incl;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int64_t acc = 0;
-      for (int w = 0; w < nw; ++w) {
-        int64_t t = warp_sums[w];
-        warp_sums[w] = acc;
-        acc += t;
-      }
-      s_total = acc;
+    int64_t w = warp_sums[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      int64_t t = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += t;
     }
-    __syncthreads();
-    if (b < c.n_bands) band_offsets[c.band_base + b] = s_run + warp_sums[wid] + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 0) s_run += s_total;
+    const int64_t before = __shfl_sync(0xffffffffu, w, wid > 0 ? wid - 1 : 0);
+    const int64_t all = __shfl_sync(0xffffffffu, w, 31);
+    if (b < c.n_bands) band_offsets[c.band_base + b] = run + (wid > 0 ? before : 0) + incl - v;
+    run += all;
     __syncthreads();
   }
-  if (threadIdx.x == 0) totals[cam] = s_run;
+  if (threadIdx.x == 0) totals[cam] = run;
 }
 
 template <typename T>
@@ -296,7 +324,7 @@ void launch_peaks(const PeakArgs& a, int n_blocks, int64_t* band_offsets, int64_
                   cudaStream_t s) {
   peaks_kernel<T, false><<<OLPT_G(n_blocks), kPeakThreads, 0, s>>>(a);
   OLPT_CUDA(cudaGetLastError());
-  band_scan_kernel<<<OLPT_G(a.n_cam), 256, 0, s>>>(a, band_offsets, totals);
+  band_scan_kernel<<<OLPT_G(a.n_cam), 1024, 0, s>>>(a, band_offsets, totals);
   OLPT_CUDA(cudaGetLastError());
   PeakArgs b = a;
   b.band_offsets = band_offsets;
@@ -365,17 +393,6 @@ __device__ __forceinline__ int tile_index(const DetCam& c, int box_h, int lr, in
 // One chunk of image row r (tile row lr) from shared memory: bit j set if pixel c0 + j
 // passes eval_chunk's tests and fit.  Pixels at or past W are the TMA's zero fill, as
 // eval_chunk's loads.
-// Threshold test of one pixel: (double)v < min_int, for integer levels as the integer
-// compare v < min_level (the same outcome for every level and every min_int).
-template <typename T>
-__device__ __forceinline__ bool below(T v, double min_int, int min_level) {
-  if constexpr (std::is_integral<T>::value) {
-    return (int)v < min_level;
-  } else {
-    return (double)v < min_int;
-  }
-}
-
 template <typename T, int N>
 __device__ __forceinline__ unsigned mask_staged(const T* tile, const DetCam& c, int box_h,
                                                 double min_int, int min_level, const double* lut,
@@ -870,8 +887,7 @@ void find_peaks_device(olpt_ctx* ctx, double min_int, bool sync_counts) {
     DetArgs a{};
     a.n_cam = ctx->n_cam;
     a.min_int = min_int;
-    // levels are 0 .. 65535: NaN or <= 0 rejects none, above 65535 rejects all
-    a.min_level = !(min_int > 0.0) ? 0 : min_int > 65535.0 ? 65536 : (int)std::ceil(min_int);
+    a.min_level = min_level_of(min_int);
     a.lut = lut;
     int blocks = 0;
     for (int c = 0; c < ctx->n_cam; ++c) {
@@ -933,6 +949,7 @@ void find_peaks_device(olpt_ctx* ctx, double min_int, bool sync_counts) {
     PeakArgs a{};
     a.n_cam = ctx->n_cam;
     a.min_int = min_int;
+    a.min_level = min_level_of(min_int);
     a.lut = lut;
     int blocks = 0;
     for (int c = 0; c < ctx->n_cam; ++c) {
@@ -944,7 +961,7 @@ void find_peaks_device(olpt_ctx* ctx, double min_int, bool sync_counts) {
       pc.pitch = im.pitch;
       pc.H = im.H;
       pc.W = im.W;
-      pc.band_rows = std::max(1, (2048 + cpr - 1) / cpr);
+      pc.band_rows = std::max(1, kBandChunks / cpr);
       pc.n_bands = (im.H + pc.band_rows - 1) / pc.band_rows;
       pc.band_base = blocks;
       pc.active = ctx->cams_h[c].is_active;
@@ -1113,11 +1130,11 @@ olpt_status_t olpt_find_peaks_noalloc(const void* d_img, olpt_dtype_t dtype, int
   try {
     const int N = 16 / esz;
     const int cpr = (W + N - 1) / N;
-    int band_rows = (2048 + cpr - 1) / cpr;
-    if (band_rows < 1) band_rows = 1;
+    const int band_rows = std::max(1, kBandChunks / cpr);
     PeakArgs a{};
     a.n_cam = 1;
     a.min_int = min_obj_int;
+    a.min_level = min_level_of(min_obj_int);
     PeakCam& pc = a.cam[0];
     pc.img = static_cast<const unsigned char*>(d_img);
     pc.pitch = pitch_bytes;
