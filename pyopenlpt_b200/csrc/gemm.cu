@@ -38,9 +38,8 @@ constexpr size_t smem_bytes() {
 }
 
 template <int BN>
-__global__ void __launch_bounds__(256, 1)
-    gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     EpiArgs g) {
+__device__ __forceinline__ void gemm_tile(const CUtensorMap& tmA, const CUtensorMap& tmB,
+                                          const EpiArgs& g, int bx, int by, int bz) {
   using namespace umma;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -52,9 +51,9 @@ __global__ void __launch_bounds__(256, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
+  const int m0 = bx * kBM, n0 = by * BN;
   const int KT = (g.K + kBK - 1) / kBK;
-  const int kt0 = blockIdx.z * g.kt_per_split;
+  const int kt0 = bz * g.kt_per_split;
   const int nk = max(0, min(KT, kt0 + g.kt_per_split) - kt0);
 
   if (threadIdx.x == 0) {
@@ -118,6 +117,9 @@ __global__ void __launch_bounds__(256, 1)
   const bool row_ok = row < g.M;
   const GemmEpilogue& e = g.e;
   const bool partial = g.splits > 1;
+  // column sums of the tile (bias gradients): per warp over its 32 rows, then the four
+  // row quarters in order
+  __shared__ float s_col[4][BN];
   for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 16) {
     float v[16];
     if (have) {
@@ -126,11 +128,32 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = 0.0f;
     }
+    if (e.colsum) {
+      float t[16];
+      const float* pp = e.gelu_pre + (size_t)row * e.ld_pre + n0 + c;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        if (row_ok && n0 + c + j < g.N) v[j] *= gelu_grad_f(pp[j]);
+        t[j] = row_ok ? v[j] : 0.0f;
+      }
+      // lanes l and l ^ o halve the columns between them: lane l ends with column l & 15
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int j = 0; j < o; ++j) {
+          const float keep = up ? t[j + o] : t[j], give = up ? t[j] : t[j + o];
+          t[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+      t[0] += __shfl_xor_sync(0xffffffffu, t[0], 16);
+      if (lane < 16) s_col[quarter][c + lane] = t[0];
+    }
     if (!row_ok || n0 + c >= g.N) continue;
     const int nb = n0 + c;
     const int nv = min(16, g.N - nb);
     if (partial) {
-      float* o = e.out_f32 + (size_t)blockIdx.z * g.M * e.ld_f32 + (size_t)row * e.ld_f32 + nb;
+      float* o = e.out_f32 + (size_t)bz * g.M * e.ld_f32 + (size_t)row * e.ld_f32 + nb;
       if (nv == 16 && ((uintptr_t)o & 15) == 0) {
 #pragma unroll
         for (int q = 0; q < 4; ++q)
@@ -147,7 +170,7 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] += e.bias[nb + j];
       }
-      if (e.gelu_pre) {
+      if (e.gelu_pre && !e.colsum) {
         const float* pp = e.gelu_pre + (size_t)row * e.ld_pre + nb;
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] *= gelu_grad_f(pp[j]);
@@ -195,7 +218,7 @@ __global__ void __launch_bounds__(256, 1)
       const int n = nb + j;
       float x = v[j];
       if (e.bias) x += e.bias[n];
-      if (e.gelu_pre) x *= gelu_grad_f(e.gelu_pre[(size_t)row * e.ld_pre + n]);
+      if (e.gelu_pre && !e.colsum) x *= gelu_grad_f(e.gelu_pre[(size_t)row * e.ld_pre + n]);
       if (e.out_f32) e.out_f32[(size_t)row * e.ld_f32 + n] = x;
       if (e.gelu) x = gelu_f(x);
       if (e.out_bf16) e.out_bf16[(size_t)row * e.ld_bf16 + n] = __float2bfloat16_rn(x);
@@ -205,7 +228,36 @@ __global__ void __launch_bounds__(256, 1)
 
   fence_before_sync();
   __syncthreads();
+  if (e.colsum)
+    for (int c = threadIdx.x; c < BN && n0 + c < g.N; c += blockDim.x)
+      e.colsum[(size_t)bx * g.N + n0 + c] =
+          s_col[0][c] + s_col[1][c] + s_col[2][c] + s_col[3][c];
   if (warp == 0) tmem_dealloc(tmem, BN);
+}
+
+template <int BN>
+__global__ void __launch_bounds__(256, 1)
+    gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ EpiArgs g) {
+  gemm_tile<BN>(tmA, tmB, g, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// Several split-K GEMMs in one launch: block ranges in order, per problem output tiles fastest,
+// then splits.
+struct GroupArgs {
+  CUtensorMap a[kGemmGroup], b[kGemmGroup];
+  EpiArgs g[kGemmGroup];
+  int first[kGemmGroup + 1];
+  int n;
+};
+
+__global__ void __launch_bounds__(256, 1) gemm_group_kernel(const __grid_constant__ GroupArgs q) {
+  int k = 0;
+  for (int i = 1; i < q.n; ++i)
+    if ((int)blockIdx.x >= q.first[i]) k = i;
+  const int t = blockIdx.x - q.first[k];
+  const int mt = (q.g[k].M + kBM - 1) / kBM, nt = (q.g[k].N + 127) / 128;
+  gemm_tile<128>(q.a[k], q.b[k], q.g[k], t % mt, t / mt % nt, t / (mt * nt));
 }
 
 // rows x cols bf16 (row stride ld elements), box box_rows x 64, 128-byte swizzle
@@ -272,6 +324,43 @@ void gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
     const CUtensorMap tb = tile_map(B, N, K, ldb, 128);
     launch<128>(ta, tb, g, dim3(mt, (N + 127) / 128, splits), s);
   }
+}
+
+int gemm_splits(int K, int splits, int* kt_per_split) {
+  const int KT = (K + kBK - 1) / kBK;
+  splits = std::max(1, std::min(splits, KT));
+  *kt_per_split = (KT + splits - 1) / splits;
+  return (KT + *kt_per_split - 1) / *kt_per_split;  // every split has at least one k tile
+}
+
+void gemm_bf16_group(const GemmProblem* p, int n, int* err, cudaStream_t s) {
+  OLPT_REQUIRE(n >= 1 && n <= kGemmGroup, OLPT_ERR_INVALID_ARG, "gemm group: bad size");
+  GroupArgs q{};
+  q.n = n;
+  int blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    const GemmProblem& r = p[i];
+    OLPT_REQUIRE(r.M > 0 && r.N > 0 && r.K > 0 && r.lda % 8 == 0 && r.ldb % 8 == 0 &&
+                     r.lda >= r.K && r.ldb >= r.K && ((uintptr_t)r.A % 16) == 0 &&
+                     ((uintptr_t)r.B % 16) == 0 && r.part,
+                 OLPT_ERR_INVALID_ARG, "gemm group: bad operands");
+    int kps = 0;
+    const int splits = gemm_splits(r.K, r.splits, &kps);
+    GemmEpilogue e;
+    e.out_f32 = r.part;
+    e.ld_f32 = r.ld_part;
+    q.a[i] = tile_map(r.A, r.M, r.K, r.lda, kBM);
+    q.b[i] = tile_map(r.B, r.N, r.K, r.ldb, 128);
+    // a single split is written as a partial too
+    q.g[i] = EpiArgs{r.M, r.N, e, err, kps, r.K, std::max(splits, 2)};
+    q.first[i] = blocks;
+    blocks += ((r.M + kBM - 1) / kBM) * ((r.N + 127) / 128) * splits;
+  }
+  q.first[n] = blocks;
+  OLPT_CUDA(cudaFuncSetAttribute(gemm_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem_bytes<128>()));
+  gemm_group_kernel<<<OLPT_G(blocks), 256, smem_bytes<128>(), s>>>(q);
+  OLPT_CUDA(cudaGetLastError());
 }
 
 }  // namespace olpt

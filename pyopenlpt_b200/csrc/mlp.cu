@@ -41,191 +41,238 @@ __global__ void pack_sq_kernel(const float* w, __nv_bfloat16* wb, __nv_bfloat16*
 }
 
 // ---------------------------------------------------------------- inputs
-// f32 rows of `in` values -> bf16 rows of in_pad (zero padded)
-__global__ void input_kernel(const float* xin, int64_t n, int in, int in_pad, __nv_bfloat16* x) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n * in_pad) return;
-  const int64_t r = i / in_pad;
-  const int c = (int)(i % in_pad);
-  x[i] = __float2bfloat16_rn(c < in ? xin[r * in + c] : 0.0f);
-}
-
-// out[c][r] = in[r][c] for r < rows, c < cols (32 x 32 tiles through shared memory)
-__global__ void transpose_kernel(const __nv_bfloat16* in, int64_t rows, int cols, int ld_in,
-                                 __nv_bfloat16* out, int64_t ld_out) {
-  __shared__ __nv_bfloat16 t[32][33];
-  const int64_t r0 = (int64_t)blockIdx.x * 32;
-  const int c0 = blockIdx.y * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int64_t r = r0 + k;
-    const int c = c0 + threadIdx.x;
-    if (r < rows && c < cols) t[k][threadIdx.x] = in[r * ld_in + c];
+// f32 rows of `in` values -> bf16 rows of in_pad (zero padded) and their transpose (rows of
+// ld_t): 64 x 64 tiles through shared memory, so that both sides move 128 bytes a warp.
+__global__ void __launch_bounds__(256) input_kernel(const float* xin, int64_t n, int in,
+                                                    int in_pad, __nv_bfloat16* x,
+                                                    __nv_bfloat16* xt, int64_t ld_t) {
+  __shared__ __nv_bfloat16 t[64][66];
+  const int64_t r0 = (int64_t)blockIdx.x * 64;
+  const int c0 = blockIdx.y * 64;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int r = w + 8 * k;
+    const float* row = xin + (r0 + r) * in;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = c0 + 32 * h + lane;
+      t[r][32 * h + lane] = __float2bfloat16_rn(r0 + r < n && c < in ? row[c] : 0.0f);
+    }
   }
   __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int c = c0 + k;
-    const int64_t r = r0 + threadIdx.x;
-    if (r < rows && c < cols) out[(int64_t)c * ld_out + r] = t[threadIdx.x][k];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int r = w + 8 * k;
+    if (r0 + r < n)
+      *reinterpret_cast<__nv_bfloat162*>(x + (r0 + r) * in_pad + c0 + 2 * lane) =
+          __nv_bfloat162(t[r][2 * lane], t[r][2 * lane + 1]);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int c = w + 8 * k;
+    const int64_t r = r0 + 2 * lane;
+    __nv_bfloat16* o = xt + (int64_t)(c0 + c) * ld_t + r;
+    if (r + 1 < n)
+      *reinterpret_cast<__nv_bfloat162*>(o) = __nv_bfloat162(t[2 * lane][c], t[2 * lane + 1][c]);
+    else if (r < n)
+      *o = t[2 * lane][c];
   }
 }
 
 // ---------------------------------------------------------------- head (256 -> 4)
-// one warp per row: o = W4 h3 + b4
-__global__ void head_fwd_kernel(const __nv_bfloat16* h3, int64_t n, const float* W4,
-                                const float* b4, float* o) {
-  const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  float acc[kMlpOut] = {0, 0, 0, 0};
-  for (int k = lane; k < kMlpHid; k += 32) {
-    const float h = __bfloat162float(h3[row * kMlpHid + k]);
-#pragma unroll
-    for (int j = 0; j < kMlpOut; ++j) acc[j] += h * W4[j * kMlpHid + k];
-  }
-#pragma unroll
-  for (int j = 0; j < kMlpOut; ++j) {
-    float v = acc[j];
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    acc[j] = v;
-  }
-  if (lane < kMlpOut) o[row * kMlpOut + lane] = acc[lane] + b4[lane];
-}
-
-// loss per row: (1 - ghost) * mean_d (o_d - t_d)^2 + w * BCE(o_3, ghost); dout = dL/do / n.
-// Per-block partial sums of the loss (double) for a fixed-order reduction.
-__global__ void loss_kernel(const float* o, const float* tgt, int64_t n, float w_ghost, float* dout,
-                            double* part) {
-  __shared__ double red[256];
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// One warp per row: o = W4 h3 + b4, the row's loss (1 - ghost) * mean_d (o_d - t_d)^2 +
+// w * BCE(o_3, ghost), and dout = dL/do / n.  Per-block partial sums of the loss (double) for
+// a fixed-order reduction.
+__global__ void __launch_bounds__(256) head_loss_kernel(const __nv_bfloat16* h3, int64_t n,
+                                                        const float* W4, const float* b4,
+                                                        const float* tgt, float w_ghost,
+                                                        float* dout, double* part) {
+  __shared__ double red[8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t row = (int64_t)blockIdx.x * 8 + w;
   double l = 0.0;
-  if (i < n) {
-    const float* oi = o + i * kMlpOut;
-    const float* ti = tgt + i * kMlpOut;
+  if (row < n) {
+    float acc[kMlpOut] = {0, 0, 0, 0};
+    for (int k = lane; k < kMlpHid; k += 32) {
+      const float h = __bfloat162float(h3[row * kMlpHid + k]);
+#pragma unroll
+      for (int j = 0; j < kMlpOut; ++j) acc[j] += h * W4[j * kMlpHid + k];
+    }
+#pragma unroll
+    for (int j = 0; j < kMlpOut; ++j) {
+      float v = acc[j];
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+      acc[j] = v + b4[j];
+    }
+    const float* ti = tgt + row * kMlpOut;
     const float y = ti[3];
     const float pos = 1.0f - y;
     const float inv_n = 1.0f / (float)n;
     float mse = 0.0f;
-    for (int d = 0; d < 3; ++d) {
-      const float e = oi[d] - ti[d];
+    float d[kMlpOut];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const float e = acc[q] - ti[q];
       mse += e * e;
-      dout[i * kMlpOut + d] = pos * (2.0f / 3.0f) * e * inv_n;
+      d[q] = pos * (2.0f / 3.0f) * e * inv_n;
     }
-    const float z = oi[3];
+    const float z = acc[3];
     const float bce = fmaxf(z, 0.0f) - z * y + log1pf(expf(-fabsf(z)));
     const float p = 1.0f / (1.0f + expf(-z));
-    dout[i * kMlpOut + 3] = w_ghost * (p - y) * inv_n;
+    d[3] = w_ghost * (p - y) * inv_n;
     l = (double)(pos * mse / 3.0f + w_ghost * bce);
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < kMlpOut; ++q) dout[row * kMlpOut + q] = d[q];
   }
-  red[threadIdx.x] = l;
+  if (lane == 0) red[w] = l;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int k = 0; k < 8; ++k) t += red[k];
+    part[blockIdx.x] = t;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-__global__ void sum_double_kernel(const double* part, int n, double* out, double scale) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0;
-  for (int i = 0; i < n; ++i) s += part[i];
-  *out = s * scale;
-}
-
-// dZ3 = (dout W4) * gelu'(z3): 32 rows per block, 256 threads (one per column);
-// writes f32 and bf16 rows and the bf16 transpose (ld_t)
-__global__ void head_bwd_kernel(const float* dout, const float* W4, const float* z3, int64_t n,
-                                float* dzf, __nv_bfloat16* dzb, __nv_bfloat16* dzt, int64_t ld_t) {
+// dZ3 = (dout W4) * gelu'(z3) for 32 rows a block, one thread a column: bf16 rows and the bf16
+// transpose (ld_t), and the block's partial sums of dW4 (4 x 256), db4 (4) and db3 (256), from
+// the same pass over dout, h3 and z3.
+constexpr int kHeadPart = kMlpOut * kMlpHid + kMlpOut + kMlpHid;
+__global__ void __launch_bounds__(kMlpHid) head_bwd_kernel(const float* dout, const float* W4,
+                                                           const float* z3,
+                                                           const __nv_bfloat16* h3, int64_t n,
+                                                           __nv_bfloat16* dzb, __nv_bfloat16* dzt,
+                                                           int64_t ld_t, float* partial) {
   __shared__ __nv_bfloat16 tile[32][kMlpHid + 8];
+  __shared__ float4 sd[32];
   const int k = threadIdx.x;
   const int64_t r0 = (int64_t)blockIdx.x * 32;
+  const int rows = (int)min((int64_t)32, n - r0);
+  if (k < 32)
+    sd[k] = k < rows ? reinterpret_cast<const float4*>(dout)[r0 + k] : make_float4(0, 0, 0, 0);
   const float w0 = W4[k], w1 = W4[kMlpHid + k], w2 = W4[2 * kMlpHid + k], w3 = W4[3 * kMlpHid + k];
+  __syncthreads();
+  float a0 = 0, a1 = 0, a2 = 0, a3 = 0, b3 = 0;
+#pragma unroll 8
   for (int rr = 0; rr < 32; ++rr) {
+    if (rr >= rows) break;
     const int64_t r = r0 + rr;
-    if (r >= n) break;
-    const float* d = dout + r * kMlpOut;
-    const float dh = d[0] * w0 + d[1] * w1 + d[2] * w2 + d[3] * w3;
+    const float4 d = sd[rr];
+    const float h = __bfloat162float(h3[r * kMlpHid + k]);
+    const float dh = d.x * w0 + d.y * w1 + d.z * w2 + d.w * w3;
     const float dz = dh * gelu_grad_f(z3[r * kMlpHid + k]);
-    dzf[r * kMlpHid + k] = dz;
     const __nv_bfloat16 b = __float2bfloat16_rn(dz);
     dzb[r * kMlpHid + k] = b;
     tile[rr][k] = b;
+    a0 += d.x * h;
+    a1 += d.y * h;
+    a2 += d.z * h;
+    a3 += d.w * h;
+    b3 += dz;
   }
-  __syncthreads();
-  // transpose: thread t writes rows k' = t/32 + 8j of the block, 32 consecutive r
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t r = r0 + lane;
-  if (r < n)
-    for (int kk = wid; kk < kMlpHid; kk += 8) dzt[(int64_t)kk * ld_t + r] = tile[lane][kk];
-}
-
-// partial dW4 (4 x 256) and db4 (4) per block of rows: partial[block][0..1027]
-__global__ void head_wgrad_kernel(const float* dout, const __nv_bfloat16* h3, int64_t n,
-                                  int64_t rows_per_blk, float* partial) {
-  const int k = threadIdx.x;  // 256 threads
-  const int64_t r0 = (int64_t)blockIdx.x * rows_per_blk;
-  const int64_t r1 = min(n, r0 + rows_per_blk);
-  float a0 = 0, a1 = 0, a2 = 0, a3 = 0, b = 0;
-  for (int64_t r = r0; r < r1; ++r) {
-    const float h = __bfloat162float(h3[r * kMlpHid + k]);
-    const float* d = dout + r * kMlpOut;
-    a0 += d[0] * h;
-    a1 += d[1] * h;
-    a2 += d[2] * h;
-    a3 += d[3] * h;
-    if (k < kMlpOut) b += d[k];
-  }
-  float* p = partial + (int64_t)blockIdx.x * (kMlpOut * kMlpHid + kMlpOut);
+  float* p = partial + (int64_t)blockIdx.x * kHeadPart;
   p[k] = a0;
   p[kMlpHid + k] = a1;
   p[2 * kMlpHid + k] = a2;
   p[3 * kMlpHid + k] = a3;
-  if (k < kMlpOut) p[kMlpOut * kMlpHid + k] = b;
+  p[kMlpOut * kMlpHid + kMlpOut + k] = b3;
+  if (k < kMlpOut) {
+    float b = 0;
+    for (int rr = 0; rr < rows; ++rr) b += reinterpret_cast<const float*>(&sd[rr])[k];
+    p[kMlpOut * kMlpHid + k] = b;
+  }
+  __syncthreads();
+  // transpose: thread t writes rows k' = t/32 + 8j of the block, 32 consecutive r
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane < rows)
+    for (int kk = wid; kk < kMlpHid; kk += 8) dzt[(int64_t)kk * ld_t + r0 + lane] = tile[lane][kk];
 }
 
-// out[i] = sum_p partial[p][i]  (i < len, partial row stride len)
-__global__ void sum_partials_kernel(const float* partial, int n_part, int len, float* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= len) return;
-  float s = 0.0f;
-  for (int p = 0; p < n_part; ++p) s += partial[(int64_t)p * len + i];
-  out[i] = s;
+// The step's last sums in one launch: out[q] = sum_p part[p * stride + q] over every segment's
+// partials (weight gradients' K splits, head and bias partials), and the mean loss.  A block
+// takes 32 outputs; its 8 warps take every 8th partial each, added in order at the end.
+struct SumSegment {
+  const float* part;
+  int n_part;
+  int64_t stride;   // between partials
+  int rows, cols;   // outputs; row stride ld in a partial, ld_out in the gradient
+  int ld, ld_out;
+  float* out;
+  int first;        // first block
+};
+constexpr int kSegments = 7;
+struct SumArgs {
+  SumSegment seg[kSegments];
+  const double* loss_part;
+  int n_loss;
+  double loss_scale;
+  double* loss;
+};
+__global__ void __launch_bounds__(256) sum_segments_kernel(const __grid_constant__ SumArgs a) {
+  __shared__ float red[8][32];
+  __shared__ double dred[256];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (blockIdx.x == gridDim.x - 1) {
+    double t = 0.0;
+    for (int i = threadIdx.x; i < a.n_loss; i += 256) t += a.loss_part[i];
+    dred[threadIdx.x] = t;
+    __syncthreads();
+    for (int k = 128; k > 0; k >>= 1) {
+      if ((int)threadIdx.x < k) dred[threadIdx.x] += dred[threadIdx.x + k];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *a.loss = dred[0] * a.loss_scale;
+    return;
+  }
+  int k = 0;
+  for (int i = 1; i < kSegments; ++i)
+    if ((int)blockIdx.x >= a.seg[i].first) k = i;
+  const SumSegment& g = a.seg[k];
+  const int q = (blockIdx.x - g.first) * 32 + lane;
+  const bool ok = q < g.rows * g.cols;
+  const int r = ok ? q / g.cols : 0, c = ok ? q - r * g.cols : 0;
+  const float* src = g.part + (int64_t)r * g.ld + c;
+  float t = 0.0f;
+#pragma unroll 4
+  for (int p = w; p < g.n_part; p += 8) t += src[p * g.stride];
+  red[w][lane] = t;
+  __syncthreads();
+  if (w == 0 && ok) {
+    float u = 0.0f;
+    for (int i = 0; i < 8; ++i) u += red[i][lane];
+    g.out[(int64_t)r * g.ld_out + c] = u;
+  }
 }
 
-// split-K partials [S][M][ld] -> out[m * ld_out + c] for c < N
-__global__ void splitk_reduce_kernel(const float* part, int S, int M, int N, int ld, float* out,
-                                     int ld_out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M * N) return;
-  const int m = i / N, c = i % N;
-  float s = 0.0f;
-  for (int z = 0; z < S; ++z) s += part[((int64_t)z * M + m) * ld + c];
-  out[(int64_t)m * ld_out + c] = s;
-}
-
-// column sums of a [n x 256] f32 matrix (bias gradients): per block of kColRows rows
-// a partial row, then sum_partials_kernel; fixed order throughout
-constexpr int kColRows = 128;
-__global__ void colsum_kernel(const float* a, int64_t n, float* partial) {
-  const int k = threadIdx.x;
-  const int64_t r0 = (int64_t)blockIdx.x * kColRows;
-  const int64_t r1 = min(n, r0 + kColRows);
-  float s = 0.0f;
-#pragma unroll 8
-  for (int64_t r = r0; r < r1; ++r) s += a[r * kMlpHid + k];
-  partial[(int64_t)blockIdx.x * kMlpHid + k] = s;
-}
-
-__global__ void adam_kernel(float* p, const float* g, float* m, float* v, int64_t n, float lr,
-                            float b1, float b2, float eps, float bc1, float bc2) {
+// Adam, and the bf16 weight copies of the GEMMs (pack_w1_kernel, pack_sq_kernel) from the new
+// value
+__global__ void adam_kernel(float* p, const float* g, float* m, float* v, MlpDims D, float lr,
+                            float b1, float b2, float eps, float bc1, float bc2,
+                            __nv_bfloat16* wb1, __nv_bfloat16* wb2, __nv_bfloat16* wt2,
+                            __nv_bfloat16* wb3, __nv_bfloat16* wt3) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= D.params) return;
   const float gi = g[i];
   const float mi = b1 * m[i] + (1.0f - b1) * gi;
   const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
   m[i] = mi;
   v[i] = vi;
-  p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+  const float w = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+  p[i] = w;
+  const __nv_bfloat16 b = __float2bfloat16_rn(w);
+  if (i < D.off_b1) {
+    const int r = (int)(i / D.in), c = (int)(i - (int64_t)r * D.in);
+    wb1[(int64_t)r * D.in_pad + c] = b;
+  } else if (i >= D.off_w2 && i < D.off_b2) {
+    const int q = (int)(i - D.off_w2), r = q / kMlpHid, c = q % kMlpHid;
+    wb2[q] = b;
+    wt2[c * kMlpHid + r] = b;
+  } else if (i >= D.off_w3 && i < D.off_b3) {
+    const int q = (int)(i - D.off_w3), r = q / kMlpHid, c = q % kMlpHid;
+    wb3[q] = b;
+    wt3[c * kMlpHid + r] = b;
+  }
 }
 
 // ---------------------------------------------------------------- sampling
@@ -327,17 +374,16 @@ void ensure_batch(olpt_ctx* ctx, int64_t n) {
   W.h1.ensure(hb * 2, s);
   W.h2.ensure(hb * 2, s);
   W.h3.ensure(hb * 2, s);
-  W.o.ensure((size_t)m * kMlpOut * 4, s);
   W.err.ensure(16, s);
   W.xin.ensure((size_t)m * D.in * 4, s);
   W.tgt.ensure((size_t)m * kMlpOut * 4, s);
   W.xt.ensure((size_t)D.in_pad * lt * 2, s);
-  for (DevBuf* b : {&W.z1, &W.z2, &W.z3, &W.dz1f, &W.dz2f, &W.dz3f}) b->ensure(hb * 4, s);
+  for (DevBuf* b : {&W.z1, &W.z2, &W.z3}) b->ensure(hb * 4, s);
   for (DevBuf* b : {&W.dz2b, &W.dz3b}) b->ensure(hb * 2, s);
   for (DevBuf* b : {&W.h1t, &W.h2t, &W.dz1t, &W.dz2t, &W.dz3t})
     b->ensure((size_t)kMlpHid * lt * 2, s);
   W.dout.ensure((size_t)m * kMlpOut * 4, s);
-  W.loss.ensure((size_t)(nblk(m) + 2) * 8, s);
+  W.loss.ensure((size_t)(nblk(m, 8) + 2) * 8, s);
 }
 
 void pack_weights(olpt_ctx* ctx) {
@@ -413,41 +459,6 @@ void forward(olpt_ctx* ctx, int64_t n) {
   e3.ld_f32 = kMlpHid;
   gemm_bf16(W.h2.as<__nv_bfloat16>(), kMlpHid, W.wb3.as<__nv_bfloat16>(), kMlpHid, (int)n, kMlpHid,
             kMlpHid, e3, 1, err, s);
-  head_fwd_kernel<<<OLPT_G(nblk(n * 32)), 256, 0, s>>>(W.h3.as<__nv_bfloat16>(), n, M + D.off_w4,
-                                                      M + D.off_b4, W.o.as<float>());
-  OLPT_CUDA(cudaGetLastError());
-}
-
-void bias_grad(olpt_ctx* ctx, const float* dz, int64_t n, float* out) {
-  MlpWork& W = ctx->mlp;
-  cudaStream_t s = ctx->stream;
-  const int nb = (int)((n + kColRows - 1) / kColRows);
-  W.hpart.ensure((size_t)nb * kMlpHid * 4 + 64, s);
-  colsum_kernel<<<OLPT_G(nb), kMlpHid, 0, s>>>(dz, n, W.hpart.as<float>());
-  sum_partials_kernel<<<OLPT_G(1), kMlpHid, 0, s>>>(W.hpart.as<float>(), nb, kMlpHid, out);
-  OLPT_CUDA(cudaGetLastError());
-}
-
-// weight gradient dW[M x N] = A^T-layout GEMM over the batch (K = n), split-K partials
-void wgrad(olpt_ctx* ctx, const __nv_bfloat16* at, const __nv_bfloat16* bt, int64_t n, int Mo,
-           int No, int ld_part, float* out, int ld_out, int n_keep) {
-  MlpWork& W = ctx->mlp;
-  cudaStream_t s = ctx->stream;
-  const int lt = (int)round8(n);
-  const int tiles = ((Mo + 127) / 128) * ((No + 127) / 128);
-  const int kt = (int)((n + 63) / 64);
-  const int splits = std::max(1, std::min(kt, 148 / tiles));
-  W.part.ensure((size_t)splits * Mo * ld_part * 4 + 64, s);
-  GemmEpilogue e;
-  e.out_f32 = W.part.as<float>();
-  e.ld_f32 = ld_part;
-  gemm_bf16(at, lt, bt, lt, Mo, No, (int)n, e, splits, W.err.as<int>(), s);
-  // the launcher may merge splits so that none is empty; recompute as it does
-  const int kps = (kt + splits - 1) / splits;
-  const int S = (kt + kps - 1) / kps;
-  splitk_reduce_kernel<<<OLPT_G(nblk((int64_t)Mo * n_keep)), 256, 0, s>>>(
-      W.part.as<float>(), S, Mo, n_keep, ld_part, out, ld_out);
-  OLPT_CUDA(cudaGetLastError());
 }
 
 }  // namespace
@@ -590,81 +601,93 @@ const double* train_enqueue(olpt_ctx* ctx, const float* x_f32, const float* tgt,
   const MlpDims& D = W.dims;
   ensure_batch(ctx, n);
   const int64_t lt = round8(n);
-  input_kernel<<<OLPT_G(nblk(n * D.in_pad)), 256, 0, s>>>(x_f32, n, D.in, D.in_pad,
-                                                          W.x.as<__nv_bfloat16>());
-  {
-    dim3 g((unsigned)((n + 31) / 32), D.in_pad / 32);
-    transpose_kernel<<<OLPT_G(g), dim3(32, 8), 0, s>>>(W.x.as<__nv_bfloat16>(), n, D.in_pad,
-                                                       D.in_pad, W.xt.as<__nv_bfloat16>(), lt);
-  }
+  input_kernel<<<OLPT_G(dim3((unsigned)((n + 63) / 64), D.in_pad / 64)), 256, 0, s>>>(
+      x_f32, n, D.in, D.in_pad, W.x.as<__nv_bfloat16>(), W.xt.as<__nv_bfloat16>(), lt);
   forward(ctx, n);
   float* G = W.grad.as<float>();
   const float* M = W.master.as<float>();
   // loss and head
-  const int lb = nblk(n);
-  loss_kernel<<<OLPT_G(lb), 256, 0, s>>>(W.o.as<float>(), tgt, n, (float)ghost_weight,
-                                         W.dout.as<float>(), W.loss.as<double>());
-  sum_double_kernel<<<OLPT_G(1), 32, 0, s>>>(W.loss.as<double>(), lb, W.loss.as<double>() + lb,
-                                             1.0 / (double)n);
-  const int64_t rpb = 256;
-  const int hb = (int)((n + rpb - 1) / rpb);
-  const int hlen = kMlpOut * kMlpHid + kMlpOut;
-  W.hpart.ensure((size_t)hb * hlen * 4 + 64, s);
-  head_wgrad_kernel<<<OLPT_G(hb), 256, 0, s>>>(W.dout.as<float>(), W.h3.as<__nv_bfloat16>(), n, rpb,
-                                               W.hpart.as<float>());
-  sum_partials_kernel<<<OLPT_G(nblk(hlen)), 256, 0, s>>>(W.hpart.as<float>(), hb, hlen,
-                                                         G + D.off_w4);
-  // (hpart is reused by the bias gradients below, after these kernels in stream order)
-  head_bwd_kernel<<<OLPT_G((unsigned)((n + 31) / 32)), 256, 0, s>>>(
-      W.dout.as<float>(), M + D.off_w4, W.z3.as<float>(), n, W.dz3f.as<float>(), W.dz3b.as<__nv_bfloat16>(),
-      W.dz3t.as<__nv_bfloat16>(), lt);
+  const int lb = nblk(n, 8);
+  head_loss_kernel<<<OLPT_G(lb), 256, 0, s>>>(W.h3.as<__nv_bfloat16>(), n, M + D.off_w4,
+                                              M + D.off_b4, tgt, (float)ghost_weight,
+                                              W.dout.as<float>(), W.loss.as<double>() + 1);
+  const int hb = nblk(n, 32), mt = nblk(n, 128);
+  W.hpart.ensure((size_t)hb * kHeadPart * 4 + (size_t)2 * mt * kMlpHid * 4 + 64, s);
+  float* hpart = W.hpart.as<float>();
+  float* cpart = hpart + (size_t)hb * kHeadPart;
+  head_bwd_kernel<<<OLPT_G(hb), kMlpHid, 0, s>>>(
+      W.dout.as<float>(), M + D.off_w4, W.z3.as<float>(), W.h3.as<__nv_bfloat16>(), n,
+      W.dz3b.as<__nv_bfloat16>(), W.dz3t.as<__nv_bfloat16>(), lt, hpart);
   OLPT_CUDA(cudaGetLastError());
   int* err = W.err.as<int>();
-  // layer 3
-  wgrad(ctx, W.dz3t.as<__nv_bfloat16>(), W.h2t.as<__nv_bfloat16>(), n, kMlpHid, kMlpHid, kMlpHid,
-        G + D.off_w3, kMlpHid, kMlpHid);
-  bias_grad(ctx, W.dz3f.as<float>(), n, G + D.off_b3);
+  // dZ2, dZ1 with their column sums
   GemmEpilogue d2;
   d2.gelu_pre = W.z2.as<float>();
   d2.ld_pre = kMlpHid;
-  d2.out_f32 = W.dz2f.as<float>();
-  d2.ld_f32 = kMlpHid;
   d2.out_bf16 = W.dz2b.as<__nv_bfloat16>();
   d2.ld_bf16 = kMlpHid;
   d2.out_bf16_t = W.dz2t.as<__nv_bfloat16>();
   d2.ld_t = (int)lt;
+  d2.colsum = cpart;
   gemm_bf16(W.dz3b.as<__nv_bfloat16>(), kMlpHid, W.wt3.as<__nv_bfloat16>(), kMlpHid, (int)n,
             kMlpHid, kMlpHid, d2, 1, err, s);
-  // layer 2
-  wgrad(ctx, W.dz2t.as<__nv_bfloat16>(), W.h1t.as<__nv_bfloat16>(), n, kMlpHid, kMlpHid, kMlpHid,
-        G + D.off_w2, kMlpHid, kMlpHid);
-  bias_grad(ctx, W.dz2f.as<float>(), n, G + D.off_b2);
   GemmEpilogue d1;
   d1.gelu_pre = W.z1.as<float>();
   d1.ld_pre = kMlpHid;
-  d1.out_f32 = W.dz1f.as<float>();
-  d1.ld_f32 = kMlpHid;
   d1.out_bf16_t = W.dz1t.as<__nv_bfloat16>();
   d1.ld_t = (int)lt;
+  d1.colsum = cpart + (size_t)mt * kMlpHid;
   gemm_bf16(W.dz2b.as<__nv_bfloat16>(), kMlpHid, W.wt2.as<__nv_bfloat16>(), kMlpHid, (int)n,
             kMlpHid, kMlpHid, d1, 1, err, s);
-  // layer 1
-  wgrad(ctx, W.dz1t.as<__nv_bfloat16>(), W.xt.as<__nv_bfloat16>(), n, kMlpHid, D.in_pad,
-        D.in_pad, G + D.off_w1, D.in, D.in);
-  bias_grad(ctx, W.dz1f.as<float>(), n, G + D.off_b1);
+  // weight gradients over the batch (K = n): split-K partials that fill the SMs once
+  const int tiles = 2 * (2 + 2 + (D.in_pad + 127) / 128);
+  const int want = std::max(1, 148 / tiles);
+  int kps = 0;
+  const int S = gemm_splits((int)n, want, &kps);
+  const size_t sq = (size_t)S * kMlpHid * kMlpHid;
+  W.part.ensure((2 * sq + (size_t)S * kMlpHid * D.in_pad) * 4 + 64, s);
+  float* p3 = W.part.as<float>();
+  float *p2 = p3 + sq, *p1 = p2 + sq;
+  auto bf = [](DevBuf& b) { return b.as<__nv_bfloat16>(); };
+  const int ltt = (int)lt;
+  const GemmProblem prob[3] = {
+      {bf(W.dz1t), ltt, bf(W.xt), ltt, kMlpHid, D.in_pad, (int)n, want, p1, D.in_pad},
+      {bf(W.dz3t), ltt, bf(W.h2t), ltt, kMlpHid, kMlpHid, (int)n, want, p3, kMlpHid},
+      {bf(W.dz2t), ltt, bf(W.h1t), ltt, kMlpHid, kMlpHid, (int)n, want, p2, kMlpHid}};
+  gemm_bf16_group(prob, 3, err, s);
+  // every remaining sum
+  SumArgs a{};
+  int blocks = 0, k = 0;
+  auto seg = [&](const float* part, int n_part, int64_t stride, int rows, int cols, int ld,
+                 float* out, int ld_out) {
+    a.seg[k++] = SumSegment{part, n_part, stride, rows, cols, ld, ld_out, out, blocks};
+    blocks += nblk((int64_t)rows * cols, 32);
+  };
+  seg(p1, S, (int64_t)kMlpHid * D.in_pad, kMlpHid, D.in, D.in_pad, G + D.off_w1, D.in);
+  seg(p2, S, kMlpHid * kMlpHid, kMlpHid, kMlpHid, kMlpHid, G + D.off_w2, kMlpHid);
+  seg(p3, S, kMlpHid * kMlpHid, kMlpHid, kMlpHid, kMlpHid, G + D.off_w3, kMlpHid);
+  seg(hpart, hb, kHeadPart, 1, kMlpOut * kMlpHid + kMlpOut, 0, G + D.off_w4, 0);  // W4, b4
+  seg(hpart + kMlpOut * kMlpHid + kMlpOut, hb, kHeadPart, 1, kMlpHid, 0, G + D.off_b3, 0);
+  seg(d2.colsum, mt, kMlpHid, 1, kMlpHid, 0, G + D.off_b2, 0);
+  seg(d1.colsum, mt, kMlpHid, 1, kMlpHid, 0, G + D.off_b1, 0);
+  a.loss_part = W.loss.as<double>() + 1;
+  a.n_loss = lb;
+  a.loss_scale = 1.0 / (double)n;
+  a.loss = W.loss.as<double>();
+  sum_segments_kernel<<<OLPT_G(blocks + 1), 256, 0, s>>>(a);
   OLPT_CUDA(cudaGetLastError());
   if (update) {
     ++W.adam_t;
     const float b1 = 0.9f, b2 = 0.999f;
     const float bc1 = 1.0f - std::pow(b1, (float)W.adam_t);
     const float bc2 = 1.0f - std::pow(b2, (float)W.adam_t);
-    adam_kernel<<<OLPT_G(nblk(D.params)), 256, 0, s>>>(W.master.as<float>(), G, W.am.as<float>(),
-                                                       W.av.as<float>(), D.params, (float)lr, b1,
-                                                       b2, 1e-8f, bc1, bc2);
+    adam_kernel<<<OLPT_G(nblk(D.params)), 256, 0, s>>>(
+        W.master.as<float>(), G, W.am.as<float>(), W.av.as<float>(), D, (float)lr, b1, b2, 1e-8f,
+        bc1, bc2, W.wb1.as<__nv_bfloat16>(), W.wb2.as<__nv_bfloat16>(), W.wt2.as<__nv_bfloat16>(),
+        W.wb3.as<__nv_bfloat16>(), W.wt3.as<__nv_bfloat16>());
     OLPT_CUDA(cudaGetLastError());
-    pack_weights(ctx);
   }
-  return W.loss.as<double>() + lb;
+  return W.loss.as<double>();
 }
 }  // namespace
 

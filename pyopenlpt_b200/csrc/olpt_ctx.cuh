@@ -332,14 +332,14 @@ struct MlpWork {
   int64_t cap = 0;  // batch capacity of the activation buffers
   DevBuf master, grad, am, av, wb1, wb2, wb3, wt2, wt3;
   DevBuf x, xt, xin, tgt, z1, z2, z3, h1, h2, h3, h1t, h2t, o, dout;
-  DevBuf dz1f, dz2f, dz3f, dz2b, dz3b, dz1t, dz2t, dz3t, part, hpart, loss, err;
+  DevBuf dz2b, dz3b, dz1t, dz2t, dz3t, part, hpart, loss, err;
   // learned shake: keep[i] = 1 for the input objects the network did not drop (the
   // objects left are the kept ones in input order), pos = their exclusive scan; fb =
   // fallback counter
   DevBuf keep, pos, start_xyz, act, nres, ds_x, ds_t, loss_hist, fb;
   void release(cudaStream_t s) {
     for (DevBuf* b : {&master, &grad, &am, &av, &wb1, &wb2, &wb3, &wt2, &wt3, &x, &xt, &xin, &tgt,
-                      &z1, &z2, &z3, &h1, &h2, &h3, &h1t, &h2t, &o, &dout, &dz1f, &dz2f, &dz3f,
+                      &z1, &z2, &z3, &h1, &h2, &h3, &h1t, &h2t, &o, &dout, 
                       &dz2b, &dz3b, &dz1t, &dz2t, &dz3t, &part, &hpart, &loss, &err, &keep, &pos,
                       &start_xyz, &act, &nres, &ds_x, &ds_t, &loss_hist, &fb})
       b->release(s);

@@ -24,12 +24,30 @@ struct GemmEpilogue {
   int ld_bf16 = 0;
   __nv_bfloat16* out_bf16_t = nullptr;  // N x ld_t
   int ld_t = 0;
+  // with gelu_pre, no bias, splits 1: f32 sums of v over every 128-row tile, (M / 128) x N
+  float* colsum = nullptr;
 };
 
 // A: M rows of K (leading dimension lda elements, a multiple of 8); B: N rows of K.
 // err: device flag, nonzero after a wait timed out.
 void gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N,
                int K, const GemmEpilogue& ep, int splits, int* err, cudaStream_t s);
+
+// Split-K products that only leave f32 partials ([split][M][ld_part]), up to kGemmGroup of
+// them in one launch.
+constexpr int kGemmGroup = 3;
+struct GemmProblem {
+  const __nv_bfloat16* A;
+  int lda;
+  const __nv_bfloat16* B;
+  int ldb;
+  int M, N, K, splits;
+  float* part;
+  int ld_part;
+};
+void gemm_bf16_group(const GemmProblem* p, int n, int* err, cudaStream_t s);
+// splits that a request for `splits` gives, and the k tiles of each
+int gemm_splits(int K, int splits, int* kt_per_split);
 
 // Device-side GELU (erf form) and its derivative, shared by the MLP kernels.
 __device__ __forceinline__ float gelu_f(float x) {
