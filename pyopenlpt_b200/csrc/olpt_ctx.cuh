@@ -126,8 +126,11 @@ struct Csr {
 // Device workspace of the shake (grown on demand).
 struct ShakeWork {
   DevBuf otfp;      // n x n_cam x 5 OTF parameters at the object centres
-  DevBuf pair_key;  // n x n_cam tile keys
-  Csr bins;         // (object, camera) pairs per image tile
+  DevBuf proj;      // projection planes of all cameras, zero between passes
+  bool proj_clean = false;
+  int proj_esz = 0;
+  int64_t proj_bytes = 0;
+  const void* proj_at = nullptr;
   DevBuf rep, hkey, has_nb, nb_pos, nb_list, scan_tmp, gpart;
   Csr hash;         // 3D hash grid of object centres
   void release(cudaStream_t s) {
@@ -135,8 +138,8 @@ struct ShakeWork {
     nb_list.release(s);
     scan_tmp.release(s);
     otfp.release(s);
-    pair_key.release(s);
-    bins.release(s);
+    proj.release(s);
+    proj_clean = false;
     rep.release(s);
     hkey.release(s);
     has_nb.release(s);

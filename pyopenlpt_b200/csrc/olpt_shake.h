@@ -31,12 +31,10 @@ struct ShakeView {
   OtfView otf;
   double r_px, ratio;
   int roi_area;          // augmented ROI pixels (side^2)
-  int win_w, win_h;      // projection window
   int exact_sums;        // FP64 path: row-major sequential sums
-  int tile_base[OLPT_MAX_CAM];
-  int n_tiles;
   PlaneView orig[OLPT_MAX_CAM];  // current images (u8/u16/f32/f64)
   PlaneView res[OLPT_MAX_CAM];   // residual planes (Real)
+  PlaneView proj[OLPT_MAX_CAM];  // projection planes (Real), 0 outside a pass
   int n_poly;            // most terms of a polynomial camera with exponents 0..3
   double fit3[2][3];     // linear and quadratic rows of the three-point parabola fit
   // shared memory of the shake kernel: the cameras' table, then the objects' arrays

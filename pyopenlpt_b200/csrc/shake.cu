@@ -7,14 +7,12 @@
 // gaussIntensity / project2DInt / calShakeResidue (:901-1045).
 //
 // B200 mapping, per shake iteration:
-//  1. prep: one thread per object projects it on every camera (FP64), evaluates the
-//     OTF at its centre and keys each (object, camera) pair by the 32x32 image tile
-//     of its projection; a counting sort turns the keys into per-tile bins.
-//  2. residual: one CTA owns one image tile, gathers the objects binned in the 3x3
-//     neighbouring tiles, max-fuses their Gaussian footprints in shared memory and
-//     writes residual = image - max projection for the whole tile.  No global
-//     atomics, and the result does not depend on object order (min-fusion in the
-//     reference is a max over projections).
+//  1. splat: one thread per (object, camera) projects the object (FP64) and evaluates
+//     the OTF there; the warp then raises every pixel of its 32 windows in a projection
+//     plane to the window's Gaussian by atomic maxima (max-fusion does not depend on
+//     order, and non-negative floats order as integers).
+//  2. residual: one streaming pass writes residual = image - projection and sets the
+//     projection plane back to 0.
 //  3. shake: a group of 8 lanes (32 for few objects) per particle stages its 8x8
 //     augmented ROI of every camera in shared memory, then runs the reference's
 //     axis-wise line search.  Projections spread (trial point, camera) pairs over the
@@ -39,112 +37,150 @@
 
 namespace olpt {
 
-constexpr int kTile = 32;
 constexpr size_t kShakeSmemMax = 200 * 1024;  // shared memory of a shake block
 
 namespace {
 
 inline int nblk(int64_t n, int t = 256) { return (int)((n + t - 1) / t); }
 
-// ---------------------------------------------------------------- 1. prep
+// ---------------------------------------------------------------- 1. splat
+__device__ __forceinline__ void raise_to(float* p, float v) {
+  atomicMax(reinterpret_cast<unsigned int*>(p), __float_as_uint(v));
+}
+__device__ __forceinline__ void raise_to(double* p, double v) {
+  atomicMax(reinterpret_cast<unsigned long long*>(p), (unsigned long long)__double_as_longlong(v));
+}
+
+// Bound by the FP64 geometry of the pairs and, per window, about 60 instructions on 16 lanes
+// (a window's row is one 16-byte run of one sector for the atomics).  Replaces a pass over the
+// objects, the counting sort of the pairs by 32x32 image tile (five launches) and a kernel in
+// which four tiles each recomputed a pair's window and Gaussian per pixel: 120,000 objects on
+// six 2048^2 cameras, the whole residual took 620 us and takes 150 us.
 template <typename Real>
-__global__ void prep_kernel(const __grid_constant__ ShakeView v, const double* xyz, int64_t n, double* uv, Real* otfp,
-                            int* pair_key, const uint8_t* flags, int all_cams) {
-  int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (o >= n) return;
-  const double X = xyz[3 * o], Y = xyz[3 * o + 1], Z = xyz[3 * o + 2];
-  const bool masked = flags && flags[o] != 0;
-  for (int c = 0; c < v.n_cam; ++c) {
-    double u, w;
-    cam_project(v.cams[c], X, Y, Z, u, w);
-    uv[(o * v.n_cam + c) * 2] = u;
-    uv[(o * v.n_cam + c) * 2 + 1] = w;
+__global__ void __launch_bounds__(256) splat_kernel(const __grid_constant__ ShakeView v,
+                                                    const double* xyz, int64_t n, double* uv,
+                                                    Real* otfp, const uint8_t* flags,
+                                                    int all_cams) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int64_t pair = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  double u = 0.0, w = 0.0;
+  Real o[5] = {0, 0, 0, 0, 0};
+  Rect r{1, 0, 1, 0};
+  int c = 0;
+  if (pair < n * v.n_cam) {
+    const int64_t obj = pair / v.n_cam;
+    c = (int)(pair - obj * v.n_cam);
+    const CamDev& cm = v.cams[c];
+    const double X = xyz[3 * obj], Y = xyz[3 * obj + 1], Z = xyz[3 * obj + 2];
+    cam_project(cm, X, Y, Z, u, w);
+    uv[2 * pair] = u;
+    uv[2 * pair + 1] = w;
     double q[5];
     otf_param(v.otf, c, X, Y, Z, q);
-    for (int k = 0; k < 5; ++k) otfp[(o * v.n_cam + c) * 5 + k] = (Real)q[k];
-    int key = -1;
-    if (!masked && (all_cams || v.cams[c].is_active)) {
-      const Rect r = roi_bound(v.cams[c].n_row, v.cams[c].n_col, u, w, v.r_px, v.r_px);
-      if (!rect_empty(r)) {
-        const int ntx = (v.cams[c].n_col + kTile - 1) / kTile;
-        key = v.tile_base[c] + (r.rmin / kTile) * ntx + (r.cmin / kTile);
-      }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      o[k] = (Real)q[k];
+      otfp[5 * pair + k] = o[k];
     }
-    pair_key[o * v.n_cam + c] = key;
+    if (!(flags && flags[obj] != 0) && (all_cams || cm.is_active))
+      r = roi_bound(cm.n_row, cm.n_col, u, w, v.r_px, v.r_px);
+  }
+  const bool some = r.rmax > r.rmin && r.cmax > r.cmin;
+  unsigned todo = __ballot_sync(kFull, some);
+  const int sub = lane & 15;
+  // two windows at a time, 16 lanes each
+  while (todo) {
+    const int a = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int b = todo ? __ffs(todo) - 1 : -1;
+    if (todo) todo &= todo - 1;
+    const bool on = lane < 16 || b >= 0;
+    const int src = lane < 16 || b < 0 ? a : b;
+    const double uu = __shfl_sync(kFull, u, src), ww = __shfl_sync(kFull, w, src);
+    Real q[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) q[k] = __shfl_sync(kFull, o[k], src);
+    const int r0 = __shfl_sync(kFull, r.rmin, src), r1 = __shfl_sync(kFull, r.rmax, src);
+    const int c0 = __shfl_sync(kFull, r.cmin, src), c1 = __shfl_sync(kFull, r.cmax, src);
+    const int cc = __shfl_sync(kFull, c, src);
+    if (!on) continue;
+    const int wd = c1 - c0, area = wd * (r1 - r0);
+    Real* plane = reinterpret_cast<Real*>(v.proj[cc].p);
+    const int64_t pitch = v.proj[cc].pitch / (int64_t)sizeof(Real);
+    for (int k = sub; k < area; k += 16) {
+      const int dr = k / wd, row = r0 + dr, col = c0 + k - dr * wd;
+      const Real g = gauss<Real>(col, row, uu, ww, q);
+      if (g > (Real)0) raise_to(plane + row * pitch + col, g);
+    }
   }
 }
 
 // ---------------------------------------------------------------- 2. residual
-__device__ __forceinline__ void smem_max(float* p, float v) {
-  atomicMax(reinterpret_cast<unsigned int*>(p), __float_as_uint(v));
-}
-__device__ __forceinline__ void smem_max(double* p, double v) {
-  atomicMax(reinterpret_cast<unsigned long long*>(p), (unsigned long long)__double_as_longlong(v));
+// residual = o where nothing projects, else min(o, o - p), clamped at 0 on request
+template <typename Real>
+__device__ __forceinline__ Real subtract(Real o, Real p, int clamp) {
+  if (!(p > (Real)0)) return o;
+  Real val = o - p;
+  if (val > o) val = o;
+  return clamp && val < (Real)0 ? (Real)0 : val;
 }
 
-// Window tiles are keyed by the tile of the window's top-left pixel, so a CTA
-// gathers bins of its own tile and the tiles up/left of it (windows < 32 px).
-template <typename Real>
-__global__ void __launch_bounds__(256) residual_kernel(const __grid_constant__ ShakeView v, const double* uv,
-                                                       const Real* otfp, const int* bin_start,
-                                                       const int* bin_items, int clamp,
-                                                       int all_cams) {
-  __shared__ Real pmax[kTile * kTile];
-  // locate camera and tile
-  int cam = 0;
-  for (int c = 1; c < v.n_cam; ++c)
-    if ((int)blockIdx.x >= v.tile_base[c]) cam = c;
-  const CamDev& cm = v.cams[cam];
-  if (!(all_cams || cm.is_active)) return;
-  const int ntx = (cm.n_col + kTile - 1) / kTile;
-  const int t = blockIdx.x - v.tile_base[cam];
-  const int ty = t / ntx, tx = t % ntx;
-  const int r0 = ty * kTile, c0 = tx * kTile;
-  for (int i = threadIdx.x; i < kTile * kTile; i += blockDim.x) pmax[i] = (Real)0;
-  __syncthreads();
-  const int nty = (cm.n_row + kTile - 1) / kTile;
-  const int win = v.win_w * v.win_h;
-  for (int dy = -1; dy <= 0; ++dy) {
-    const int by = ty + dy;
-    if (by < 0 || by >= nty) continue;
-    for (int dx = -1; dx <= 0; ++dx) {
-      const int bx = tx + dx;
-      if (bx < 0 || bx >= ntx) continue;
-      const int b = v.tile_base[cam] + by * ntx + bx;
-      const int s0 = bin_start[b], s1 = bin_start[b + 1];
-      const int total = (s1 - s0) * win;
-      for (int k = threadIdx.x; k < total; k += blockDim.x) {
-        const int pair = bin_items[s0 + k / win];
-        const int pix = k % win;
-        const int64_t o = pair / v.n_cam;
-        const double u = uv[2 * (int64_t)pair], w = uv[2 * (int64_t)pair + 1];
-        const Rect r = roi_bound(cm.n_row, cm.n_col, u, w, v.r_px, v.r_px);
-        const int rr = r.rmin + pix / v.win_w, cc = r.cmin + pix % v.win_w;
-        if (rr >= r.rmax || cc >= r.cmax) continue;
-        if (rr < r0 || rr >= r0 + kTile || cc < c0 || cc >= c0 + kTile) continue;
-        const Real p = gauss<Real>(cc, rr, u, w, otfp + (int64_t)pair * 5);
-        (void)o;
-        if (p == (Real)0) continue;
-        smem_max(&pmax[(rr - r0) * kTile + (cc - c0)], p);
-      }
+// Streaming: four pixels a thread, 4-byte to 32-byte loads by type.  The projection planes
+// are read and, where something projected, set back to 0 for the next pass.
+template <typename Real, typename T>
+__device__ __forceinline__ void residual_row4(const T* src, Real* proj, Real* dst, int col, int W,
+                                              int clamp) {
+  struct alignas(4 * sizeof(T) > 16 ? 16 : 4 * sizeof(T)) Quad {
+    T v[4];
+  };
+  struct alignas(16) QuadR {
+    Real v[4];
+  };
+  if (col + 4 <= W) {
+    const Quad o = *reinterpret_cast<const Quad*>(src + col);
+    const QuadR p = *reinterpret_cast<const QuadR*>(proj + col);
+    QuadR r;
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      r.v[k] = subtract<Real>((Real)o.v[k], p.v[k], clamp);
+      any |= p.v[k] != (Real)0;
+    }
+    *reinterpret_cast<QuadR*>(dst + col) = r;
+    if (any) *reinterpret_cast<QuadR*>(proj + col) = QuadR{{0, 0, 0, 0}};
+  } else {
+    for (int k = col; k < W; ++k) {
+      dst[k] = subtract<Real>((Real)src[k], proj[k], clamp);
+      proj[k] = (Real)0;
     }
   }
-  __syncthreads();
-  const PlaneView& src = v.orig[cam];
-  Real* dst = reinterpret_cast<Real*>(v.res[cam].p);
-  const int64_t dpitch = v.res[cam].pitch / (int64_t)sizeof(Real);
-  for (int i = threadIdx.x; i < kTile * kTile; i += blockDim.x) {
-    const int rr = r0 + i / kTile, cc = c0 + i % kTile;
-    if (rr >= cm.n_row || cc >= cm.n_col) continue;
-    const Real o = (Real)load_any(src, rr, cc);
-    const Real pm = pmax[i];
-    Real val = o;
-    if (pm > (Real)0) {
-      val = o - pm;
-      if (val > o) val = o;  // keep min(o, o - p)
-      if (clamp && val < (Real)0) val = (Real)0;
-    }
-    dst[(int64_t)rr * dpitch + cc] = val;
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(256) residual_kernel(const __grid_constant__ ShakeView v,
+                                                       int clamp, int all_cams) {
+  const int cam = blockIdx.z;
+  const CamDev& cm = v.cams[cam];
+  if (!(all_cams || cm.is_active)) return;
+  const PlaneView& s = v.orig[cam];
+  const int col = 4 * (blockIdx.x * blockDim.x + threadIdx.x), row = blockIdx.y;
+  if (row >= s.H || col >= s.W) return;
+  Real* proj = reinterpret_cast<Real*>(v.proj[cam].p + row * v.proj[cam].pitch);
+  Real* dst = reinterpret_cast<Real*>(v.res[cam].p + row * v.res[cam].pitch);
+  const unsigned char* src = s.p + row * s.pitch;
+  switch (s.dtype) {
+    case OLPT_U8:
+      residual_row4<Real>(src, proj, dst, col, s.W, clamp);
+      break;
+    case OLPT_U16:
+      residual_row4<Real>(reinterpret_cast<const uint16_t*>(src), proj, dst, col, s.W, clamp);
+      break;
+    case OLPT_F32:
+      residual_row4<Real>(reinterpret_cast<const float*>(src), proj, dst, col, s.W, clamp);
+      break;
+    default:
+      residual_row4<Real>(reinterpret_cast<const double*>(src), proj, dst, col, s.W, clamp);
   }
 }
 
@@ -1231,22 +1267,18 @@ static ShakeView make_view(olpt_ctx* ctx, const ShakeParams& sp, bool fp64) {
   OLPT_REQUIRE(side >= 1 && side <= 16, OLPT_ERR_UNSUPPORTED,
                "augmented ROI side round(2 * radius_obj * ratio_augimg) must be in [1, 16]");
   v.roi_area = side * side;
-  v.win_w = v.win_h = (int)std::lround(2.0 * sp.radius_obj);
-  OLPT_REQUIRE(v.win_w >= 1 && v.win_w < kTile, OLPT_ERR_UNSUPPORTED,
+  const int win = (int)std::lround(2.0 * sp.radius_obj);
+  OLPT_REQUIRE(win >= 1 && win < 32, OLPT_ERR_UNSUPPORTED,
                "projection window round(2 * radius_obj) must be below 32 px");
   v.exact_sums = fp64 ? 1 : 0;
-  int tiles = 0;
   for (int c = 0; c < ctx->n_cam; ++c) {
     const CamDev& cm = ctx->cams_h[c];
-    v.tile_base[c] = tiles;
-    tiles += ((cm.n_row + kTile - 1) / kTile) * ((cm.n_col + kTile - 1) / kTile);
     const ImagePlane& im = ctx->img[c];
     OLPT_REQUIRE(im.buf.p, OLPT_ERR_INVALID_ARG, "no image for camera");
     OLPT_REQUIRE(im.H == cm.n_row && im.W == cm.n_col, OLPT_ERR_INVALID_ARG,
                  "image size differs from the camera's n_row x n_col");
     v.orig[c] = PlaneView{im.buf.as<unsigned char>(), im.pitch, im.H, im.W, im.dtype};
   }
-  v.n_tiles = tiles;
   for (int c = 0; c < ctx->n_cam; ++c) {
     const CamDev& cm = ctx->cams_h[c];
     if (cm.type == CAM_POLYNOMIAL && cm.pow3) v.n_poly = std::max(v.n_poly, cm.n_coeff);
@@ -1271,6 +1303,28 @@ static void ensure_residual_planes(olpt_ctx* ctx, ShakeView& v, bool fp64) {
   }
 }
 
+// Projection planes: zero between passes (the residual kernel leaves them so); allocated and
+// zeroed when the geometry or the type changes, or when a pass did not get to its end.
+static void ensure_projection_planes(olpt_ctx* ctx, ShakeView& v, bool fp64) {
+  ShakeWork& W = ctx->shk;
+  const int esz = fp64 ? 8 : 4;
+  int64_t need = 0;
+  for (int c = 0; c < ctx->n_cam; ++c) need += v.res[c].pitch * v.res[c].H;
+  bool same = W.proj_clean && W.proj_esz == esz && W.proj_bytes == need;
+  W.proj.ensure((size_t)need + 64, ctx->stream);
+  if (!same || W.proj.p != W.proj_at)
+    OLPT_CUDA(cudaMemsetAsync(W.proj.p, 0, (size_t)need, ctx->stream));
+  W.proj_at = W.proj.p;
+  W.proj_esz = esz;
+  W.proj_bytes = need;
+  int64_t off = 0;
+  for (int c = 0; c < ctx->n_cam; ++c) {
+    v.proj[c] = v.res[c];
+    v.proj[c].p = W.proj.as<unsigned char>() + off;
+    off += v.res[c].pitch * v.res[c].H;
+  }
+}
+
 template <typename Real>
 static void residual_pass(olpt_ctx* ctx, ShakeView& v, const uint8_t* flags, int all_cams,
                           int clamp) {
@@ -1279,27 +1333,42 @@ static void residual_pass(olpt_ctx* ctx, ShakeView& v, const uint8_t* flags, int
   const int64_t n = ctx->obj.n;
   const int C = ctx->n_cam;
   W.otfp.ensure((n * C + 1) * 5 * sizeof(Real), s);
-  W.pair_key.ensure((n * C + 1) * sizeof(int), s);
+  ensure_projection_planes(ctx, v, sizeof(Real) == 8);
+  W.proj_clean = false;
   if (n > 0)
-    prep_kernel<Real><<<OLPT_G(nblk(n, 128)), 128, 0, s>>>(v, ctx->obj.xyz.as<double>(), n,
-                                                   ctx->obj.uv.as<double>(), W.otfp.as<Real>(),
-                                                   W.pair_key.as<int>(), flags, all_cams);
+    splat_kernel<Real><<<OLPT_G(nblk(n * C)), 256, 0, s>>>(v, ctx->obj.xyz.as<double>(), n,
+                                                          ctx->obj.uv.as<double>(),
+                                                          W.otfp.as<Real>(), flags, all_cams);
   OLPT_CUDA(cudaGetLastError());
-  W.bins.build(W.pair_key.as<int>(), (int)(n * C), v.n_tiles, s);
   // algorithmic bytes: read the image, write the residual, for every computed camera
   double bytes = 0;
+  int rows = 1, cols = 1;
   for (int c = 0; c < C; ++c) {
+    rows = std::max(rows, v.orig[c].H);
+    cols = std::max(cols, v.orig[c].W);
     if (!(all_cams || ctx->cams_h[c].is_active)) continue;
     const int d = v.orig[c].dtype;
     const int esz = d == OLPT_U8 ? 1 : d == OLPT_U16 ? 2 : d == OLPT_F32 ? 4 : 8;
     bytes += (double)v.orig[c].H * v.orig[c].W * (esz + sizeof(Real));
   }
   const int pid = ctx->prof.begin(PROF_RESIDUAL, s);
-  residual_kernel<Real><<<OLPT_G(v.n_tiles), ctx->tune.residual_threads, 0, s>>>(v, ctx->obj.uv.as<double>(), W.otfp.as<Real>(),
-                                                  W.bins.start.as<int>(), W.bins.items.as<int>(),
-                                                  clamp, all_cams);
+  const int t = ctx->tune.residual_threads;
+  for (int y = 0; y < rows; y += 65535) {
+    // one grid row per image row (a second launch past the grid's 65,535 rows)
+    ShakeView part = v;
+    if (y > 0)
+      for (int c = 0; c < C; ++c) {
+        for (PlaneView* p : {&part.orig[c], &part.proj[c], &part.res[c]}) {
+          p->p += (int64_t)y * p->pitch;
+          p->H = std::max(0, p->H - y);
+        }
+      }
+    const dim3 grid((unsigned)nblk((cols + 3) / 4, t), (unsigned)std::min(rows - y, 65535), C);
+    residual_kernel<Real><<<OLPT_G(grid), t, 0, s>>>(part, clamp, all_cams);
+  }
   ctx->prof.end(PROF_RESIDUAL, pid, s, bytes);
   OLPT_CUDA(cudaGetLastError());
+  W.proj_clean = true;
 }
 
 // Shared memory of one object's arrays (struct Obj).  The stride between the objects of a
