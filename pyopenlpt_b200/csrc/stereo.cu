@@ -18,7 +18,7 @@
 //  * The depth-first search over build cameras is expanded breadth-first: level k
 //    holds all partial paths with k chosen cameras and the target camera of their
 //    next choice.  enum_kernel finds the detections of the target camera inside the
-//    path's strips, tri_kernel applies the back-projection test and the triangulation
+//    path's strips that pass the back-projection test, tri_kernel applies the triangulation
 //    gate to them.  Children are appended with atomics; the final candidate list is
 //    sorted by ids, so append order never shows.
 //  * 2D tests are decided in FP32 where the distance is clear of the tolerance by more
@@ -502,8 +502,8 @@ __device__ __forceinline__ double clamped_dot(const double a[3], const double b[
 // the smallest pairwise parallax lies inside (6, 174) degrees.
 constexpr double kCos6 = 0.99452189536827329;
 
-// A path and the position of one of its candidates on the target camera: inside all strips,
-// or (kEdge) so close to a strip's border that FP64 has to decide.
+// A path and the position of one of its candidates on the target camera: past all 2D tests,
+// or (kEdge) so close to a tolerance that FP64 has to decide.
 struct Pair {
   int path;
   unsigned g;
@@ -669,9 +669,13 @@ __global__ void __launch_bounds__(256) enum_log_kernel(const __grid_constant__ S
 // four rows at a time (K >= 2: one path a lane, whose strips meet in a few rows; K = 1: one
 // path a warp, its rows over the lanes), looks up their runs of positions together and walks
 // them.  FP32 decides each distance; pairs whose distance is within the bound of the tolerance
-// are marked for FP64.  Accepted pairs collect in shared memory, and one atomic serves a
-// buffer of them.
-constexpr int kPairBuf = 160;  // entries a warp; flushed above 128
+// are marked for FP64.  Detections inside the strips collect in a buffer of the warp, from
+// which 32 at a time take the back-projection test (its lines are gathers, and half of the
+// detections fail it; tested by tri_kernel, after a trip through memory, these left half of
+// its lanes idle: 419,000 detections on each of six cameras, 9.5 -> 7.9 ms a call); what
+// passes collects in a second buffer, and one atomic serves up to 128.
+constexpr int kHitBuf = 64;    // detections inside the strips; tested from 32 on
+constexpr int kPairBuf = 160;  // pairs; flushed above 128
 
 template <int K>
 __global__ void __launch_bounds__(256, K <= 2 ? 4 : 3) enum_kernel(
@@ -680,11 +684,13 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : 3) enum_kernel(
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kRowStep = K == 1 ? 32 : 1;
   __shared__ Pair buf_s[8][kPairBuf];
+  __shared__ uint2 hit_s[8][kHitBuf];  // (path's lane, position with its edge mark)
   const int lane = threadIdx.x & 31;
   Pair* buf = buf_s[threadIdx.x >> 5];
+  uint2* hit = hit_s[threadIdx.x >> 5];
   const PathN<K>* in = static_cast<const PathN<K>*>(in_v);
   const float tol = (float)v.tol2d;
-  int fill = 0;
+  int fill = 0, hits = 0;
   auto flush = [&] {
     int base = 0;
     if (lane == 0) base = atomicAdd(pair_count, fill);
@@ -751,6 +757,37 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : 3) enum_kernel(
       row_lo = (int)fminf(fmaxf(lo, 0.0f), (float)rows);
       row_hi = live ? (int)fmaxf(fminf(hi, (float)(rows - 1)), -1.0f) : -1;
     }
+    // the first min(hits, 32) entries of the hit buffer through the back-projection test
+    // (checkBackProjection, StereoMatch.cpp:1206-1227); the rest moves up
+    auto test_hits = [&] {
+      __syncwarp();
+      const int n = min(hits, 32);
+      const uint2 e = hit[lane < n ? lane : 0];
+      const int o = (int)e.x;
+      const int g = (int)(e.y & ~kEdge);
+      bool ok = lane < n, edge = (e.y & kEdge) != 0;
+      const unsigned cams = __shfl_sync(kFull, P.cams, o);
+#pragma unroll
+      for (int i = 0; i < K; ++i) {
+        const int id = __shfl_sync(kFull, P.ids[i], o);
+        const float2 p = v.fxy[id];
+        const float4 L = v.fl[(int64_t)g * v.n_cam + (int)((cams >> (4 * i)) & 15u)];
+        const float z = fabsf(fmaf(L.x, p.x, fmaf(L.y, p.y, L.z)));
+        const float b = v.eps + 5e-7f * fabsf(L.z);
+        ok = ok && !(z > tol + b);
+        edge = edge || !(z < tol - b);
+      }
+      const int path = __shfl_sync(kFull, pidx, o);
+      const unsigned m = __ballot_sync(kFull, ok);
+      if (ok)
+        buf[fill + __popc(m & ((1u << lane) - 1u))] = Pair{path, (unsigned)g | (edge ? kEdge : 0u)};
+      fill += __popc(m);
+      const uint2 rest = hit[min(n + lane, kHitBuf - 1)];
+      __syncwarp();
+      if (n + lane < hits) hit[lane] = rest;
+      hits -= n;
+      if (fill > kPairBuf - 32) flush();
+    };
     const int base = v.cell_off[t];
     const int n_row = max(0, row_hi - row_lo + 1);
     const int n_max = __reduce_max_sync(kFull, n_row);
@@ -805,13 +842,14 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : 3) enum_kernel(
         const unsigned m = __ballot_sync(kFull, ok);
         if (m) {
           if (ok)
-            buf[fill + __popc(m & ((1u << lane) - 1u))] =
-                Pair{pidx, (unsigned)q | (edge ? kEdge : 0u)};
-          fill += __popc(m);
-          if (fill > kPairBuf - 32) flush();
+            hit[hits + __popc(m & ((1u << lane) - 1u))] =
+                make_uint2(lane, (unsigned)q | (edge ? kEdge : 0u));
+          hits += __popc(m);
+          if (hits > kHitBuf - 32) test_hits();
         }
       }
     }
+    while (hits) test_hits();  // before the lanes take other paths
   }
   if (fill) flush();
 }
@@ -1001,11 +1039,10 @@ __device__ __forceinline__ int next_camera(const SmView& v, const PathN<N>& ch) 
   return next_camera_exact<N>(v, ch);
 }
 
-// Expand one level, second half: one thread per (path, candidate) pair.  The
-// back-projection test (in FP32 where it is clear, else all 2D tests in FP64), the quick
-// triangulation gate (computeMinParallaxDeg, calTriangulateTol, TriangulationCheckWithTol:
-// StereoMatch.cpp:1072-1141), then the child path (terminal, or with its next target camera).
-// Bound by the gathers of the candidates' lines (about 150 B each).
+// Expand one level, second half: one thread per (path, candidate) pair.  All 2D tests in FP64
+// for the pairs that FP32 could not decide, the quick triangulation gate (computeMinParallaxDeg,
+// calTriangulateTol, TriangulationCheckWithTol: StereoMatch.cpp:1072-1141), then the child path
+// (terminal, or with its next target camera).  Bound by the gathers of the lines of sight.
 template <int K>
 __global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
     const __grid_constant__ SmView v, const void* in_v, const Pair* pairs, int n_pairs,
@@ -1020,18 +1057,7 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
     const Pair pr = pairs[gi];
     const PathN<K> P = static_cast<const PathN<K>*>(in_v)[pr.path];
     const int g = (int)(pr.g & ~kEdge);
-    bool edge = (pr.g & kEdge) != 0;
-    const float tol = (float)v.tol2d;
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      const float4 L = v.fl[(int64_t)g * v.n_cam + P.cam(i)];
-      const float2 p = v.fxy[P.ids[i]];
-      const float z = fabsf(fmaf(L.x, p.x, fmaf(L.y, p.y, L.z)));
-      const float e = v.eps + 5e-7f * fabsf(L.z);
-      ok = ok && !(z > tol + e);
-      edge = edge || !(z < tol - e);
-    }
-    if (ok && edge) ok = exact_2d<K, false>(v, P, g);
+    if (pr.g & kEdge) ok = exact_2d<K, false>(v, P, g);
     if (ok) {
       Rays<K> r;
 #pragma unroll
