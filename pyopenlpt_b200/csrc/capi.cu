@@ -159,6 +159,11 @@ OtfView otf_view(olpt_ctx* ctx) {
   return v;
 }
 
+__global__ void pair_xy_kernel(const double* x, const double* y, int64_t n, double2* out) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) out[i] = make_double2(x[i], y[i]);
+}
+
 }  // namespace olpt
 
 using namespace olpt;
@@ -178,6 +183,11 @@ olpt_status_t olpt_ctx_create(olpt_ctx** out, int device) {
     return OLPT_ERR_CUDA;
   }
   ctx->own_stream = true;
+  // without it the read-backs go to pageable memory
+  if (cudaMallocHost(&ctx->pinned.p, kReadBackBytes) == cudaSuccess)
+    ctx->pinned.bytes = kReadBackBytes;
+  else
+    cudaGetLastError();
   *out = ctx;
   return OLPT_OK;
 }
@@ -540,20 +550,16 @@ olpt_status_t olpt_get_peaks(olpt_ctx* ctx, int cam, double* xy, int32_t* rc, in
     const int64_t n = std::min<int64_t>(cap, ctx->det_counts_h[cam]);
     if (n <= 0) return;
     Dets& d = ctx->dets[cam];
+    ReadBack rb(ctx);
     if (xy) {
-      std::vector<double> hx(n), hy(n);
-      OLPT_CUDA(cudaMemcpyAsync(hx.data(), d.x.p, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-      OLPT_CUDA(cudaMemcpyAsync(hy.data(), d.y.p, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-      OLPT_CUDA(cudaStreamSynchronize(ctx->stream));
-      for (int64_t i = 0; i < n; ++i) {
-        xy[2 * i] = hx[i];
-        xy[2 * i + 1] = hy[i];
-      }
+      ctx->scratch.ensure((size_t)n * sizeof(double2), ctx->stream);
+      pair_xy_kernel<<<OLPT_G((int)((n + 255) / 256)), 256, 0, ctx->stream>>>(
+          d.x.as<double>(), d.y.as<double>(), n, ctx->scratch.as<double2>());
+      OLPT_CUDA(cudaGetLastError());
+      rb.add(xy, ctx->scratch.p, (size_t)n * sizeof(double2));
     }
-    if (rc) {
-      OLPT_CUDA(cudaMemcpyAsync(rc, d.rc.p, n * sizeof(int2), cudaMemcpyDeviceToHost, ctx->stream));
-      OLPT_CUDA(cudaStreamSynchronize(ctx->stream));
-    }
+    if (rc) rb.add(rc, d.rc.p, n * sizeof(int2));
+    rb.finish();
   });
 }
 
@@ -763,8 +769,8 @@ olpt_status_t olpt_prune_matches_device(olpt_ctx* ctx, int n_cam, int64_t M, con
 olpt_status_t olpt_get_matches(olpt_ctx* ctx, int32_t* ids, double* xyz) {
   return guard(ctx, [&] {
     StereoResult& r = ctx->sm_result;
-    stereo_result_to_host(ctx, r);
     const int n = r.n_cam;
+    if (r.on_device) return stereo_matches(ctx, r, ids, xyz);
     int64_t k = 0;
     for (size_t j = 0; j < r.e.size(); ++j) {
       if (!r.selected[j]) continue;
@@ -835,13 +841,12 @@ olpt_status_t olpt_objects_download(olpt_ctx* ctx, double* xyz, double* uv, uint
   return guard(ctx, [&] {
     const int64_t n = ctx->obj.n;
     if (n <= 0) return;
-    cudaStream_t s = ctx->stream;
-    if (xyz) OLPT_CUDA(cudaMemcpyAsync(xyz, ctx->obj.xyz.p, n * 3 * 8, cudaMemcpyDeviceToHost, s));
-    if (uv)
-      OLPT_CUDA(cudaMemcpyAsync(uv, ctx->obj.uv.p, n * ctx->n_cam * 2 * 8, cudaMemcpyDeviceToHost, s));
-    if (flags) OLPT_CUDA(cudaMemcpyAsync(flags, ctx->obj.flags.p, n, cudaMemcpyDeviceToHost, s));
-    if (score) OLPT_CUDA(cudaMemcpyAsync(score, ctx->obj.score.p, n * 8, cudaMemcpyDeviceToHost, s));
-    OLPT_CUDA(cudaStreamSynchronize(s));
+    ReadBack rb(ctx);
+    if (xyz) rb.add(xyz, ctx->obj.xyz.p, n * 3 * 8);
+    if (uv) rb.add(uv, ctx->obj.uv.p, n * ctx->n_cam * 2 * 8);
+    if (flags) rb.add(flags, ctx->obj.flags.p, n);
+    if (score) rb.add(score, ctx->obj.score.p, n * 8);
+    rb.finish();
   });
 }
 
@@ -1122,13 +1127,10 @@ olpt_status_t olpt_ipr_result(olpt_ctx* ctx, double* xyz, double* uv) {
   return guard(ctx, [&] {
     const int64_t n = ctx->ipr.n_out;
     if (n <= 0) return;
-    if (xyz)
-      OLPT_CUDA(cudaMemcpyAsync(xyz, ctx->ipr.out_xyz.p, n * 3 * sizeof(double),
-                                cudaMemcpyDeviceToHost, ctx->stream));
-    if (uv)
-      OLPT_CUDA(cudaMemcpyAsync(uv, ctx->ipr.out_uv.p, n * ctx->n_cam * 2 * sizeof(double),
-                                cudaMemcpyDeviceToHost, ctx->stream));
-    OLPT_CUDA(cudaStreamSynchronize(ctx->stream));
+    ReadBack rb(ctx);
+    if (xyz) rb.add(xyz, ctx->ipr.out_xyz.p, n * 3 * sizeof(double));
+    if (uv) rb.add(uv, ctx->ipr.out_uv.p, n * ctx->n_cam * 2 * sizeof(double));
+    rb.finish();
   });
 }
 

@@ -126,9 +126,7 @@ void append_result(olpt_ctx* ctx) {
   W.pos.ensure((n + 1) * sizeof(int), s);
   keep_flags_kernel<<<OLPT_G(nblk(n)), 256, 0, s>>>(ctx->obj.flags.as<uint8_t>(), n, W.keep.as<int>());
   exclusive_scan(W.keep.as<int>(), (int)n, W.pos.as<int>(), W.scan_tmp, s);
-  int kept = 0;
-  OLPT_CUDA(cudaMemcpyAsync(&kept, W.pos.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-  OLPT_CUDA(cudaStreamSynchronize(s));
+  const int kept = read_back(ctx, W.pos.as<int>() + n);
   const int64_t need = W.n_out + kept;
   if (need > W.cap_out) {
     // grow, keeping what is there

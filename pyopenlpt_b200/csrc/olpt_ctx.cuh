@@ -260,6 +260,8 @@ bool prune_select_device(olpt_ctx* ctx, const PruneView& pv, int M, int n_cam,
                          int64_t total_points, char* selected);
 // Download a device-resident stereo result (no-op for a host one).
 void stereo_result_to_host(olpt_ctx* ctx, StereoResult& r);
+// the selected candidates of a result that is on the device, read back to the host
+void stereo_matches(olpt_ctx* ctx, const StereoResult& r, int* ids, double* xyz);
 // The kept matches become the context's 3D objects (triangulateMatch order); returns
 // their number.
 int64_t stereo_objects(olpt_ctx* ctx, const StereoResult& r);
@@ -451,7 +453,61 @@ struct olpt_ctx {
   // optional per-kernel event timing
   olpt::Prof prof;
 
-  // scratch
+  // scratch, and the pinned block of the read-backs
   olpt::DevBuf scratch;
   olpt::HostBuf pinned;
 };
+
+namespace olpt {
+
+// Results read back to the host: copies into the context's pinned block, one synchronisation,
+// and from there to where they belong.  A copy to pageable memory waits for the stream by
+// itself, and goes through a staging area of the driver (a detection list of 1,700 spots in
+// three of them: 30 us, this way 12 us).  What does not fit into the block (results so large
+// that the copy itself counts) is copied directly.  One user at a time, like the context.
+constexpr size_t kReadBackBytes = 1 << 20;
+
+class ReadBack {
+ public:
+  explicit ReadBack(olpt_ctx* c) : c_(c) {}
+  void add(void* dst, const void* src, size_t bytes) {
+    if (!bytes) return;
+    if (n_ < kMax && c_->pinned.p && used_ + bytes <= kReadBackBytes) {
+      char* at = c_->pinned.as<char>() + used_;
+      OLPT_CUDA(cudaMemcpyAsync(at, src, bytes, cudaMemcpyDeviceToHost, c_->stream));
+      part_[n_++] = {dst, at, bytes};
+      used_ += (bytes + 15) / 16 * 16;
+    } else {
+      OLPT_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c_->stream));
+    }
+  }
+  void finish() {
+    OLPT_CUDA(cudaStreamSynchronize(c_->stream));
+    for (int i = 0; i < n_; ++i) std::memcpy(part_[i].dst, part_[i].at, part_[i].bytes);
+    n_ = 0;
+    used_ = 0;
+  }
+
+ private:
+  static constexpr int kMax = 8;
+  struct Part {
+    void* dst;
+    const void* at;
+    size_t bytes;
+  };
+  olpt_ctx* c_;
+  Part part_[kMax];
+  int n_ = 0;
+  size_t used_ = 0;
+};
+
+template <class T>
+T read_back(olpt_ctx* c, const T* src) {
+  T v;
+  ReadBack rb(c);
+  rb.add(&v, src, sizeof(T));
+  rb.finish();
+  return v;
+}
+
+}  // namespace olpt

@@ -984,9 +984,9 @@ void find_peaks_device(olpt_ctx* ctx, double min_int, bool sync_counts) {
   ctx->det_counts_h.assign(ctx->n_cam, 0);
   if (sync_counts) {
     int64_t h[kDcErr + 1];
-    OLPT_CUDA(cudaMemcpyAsync(h, ctx->det_counts.p, sizeof(h), cudaMemcpyDeviceToHost,
-                              ctx->stream));
-    OLPT_CUDA(cudaStreamSynchronize(ctx->stream));
+    ReadBack rb(ctx);
+    rb.add(h, ctx->det_counts.p, sizeof(h));
+    rb.finish();
     OLPT_REQUIRE(h[kDcErr] == 0, OLPT_ERR_TIMEOUT,
                  "peak detection: a staging or look-back wait timed out");
     for (int c = 0; c < ctx->n_cam; ++c) ctx->det_counts_h[c] = h[c];

@@ -1579,9 +1579,7 @@ static void learned_impl(olpt_ctx* ctx, const ShakeParams& sp) {
                                                         n, lp.out_scale_mm, (float)lp.ghost_logit,
                                                         M.keep.as<int>());
     exclusive_scan(M.keep.as<int>(), (int)n, M.pos.as<int>(), ctx->shk.scan_tmp, s);
-    int kept = 0;
-    OLPT_CUDA(cudaMemcpyAsync(&kept, M.pos.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-    OLPT_CUDA(cudaStreamSynchronize(s));
+    const int kept = read_back(ctx, M.pos.as<int>() + n);
     // compacted copies (through the scratch pair act / nres, then back)
     M.act.ensure((size_t)(n + 1) * 3 * sizeof(double), s);
     M.nres.ensure((size_t)(n + 1) * 3 * sizeof(double), s);
@@ -1615,9 +1613,7 @@ static void learned_impl(olpt_ctx* ctx, const ShakeParams& sp) {
         lp.fallback_residual, M.act.as<uint8_t>(), ctx->obj.xyz.as<double>(),
         M.start_xyz.as<double>(), ctx->obj.score.as<double>(), cnt);
     OLPT_CUDA(cudaGetLastError());
-    int n_fb = 0;
-    OLPT_CUDA(cudaMemcpyAsync(&n_fb, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
-    OLPT_CUDA(cudaStreamSynchronize(s));
+    const int n_fb = read_back(ctx, cnt);
     M.n_fallback += n_fb;
     M.n_learned += n;
     if (n_fb > 0)

@@ -579,10 +579,11 @@ T* upload(DevBuf& b, const std::vector<T>& v, cudaStream_t s) {
 }
 
 template <class T>
-std::vector<T> download(const T* p, size_t n, cudaStream_t s) {
+std::vector<T> download(olpt_ctx* ctx, const T* p, size_t n) {
   std::vector<T> v(n);
-  if (n) OLPT_CUDA(cudaMemcpyAsync(v.data(), p, n * sizeof(T), cudaMemcpyDeviceToHost, s));
-  OLPT_CUDA(cudaStreamSynchronize(s));
+  ReadBack rb(ctx);
+  rb.add(v.data(), p, n * sizeof(T));
+  rb.finish();
   return v;
 }
 
@@ -746,7 +747,7 @@ void snapshot_images(olpt_ctx* ctx) {
 // IPR::runIPR on the current images; the objects come back to the host.
 std::vector<double> run_ipr_host(olpt_ctx* ctx) {
   ipr_device(ctx, ctx->stb.ipr);
-  return download(ctx->ipr.out_xyz.as<double>(), (size_t)ctx->ipr.n_out * 3, ctx->stream);
+  return download(ctx, ctx->ipr.out_xyz.as<double>(), (size_t)ctx->ipr.n_out * 3);
 }
 
 // STB::saveTracks (STB.cpp:967-1004) + Track::saveTrack + Tracer3D::saveObject3D
@@ -869,7 +870,7 @@ const double* cal_pred_field(olpt_ctx* ctx, int i) {
                                                    W.flag.as<int>());
   ctx->prof.end(PROF_PF, pid, s, (double)(np + nc) * 24.0 + n_grid * 24.0);
   OLPT_CUDA(cudaGetLastError());
-  const int ovf = download(W.flag.as<int>(), 1, s)[0];
+  const int ovf = download(ctx, W.flag.as<int>(), 1)[0];
   OLPT_REQUIRE(!ovf, OLPT_ERR_UNSUPPORTED,
                "predictive field: more than 4096 objects inside one search cube");
   double* A = W.field.as<double>();
@@ -892,7 +893,7 @@ const double* cal_pred_field(olpt_ctx* ctx, int i) {
   }
   if (!S.p.output_path.empty()) {
     const int fid = i + S.p.frame_start;  // named as in runInitPhase (STB.cpp:121-123)
-    save_pred_field(download(A, 3 * (size_t)n_grid, s),
+    save_pred_field(download(ctx, A, 3 * (size_t)n_grid),
                     S.p.output_path + "PredField_" + std::to_string(fid) + "_" +
                         std::to_string(fid + 1) + ".csv");
   }
@@ -924,7 +925,7 @@ void build_from_pf(olpt_ctx* ctx, int idx, const double* d_field, int frame) {
       nn_kernel<<<OLPT_G(nblk(n_sa)), 256, 0, s>>>(W.b.as<double>(), n_sa, go, r * r,
                                                   W.link.as<int>());
       OLPT_CUDA(cudaGetLastError());
-      link = download(W.link.as<int>(), n_sa, s);
+      link = download(ctx, W.link.as<int>(), n_sa);
     }
     TrackList kept;
     for (int j = 0; j < n_sa; ++j) {
@@ -1021,8 +1022,12 @@ void conv_phase(olpt_ctx* ctx, int frame) {
     predict_kernel<<<OLPT_G(nblk(n_la, 128)), 128, 0, s>>>(d_pts, d_np, n_la, v, W.b.as<double>(),
                                                           W.link.as<int>());
     OLPT_CUDA(cudaGetLastError());
-    pred = download(W.b.as<double>(), 3 * (size_t)n_la, s);
-    const std::vector<int> in_range = download(W.link.as<int>(), n_la, s);
+    pred.resize(3 * (size_t)n_la);
+    std::vector<int> in_range(n_la);
+    ReadBack rb(ctx);
+    rb.add(pred.data(), W.b.p, pred.size() * sizeof(double));
+    rb.add(in_range.data(), W.link.p, in_range.size() * sizeof(int));
+    rb.finish();
     TrackList kept = take_list(S.spare_long, n_la);
     size_t w = 0;
     for (int i = 0; i < n_la; ++i) {
@@ -1065,12 +1070,16 @@ void conv_phase(olpt_ctx* ctx, int frame) {
     resume();
     t_part = std::chrono::steady_clock::now();
     const int64_t n_out = ctx->obj.n;
-    const std::vector<double> sx0 = download(ctx->obj.xyz.as<double>(), 3 * (size_t)n_out, s);
-    const std::vector<uint8_t> fl0 = download(ctx->obj.flags.as<uint8_t>(), (size_t)n_out, s);
+    std::vector<double> sx0(3 * (size_t)n_out);
+    std::vector<uint8_t> fl0(n_out);
+    ReadBack rb(ctx);
+    rb.add(sx0.data(), ctx->obj.xyz.p, sx0.size() * sizeof(double));
+    rb.add(fl0.data(), ctx->obj.flags.p, fl0.size());
+    rb.finish();
     std::vector<double> sx(3 * (size_t)n_la, 0.0);
     std::vector<uint8_t> fl(n_la, 1);
     if (learned) {
-      const std::vector<int> keep = download(ctx->mlp.keep.as<int>(), n_la, s);
+      const std::vector<int> keep = download(ctx, ctx->mlp.keep.as<int>(), n_la);
       int64_t j = 0;
       for (int i = 0; i < n_la; ++i)
         if (keep[i] && j < n_out) {
@@ -1119,7 +1128,7 @@ void conv_phase(olpt_ctx* ctx, int frame) {
     W.link.ensure((n_obj + 1) * sizeof(int), s);
     repeat_kernel<<<OLPT_G(nblk(n_obj)), 256, 0, s>>>(d_obj, n_obj, g, tol, W.link.as<int>());
     OLPT_CUDA(cudaGetLastError());
-    const std::vector<int> rep = download(W.link.as<int>(), n_obj, s);
+    const std::vector<int> rep = download(ctx, W.link.as<int>(), n_obj);
     size_t w = 0;
     for (int i = 0; i < n_obj; ++i)
       if (!rep[i]) {
@@ -1165,7 +1174,7 @@ void conv_phase(olpt_ctx* ctx, int frame) {
       link_kernel<<<OLPT_G(nblk(n_sa, 128)), 128, 0, s>>>(d_pl, d_len, n_sa, tg, d_disp, go, base_r,
                                                          W.link.as<int>());
       OLPT_CUDA(cudaGetLastError());
-      link = download(W.link.as<int>(), n_sa, s);
+      link = download(ctx, W.link.as<int>(), n_sa);
     }
     // first come, first served
     std::vector<int> owner(n_obj, -1);
@@ -1222,7 +1231,7 @@ void conv_phase(olpt_ctx* ctx, int frame) {
     linfit_kernel<<<OLPT_G(nblk(n_la)), 256, 0, s>>>(d_pts, d_len, n_la, n_pts, d_k,
                                                     W.link.as<int>());
     OLPT_CUDA(cudaGetLastError());
-    const std::vector<int> ok = download(W.link.as<int>(), n_la, s);
+    const std::vector<int> ok = download(ctx, W.link.as<int>(), n_la);
     TrackList kept = take_list(S.spare_long, n_la);
     for (int i = 0; i < n_la; ++i) {
       TrackH& tr = S.long_active[i];

@@ -1166,10 +1166,10 @@ bool prune_select_device(olpt_ctx* ctx, const PruneView& pv, int M, int n_cam,
   PruneWork& P = ctx->prune;
   prune_device(P, pv, M, n_cam, total_points, s);
   int cnt[PC_N];
-  OLPT_CUDA(cudaMemcpyAsync(cnt, P.counts.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
-  OLPT_CUDA(cudaMemcpyAsync(&P.n_sel, P.spos.as<int>() + M, sizeof(int), cudaMemcpyDeviceToHost,
-                            s));
-  OLPT_CUDA(cudaStreamSynchronize(s));
+  ReadBack rb(ctx);
+  rb.add(cnt, P.counts.p, sizeof(cnt));
+  rb.add(&P.n_sel, P.spos.as<int>() + M, sizeof(int));
+  rb.finish();
   if (cnt[PC_FLAG]) return false;
   const int G = cnt[PC_BOTH];
   if (!cnt[PC_REPLACE]) {
@@ -1331,10 +1331,7 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
   W.counters.ensure(8 * sizeof(int), s);
   int* cnt = W.counters.as<int>();
   auto read_count = [&](int idx) {
-    int h = 0;
-    OLPT_CUDA(cudaMemcpyAsync(&h, cnt + idx, sizeof(int), cudaMemcpyDeviceToHost, s));
-    OLPT_CUDA(cudaStreamSynchronize(s));
-    return h;
+    return read_back(ctx, cnt + idx);
   };
   const int64_t n_ref = v.raw_off[ref + 1] - v.raw_off[ref];
   int cap_a = (int)std::max<int64_t>(n_ref, 1024);
@@ -1425,8 +1422,9 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
       ctx->prof.end(PROF_STEREO, pid, s, 0.0);
       OLPT_CUDA(cudaGetLastError());
       int h[2];
-      OLPT_CUDA(cudaMemcpyAsync(h, cnt + 1, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-      OLPT_CUDA(cudaStreamSynchronize(s));
+      ReadBack rb(ctx);
+      rb.add(h, cnt + 1, sizeof(h));
+      rb.finish();
       if (h[0] > out_cap || h[1] > term_cap) {  // grow and redo this level
         out_cap = std::max(out_cap, h[0] + h[0] / 4 + 1024);
         term_cap = std::max(term_cap, h[1] + h[1] / 4 + 1024);
@@ -1503,14 +1501,40 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
   prune_candidates(res, counts, active);
 }
 
+// The selected candidates' points and (when asked for) ids, in candidate order.
 __global__ void sel_gather_kernel(const uint8_t* sel, const int* pos, int M, const double* X,
-                                  double* out) {
+                                  double* out, const int* ids, int n, int* out_ids) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= M || !sel[i]) return;
-  const int k = pos[i];
-  out[3 * k] = X[3 * i];
-  out[3 * k + 1] = X[3 * i + 1];
-  out[3 * k + 2] = X[3 * i + 2];
+  const int64_t k = pos[i], j = i;
+  if (out) {
+    out[3 * k] = X[3 * j];
+    out[3 * k + 1] = X[3 * j + 1];
+    out[3 * k + 2] = X[3 * j + 2];
+  }
+  if (out_ids)
+    for (int c = 0; c < n; ++c) out_ids[k * n + c] = ids[j * n + c];
+}
+
+// The matches of a result that is still on the device: gathered there (a tenth of the
+// candidates), so that the others need not come over.
+void stereo_matches(olpt_ctx* ctx, const StereoResult& r, int* ids, double* xyz) {
+  cudaStream_t s = ctx->stream;
+  PruneWork& P = ctx->prune;
+  const int M = (int)r.M, n = r.n_cam;
+  const size_t k = (size_t)P.n_sel, b_xyz = k * 3 * sizeof(double), b_ids = k * n * sizeof(int);
+  if (k == 0 || (!ids && !xyz)) return;
+  ctx->scratch.ensure(b_xyz + b_ids, s);
+  double* dx = ctx->scratch.as<double>();
+  int* di = reinterpret_cast<int*>(ctx->scratch.as<char>() + b_xyz);
+  sel_gather_kernel<<<OLPT_G(nblk(M)), 256, 0, s>>>(P.sel.as<uint8_t>(), P.spos.as<int>(), M,
+                                                   P.X_s.as<double>(), xyz ? dx : nullptr,
+                                                   P.ids_s.as<int>(), n, ids ? di : nullptr);
+  OLPT_CUDA(cudaGetLastError());
+  ReadBack rb(ctx);
+  if (ids) rb.add(ids, di, b_ids);
+  if (xyz) rb.add(xyz, dx, b_xyz);
+  rb.finish();
 }
 
 void stereo_result_to_host(olpt_ctx* ctx, StereoResult& r) {
@@ -1547,7 +1571,8 @@ int64_t stereo_objects(olpt_ctx* ctx, const StereoResult& r) {
     ctx->obj.n = n;
     if (n > 0)
       sel_gather_kernel<<<OLPT_G(nblk(M)), 256, 0, s>>>(P.sel.as<uint8_t>(), P.spos.as<int>(), M,
-                                                       P.X_s.as<double>(), ctx->obj.xyz.as<double>());
+                                                       P.X_s.as<double>(), ctx->obj.xyz.as<double>(),
+                                                       nullptr, 0, nullptr);
     OLPT_CUDA(cudaGetLastError());
     return n;
   }
