@@ -652,14 +652,16 @@ __device__ __noinline__ void visit_cells(const SmView& v, const PathN<K>& P, int
 // visit_cells for every path: a warp per path at level 1, else a thread.
 template <int K>
 __global__ void __launch_bounds__(256) enum_log_kernel(const __grid_constant__ SmView v,
-                                                       const void* in_v, int n_in, Pair* pairs,
-                                                       int* pair_count, int pair_cap) {
+                                                       const void* in_v, const int* n_ptr,
+                                                       int in_cap, Pair* pairs, int* pair_count,
+                                                       int pair_cap) {
   constexpr int L = K == 1 ? 32 : 1;
-  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  const int pidx = gt / L;
-  if (pidx >= n_in) return;
-  visit_cells<K, true>(v, static_cast<const PathN<K>*>(in_v)[pidx], pidx, gt % L, L, pairs,
-                       pair_count, pair_cap);
+  const int n_in = *n_ptr;
+  if (n_in > in_cap) return;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; gt / L < n_in; gt += step)
+    visit_cells<K, true>(v, static_cast<const PathN<K>*>(in_v)[gt / L], (int)(gt / L),
+                         (int)(gt % L), L, pairs, pair_count, pair_cap);
 }
 
 // Expand one level, first half: the detections of the target camera inside the strips of a
@@ -679,10 +681,12 @@ constexpr int kPairBuf = 160;  // pairs; flushed above 128
 
 template <int K>
 __global__ void __launch_bounds__(256, K <= 2 ? 4 : 3) enum_kernel(
-    const __grid_constant__ SmView v, const void* in_v, int n_in, Pair* pairs, int* pair_count,
-    int pair_cap) {
+    const __grid_constant__ SmView v, const void* in_v, const int* n_ptr, int in_cap, Pair* pairs,
+    int* pair_count, int pair_cap) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kRowStep = K == 1 ? 32 : 1;
+  const int n_in = *n_ptr;
+  if (n_in > in_cap) return;  // paths are missing: the level before is repeated
   __shared__ Pair buf_s[8][kPairBuf];
   __shared__ uint2 hit_s[8][kHitBuf];  // (path's lane, position with its edge mark)
   const int lane = threadIdx.x & 31;
@@ -1045,12 +1049,15 @@ __device__ __forceinline__ int next_camera(const SmView& v, const PathN<N>& ch) 
 // (terminal, or with its next target camera).  Bound by the gathers of the lines of sight.
 template <int K>
 __global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
-    const __grid_constant__ SmView v, const void* in_v, const Pair* pairs, int n_pairs,
-    void* out_v, int* out_count, int out_cap, Path* term, int* term_count, int term_cap) {
+    const __grid_constant__ SmView v, const void* in_v, const Pair* pairs, const int* n_ptr,
+    int pair_cap, void* out_v, int* out_count, int out_cap) {
   __shared__ int s_cnt[8], s_base;
-  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool last = K + 1 == v.m;
+  const int n_pairs = *n_ptr;
+  if (n_pairs > pair_cap) return;  // pairs are missing: the level is repeated
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gi - (int)threadIdx.x >= n_pairs) return;
   PathN<K + 1> ch;
   bool ok = gi < n_pairs;
   if (ok) {
@@ -1097,7 +1104,7 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
       s_cnt[w] = t;
       t += k;
     }
-    s_base = t ? atomicAdd(last ? term_count : out_count, t) : 0;
+    s_base = t ? atomicAdd(out_count, t) : 0;
   }
   __syncthreads();
   if (!ok) return;
@@ -1106,7 +1113,7 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
     if (slot < out_cap) static_cast<PathN<K + 1>*>(out_v)[slot] = ch;
     return;
   }
-  if (slot >= term_cap) return;
+  if (slot >= out_cap) return;
   Path full;
 #pragma unroll
   for (int i = 0; i < OLPT_MAX_CAM; ++i) {
@@ -1115,16 +1122,14 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
   }
   full.k = K + 1;
   full.target = -1;
-  term[slot] = full;
+  static_cast<Path*>(out_v)[slot] = full;
 }
 
 // StereoMatch::checkMatch, case "every active camera was used to build"
 // (StereoMatch.cpp:520-540): triangulate in camera order, gate on tol_3d and limit.
-__global__ void check_kernel(const __grid_constant__ SmView v, const Path* term, int n_term, int* cand_ids,
-                             double* cand_e, double* cand_x, int* cand_count, int cap) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_term) return;
-  const Path P = term[i];
+__device__ __forceinline__ void check_path(const SmView& v, const Path& P, int* cand_ids,
+                                           double* cand_e, double* cand_x, int* cand_count,
+                                           int cap) {
   int ids[OLPT_MAX_CAM];
   for (int c = 0; c < v.n_cam; ++c) ids[c] = -1;
   for (int j = 0; j < P.k; ++j) ids[P.cams[j]] = P.ids[j];
@@ -1151,6 +1156,16 @@ __global__ void check_kernel(const __grid_constant__ SmView v, const Path* term,
   cand_x[3 * slot] = X[0];
   cand_x[3 * slot + 1] = X[1];
   cand_x[3 * slot + 2] = X[2];
+}
+
+__global__ void check_kernel(const __grid_constant__ SmView v, const Path* term, const int* n_ptr,
+                             int* cand_ids, double* cand_e, double* cand_x, int* cand_count,
+                             int cap) {
+  const int n = *n_ptr;
+  if (n > cap) return;
+  const int step = gridDim.x * blockDim.x;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step)
+    check_path(v, term[i], cand_ids, cand_e, cand_x, cand_count, cap);
 }
 
 }  // namespace
@@ -1327,16 +1342,21 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
   }
   OLPT_CUDA(cudaGetLastError());
 
-  // breadth-first expansion of the build DFS
-  W.counters.ensure(8 * sizeof(int), s);
+  // Breadth-first expansion of the build DFS.  Counters: [0] the paths of level 1, [2l - 1] the
+  // pairs of level l, [2l] its children (at the last level, the complete paths), [15] the
+  // candidates.  The kernels read the counts on the device, and one whose input exceeds its
+  // buffer does nothing, so that a level can be repeated over larger buffers.
+  constexpr int kCand = 15;
+  static_assert(2 * (OLPT_MAX_CAM - 1) < kCand, "stereo counters");
+  W.counters.ensure(16 * sizeof(int), s);
   int* cnt = W.counters.as<int>();
-  auto read_count = [&](int idx) {
-    return read_back(ctx, cnt + idx);
-  };
+  int h[16] = {0};
   const int64_t n_ref = v.raw_off[ref + 1] - v.raw_off[ref];
-  int cap_a = (int)std::max<int64_t>(n_ref, 1024);
+  const int cap_a = (int)std::max<int64_t>(n_ref, 1024);
+  const int last = v.m - 1;
   // bytes of a partial path of k points
-  auto rec = [](int k) -> size_t {
+  auto rec = [&](int k) -> size_t {
+    if (k >= v.m) return sizeof(Path);
     switch (k) {
       case 1: return sizeof(PathN<1>);
       case 2: return sizeof(PathN<2>);
@@ -1347,29 +1367,47 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
       default: return sizeof(PathN<8>);
     }
   };
-  W.path_a.ensure(cap_a * rec(1), s);
-  OLPT_CUDA(cudaMemsetAsync(cnt, 0, 8 * sizeof(int), s));
+  // A look at the counts after every step lets the buffers and grids follow them, but leaves
+  // the device idle for about 10 us.  Up to 16,384 seeds the levels are enqueued without one
+  // (buffers of 16 paths and 8 pairs a seed or what earlier calls needed; 10,000 detections on
+  // each of four cameras: 860 -> 745 us a call).  Above, the looks do not show, while grids
+  // sized by the buffers do (51,000 detections: 114 ms a track sequence with the looks, 117
+  // to 120 without).
+  bool look = v.near_band > 0.0 || n_ref > 16384;
+  const int64_t path_guess = std::min<int64_t>(INT32_MAX, std::max<int64_t>(16 * n_ref, 4096));
+  int pair_cap = (int)std::min<int64_t>(INT32_MAX, std::max<int64_t>(8 * n_ref, 4096));
+  // buffers are grow-only: their capacity from earlier calls avoids a redo
+  pair_cap = (int)std::max<int64_t>(pair_cap, (int64_t)(W.pairs.bytes / sizeof(Pair)) - 1);
+  DevBuf* in_buf = &W.path_a;
+  DevBuf* out_buf = &W.path_b;
+  W.path_a.ensure(std::max(cap_a * rec(1), look ? 0 : (size_t)path_guess * rec(last)), s);
+  if (!look) W.path_b.ensure((size_t)path_guess * rec(last), s);
+  OLPT_CUDA(cudaMemsetAsync(cnt, 0, 16 * sizeof(int), s));
   if (n_ref > 0)
     seed_kernel<<<OLPT_G(nblk(n_ref)), 256, 0, s>>>(v, ref, W.path_a.as<PathN<1>>(), cnt, cap_a);
   OLPT_CUDA(cudaGetLastError());
-  int n_in = read_count(0);
-  int term_cap = (int)std::max<int64_t>(4 * n_ref, 4096);
-  W.term.ensure(term_cap * sizeof(Path), s);
-  int n_term = 0;
-  DevBuf* in_buf = &W.path_a;
-  DevBuf* out_buf = &W.path_b;
-  int out_cap = (int)std::max<int64_t>(16 * (int64_t)n_in, 4096);
-  int pair_cap = (int)std::max<int64_t>(8 * (int64_t)n_in, 4096);
-  for (int level = 1; level < v.m && n_in > 0; ++level) {
-    // candidates of every path that pass the 2D tests
-    int n_pairs = 0;
-    // buffers are grow-only: their capacity from earlier calls avoids a redo
-    pair_cap = (int)std::max<int64_t>(pair_cap, (int64_t)(W.pairs.bytes / sizeof(Pair)) - 1);
-    for (;;) {
+
+  int in_cap = cap_a, out_cap = 0, cap_c = 0, level = 1;
+  bool enumerate = true;
+  auto check = [&] {
+    W.cand_ids.ensure((size_t)cap_c * n_cam * sizeof(int), s);
+    W.cand_e.ensure((size_t)cap_c * sizeof(double), s);
+    W.cand_x.ensure((size_t)cap_c * 3 * sizeof(double), s);
+    check_kernel<<<OLPT_G(std::min(nblk(cap_c, 128), 148 * 64)), 128, 0, s>>>(
+        v, W.term.as<Path>(), cnt + 2 * last, W.cand_ids.as<int>(), W.cand_e.as<double>(),
+        W.cand_x.as<double>(), cnt + kCand, cap_c);
+    OLPT_CUDA(cudaGetLastError());
+  };
+  auto read_counts = [&] {
+    ReadBack rb(ctx);
+    rb.add(h, cnt, sizeof(h));
+    rb.finish();
+  };
+  int caps_pair[OLPT_MAX_CAM + 1], caps_out[OLPT_MAX_CAM + 1];
+  while (n_ref > 0) {
+    const bool log = v.near_band > 0.0;
+    if (enumerate) {
       W.pairs.ensure((size_t)pair_cap * sizeof(Pair), s);
-      OLPT_CUDA(cudaMemsetAsync(cnt + 4, 0, sizeof(int), s));
-      const int pid = ctx->prof.begin(PROF_STEREO, s);
-      const bool log = v.near_band > 0.0;
       auto kern = log ? enum_log_kernel<1> : enum_kernel<1>;
       switch (level) {
         case 1: break;
@@ -1380,76 +1418,87 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
         case 6: kern = log ? enum_log_kernel<6> : enum_kernel<6>; break;
         default: kern = log ? enum_log_kernel<7> : enum_kernel<7>; break;
       }
-      const int64_t work = level == 1 ? (int64_t)n_in * 32 : (int64_t)n_in;
-      // enum_kernel: at most eight chunks a warp slot, so that a warp's buffer fills
-      const int64_t blocks = log ? nblk(work) : std::min<int64_t>(nblk(work), 148 * 32);
-      kern<<<OLPT_G((int)blocks), 256, 0, s>>>(v, in_buf->p, n_in, W.pairs.as<Pair>(), cnt + 4,
-                                               pair_cap);
-      ctx->prof.end(PROF_STEREO, pid, s, 0.0);
-      OLPT_CUDA(cudaGetLastError());
-      n_pairs = read_count(4);
-      if (n_pairs > pair_cap) {  // grow and redo
-        pair_cap = n_pairs + n_pairs / 4 + 1024;
-        continue;
-      }
-      break;
-    }
-    // quick triangulation gate and the children
-    out_cap = (int)std::max<int64_t>(
-        out_cap, std::min<int64_t>(INT32_MAX, (int64_t)(out_buf->bytes / rec(level + 1)) - 1));
-    term_cap = (int)std::max<int64_t>(term_cap, (int64_t)(W.term.bytes / sizeof(Path)) - 1);
-    for (;;) {
-      if (level + 1 < v.m) out_buf->ensure((size_t)out_cap * rec(level + 1), s);
-      W.term.ensure((size_t)term_cap * sizeof(Path), s);
-      // counters: [1] = children, [2] = terminals (terminals accumulate across levels)
-      OLPT_CUDA(cudaMemsetAsync(cnt + 1, 0, sizeof(int), s));
-      OLPT_CUDA(cudaMemcpyAsync(cnt + 2, &n_term, sizeof(int), cudaMemcpyHostToDevice, s));
+      // so many blocks that a warp slot gets several chunks of the larger levels, which vary
+      const int64_t work =
+          level == 1 ? 32 * (int64_t)in_cap : look ? h[2 * level - 2] : in_cap;
       const int pid = ctx->prof.begin(PROF_STEREO, s);
-      auto kern = tri_kernel<1>;
-      switch (level) {
-        case 1: kern = tri_kernel<1>; break;
-        case 2: kern = tri_kernel<2>; break;
-        case 3: kern = tri_kernel<3>; break;
-        case 4: kern = tri_kernel<4>; break;
-        case 5: kern = tri_kernel<5>; break;
-        case 6: kern = tri_kernel<6>; break;
-        default: kern = tri_kernel<7>; break;
-      }
-      if (n_pairs > 0)
-        kern<<<OLPT_G(nblk(n_pairs)), 256, 0, s>>>(v, in_buf->p, W.pairs.as<Pair>(), n_pairs,
-                                                   out_buf->p, cnt + 1, out_cap,
-                                                   W.term.as<Path>(), cnt + 2, term_cap);
+      kern<<<OLPT_G((int)std::min<int64_t>(nblk(work), 148 * 32)), 256, 0, s>>>(
+          v, in_buf->p, cnt + 2 * level - 2, in_cap, W.pairs.as<Pair>(), cnt + 2 * level - 1,
+          pair_cap);
       ctx->prof.end(PROF_STEREO, pid, s, 0.0);
       OLPT_CUDA(cudaGetLastError());
-      int h[2];
-      ReadBack rb(ctx);
-      rb.add(h, cnt + 1, sizeof(h));
-      rb.finish();
-      if (h[0] > out_cap || h[1] > term_cap) {  // grow and redo this level
-        out_cap = std::max(out_cap, h[0] + h[0] / 4 + 1024);
-        term_cap = std::max(term_cap, h[1] + h[1] / 4 + 1024);
+    }
+    if (look) read_counts();
+    // the triangulation gate and the children
+    DevBuf* dst = level == last ? &W.term : out_buf;
+    const int64_t guess =
+        level == last ? std::max<int64_t>(4 * n_ref, 4096)
+        : !look || level == 1 ? path_guess
+                              : std::max<int64_t>(4 * (int64_t)h[2 * level - 2], 4096);
+    out_cap = (int)std::min<int64_t>(
+        INT32_MAX, std::max<int64_t>({(int64_t)out_cap, guess,
+                                      (int64_t)(dst->bytes / rec(level + 1)) - 1}));
+    dst->ensure((size_t)out_cap * rec(level + 1), s);
+    auto kern = tri_kernel<1>;
+    switch (level) {
+      case 1: break;
+      case 2: kern = tri_kernel<2>; break;
+      case 3: kern = tri_kernel<3>; break;
+      case 4: kern = tri_kernel<4>; break;
+      case 5: kern = tri_kernel<5>; break;
+      case 6: kern = tri_kernel<6>; break;
+      default: kern = tri_kernel<7>; break;
+    }
+    const int pid = ctx->prof.begin(PROF_STEREO, s);
+    // a block per 256 pairs; those past the count leave at once
+    const int tiles = nblk(look ? std::min(h[2 * level - 1], pair_cap) : pair_cap);
+    kern<<<OLPT_G(std::max(tiles, 1)), 256, 0, s>>>(
+        v, in_buf->p, W.pairs.as<Pair>(), cnt + 2 * level - 1, pair_cap, dst->p, cnt + 2 * level,
+        out_cap);
+    ctx->prof.end(PROF_STEREO, pid, s, 0.0);
+    OLPT_CUDA(cudaGetLastError());
+    caps_pair[level] = pair_cap;
+    caps_out[level] = out_cap;
+    const bool done = level == last;
+    if (done) {
+      cap_c = out_cap;
+      if (!look) check();
+    }
+    if (done || look) {
+      read_counts();
+      // the first level whose pairs or children did not fit: the levels after it did nothing
+      int bad = look ? level : 1;
+      while (bad <= level && h[2 * bad - 1] <= caps_pair[bad] && h[2 * bad] <= caps_out[bad]) ++bad;
+      if (bad <= level) {
+        look = true;  // from here on the buffers follow the counts
+        if ((level - bad) & 1) std::swap(in_buf, out_buf);
+        level = bad;
+        in_cap = bad == 1 ? cap_a : caps_out[bad - 1];
+        enumerate = h[2 * bad - 1] > caps_pair[bad];
+        const int from = enumerate ? 2 * bad - 1 : 2 * bad;
+        const int cap = (int)std::min<int64_t>(INT32_MAX, h[from] + (int64_t)h[from] / 4 + 1024);
+        if (enumerate) pair_cap = cap;
+        out_cap = enumerate ? 0 : cap;
+        OLPT_CUDA(cudaMemsetAsync(cnt + from, 0, (16 - from) * sizeof(int), s));
         continue;
       }
-      n_in = h[0];
-      n_term = h[1];
+      if (!done && h[2 * level] == 0) break;  // no children; the counts after it are 0
+    }
+    if (done) {
+      if (look) {
+        cap_c = std::max(h[2 * last], 1);
+        check();
+        read_counts();
+      }
       break;
     }
+    in_cap = out_cap;
+    out_cap = 0;
+    enumerate = true;
     std::swap(in_buf, out_buf);
-    out_cap = (int)std::max<int64_t>(4 * (int64_t)n_in, 4096);
+    ++level;
   }
-
-  // check + candidate list
-  int cap_c = std::max(n_term, 1);
-  W.cand_ids.ensure((size_t)cap_c * n_cam * sizeof(int), s);
-  W.cand_e.ensure((size_t)cap_c * sizeof(double), s);
-  W.cand_x.ensure((size_t)cap_c * 3 * sizeof(double), s);
-  OLPT_CUDA(cudaMemsetAsync(cnt + 3, 0, sizeof(int), s));
-  if (n_term > 0)
-    check_kernel<<<OLPT_G(nblk(n_term, 128)), 128, 0, s>>>(v, W.term.as<Path>(), n_term, W.cand_ids.as<int>(),
-                                              W.cand_e.as<double>(), W.cand_x.as<double>(), cnt + 3,
-                                              cap_c);
-  OLPT_CUDA(cudaGetLastError());
-  const int M = read_count(3);
+  const int M = h[kCand];
   res.n_cam = n_cam;
   PhaseTimer pt(ctx->prof, PH_PRUNE);
   std::vector<int> counts(n_cam);
