@@ -16,8 +16,8 @@ enum PruneCount : int {
   PC_MIXED,      // some e_check class has members that differ in value
   PC_FLAG,       // a comparator sort must run on the host (a class is not transitive)
   PC_REPLACE,    // the greedy's replacement rule would fire
-  PC_LEFT,       // greedy rounds: candidates left undecided (two words)
-  PC_N = PC_LEFT + 2
+  PC_LEFT,       // greedy rounds: candidates left undecided (three words)
+  PC_N = PC_LEFT + 3
 };
 
 bool sort_candidates_device(PruneWork& W, const int* ids, const double* e, const double* X, int M,

@@ -381,11 +381,14 @@ __global__ void flat_kernel(const int* ids, int M, int n, PruneView pv, int* fl,
   fcnt[j] = (uint8_t)k;
 }
 
-// Per 2D point, one warp: percentile of each candidate of the point's pool.  Pools
-// of up to kPoolMax candidates live in shared memory, larger ones in the global
-// scratch (indexed by their position in the point -> candidate list).
+// Per 2D point, one warp: percentile of each candidate of the point's pool.  Pools of up to 32
+// candidates stay in registers, larger ones of up to kPoolMax in shared memory, the rest in
+// the global scratch (indexed by their position in the point -> candidate list).  Bound by the
+// latency of the gathers, so by the warps in flight: shared memory for pools of 512 in every
+// warp left room for 16 of them an SM (2.5 million points, 850 -> 420 us; 200,000 points with
+// pools of dozens, 175 -> 110 us).
 constexpr int kPctWarps = 4;
-constexpr int kPoolMax = 512;
+constexpr int kPoolMax = 128;
 struct PoolSmem {
   double e[kPoolMax];
   int j[kPoolMax];
@@ -410,6 +413,51 @@ __global__ void __launch_bounds__(kPctWarps * 32) pct_kernel(const int* pstart, 
   if (f >= n_points) return;
   const int b = pstart[f], end = pstart[f + 1];
   const unsigned lt = (1u << lane) - 1u;
+  if (end - b <= 32) {
+    if (end == b) return;
+    const int slot = items[min(b + lane, end - 1)];
+    const int j = slot / n;
+    const double ev = e[j];
+    const bool fin = b + lane < end && isfinite(ev);
+    const unsigned m = __ballot_sync(0xffffffffu, fin);
+    const int np = __popc(m);
+    if (np <= 1) {
+      if (fin) {
+        slot_pct[slot] = 0.0;
+        slot_used[slot] = 1;
+      }
+      return;
+    }
+    // exact order by (e, j)
+    int r = 0;
+    for (unsigned k = m; k; k &= k - 1) {
+      const double ek = __shfl_sync(0xffffffffu, ev, __ffs(k) - 1);
+      const int jk = __shfl_sync(0xffffffffu, j, __ffs(k) - 1);
+      r += ek < ev || (ek == ev && jk < j) ? 1 : 0;
+    }
+    if (fin) {
+      S.e[r] = ev;
+      S.slot[r] = slot;
+    }
+    __syncwarp();
+    // tolerance classes over the sorted values: lane p is the p-th
+    const bool valid = lane < np;
+    const double mine = S.e[valid ? lane : 0];
+    const unsigned starts = __ballot_sync(
+        0xffffffffu, valid && (lane == 0 || !eq_eps(S.e[valid && lane ? lane - 1 : 0], mine)));
+    const int s0 = 31 - __clz(starts & (lt | (1u << lane)));
+    const unsigned above = starts & ~(lt | (1u << lane));
+    const int s1 = above ? __ffs(above) - 2 : np - 1;
+    bool bad = false;
+    if (valid) {
+      bad = !eq_eps(S.e[s0], mine);
+      const double avg_rank = 0.5 * (double)(s0 + s1);
+      slot_pct[S.slot[lane]] = avg_rank / (double)(np - 1);
+      slot_used[S.slot[lane]] = 1;
+    }
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(flag, 2);
+    return;
+  }
   int np = 0;
   for (int base = b; base < end; base += 32) {
     const int q = base + lane;
@@ -665,11 +713,13 @@ __global__ void gather_greedy_kernel(const int* order, const int* counts, int n,
 // candidate on every one of its points.  Then every rejected candidate evaluates the
 // replacement rule against its owners (the taken candidates before it on its points)
 // exactly as the sequential loop would; if any would replace, the caller runs the
-// sequential loop instead.  One cooperative launch: a round is one pass of atomic minima
-// over the undecided candidates' points and one of decisions (rounds used to be two launches
-// each over sorted point lists, with a look from the host every four).  first[f] holds the
-// round's complement above the candidate, so that a later round's minima replace an earlier
-// one's without clearing.
+// sequential loop instead.  One cooperative launch with one grid barrier a round: a thread
+// decides its candidates from the round's minima over their points, and enters those that stay
+// undecided into the next round's at once.  The rounds' minima alternate between two arrays,
+// and hold the round's complement above the candidate, so that a later round's replace an
+// earlier one's without clearing.  (A candidate whose owner was taken in the same round enters
+// the next one's minima; it would also with a barrier in between.)  Bound by the barriers and
+// the rounds' dependent reads: 240 -> 195 us at 200,000 points with two barriers -> one.
 constexpr uint8_t kUndecided = 0, kTaken = 1, kRejected = 2, kSkipped = 3;
 constexpr int kGreedyThreads = 512;
 
@@ -701,25 +751,30 @@ __device__ bool replaces(const int* g_pts, int cnt, int i, int n, const int* own
 
 __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(
     int* counts, const int* g_pts, const uint8_t* g_cnt, int n, uint8_t* state,
-    unsigned long long* first, int* owner, const int* order, const double* g_pct,
+    unsigned long long* first, int n_points, int* owner, const int* order, const double* g_pct,
     const double* g_e, uint8_t* sel, int* scnt) {
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
   const int G = counts[PC_BOTH];
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  auto enter = [&](int i, unsigned round) {
+    const unsigned long long mark = (unsigned long long)(0xffffffffu - round) << 32 | (unsigned)i;
+    unsigned long long* f = first + (round & 1u) * (size_t)n_points;
+    for (int k = 0; k < g_cnt[i]; ++k) atomicMin(&f[g_pts[(int64_t)i * n + k]], mark);
+  };
   // candidates without a point are passed over by the loop (neither kept nor owners)
-  for (int i = t0; i < G; i += step) state[i] = g_cnt[i] == 0 ? kSkipped : kUndecided;
+  for (int i = t0; i < G; i += step) {
+    state[i] = g_cnt[i] == 0 ? kSkipped : kUndecided;
+    enter(i, 0);
+  }
+  grid.sync();
   // every round decides at least the earliest undecided candidate
   for (unsigned round = 0; round <= (unsigned)G; ++round) {
-    int* left = counts + PC_LEFT + (round & 1u);
-    if (t0 == 0) *left = 0;
+    // three flags: the next round's is cleared while nobody reads or sets it
+    int* left = counts + PC_LEFT + round % 3;
+    if (t0 == 0) counts[PC_LEFT + (round + 1) % 3] = 0;
     const unsigned long long hi = (unsigned long long)(0xffffffffu - round) << 32;
-    for (int i = t0; i < G; i += step) {
-      if (state[i] != kUndecided) continue;
-      for (int k = 0; k < g_cnt[i]; ++k)
-        atomicMin(&first[g_pts[(int64_t)i * n + k]], hi | (unsigned)i);
-    }
-    grid.sync();
+    const unsigned long long* now = first + (round & 1u) * (size_t)n_points;
     bool und = false;
     for (int i = t0; i < G; i += step) {
       if (state[i] != kUndecided) continue;
@@ -727,7 +782,7 @@ __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(
       for (int k = 0; k < g_cnt[i]; ++k) {
         const int f = g_pts[(int64_t)i * n + k];
         blocked = blocked || __ldcg(owner + f) >= 0;
-        all_first = all_first && __ldcg(first + f) == (hi | (unsigned)i);
+        all_first = all_first && __ldcg(now + f) == (hi | (unsigned)i);
       }
       if (blocked) {
         state[i] = kRejected;
@@ -735,6 +790,7 @@ __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(
         state[i] = kTaken;
         for (int k = 0; k < g_cnt[i]; ++k) __stcg(owner + g_pts[(int64_t)i * n + k], i);
       } else {
+        enter(i, round + 1);
         und = true;
       }
     }
@@ -949,9 +1005,9 @@ void prune_device(PruneWork& W, const PruneView& pv, int M, int n, int64_t total
         W.g_e.as<double>());
     OLPT_CUDA(cudaGetLastError());
     W.gstate.ensure(M + 16, s);
-    W.gfirst.ensure(pts * sizeof(unsigned long long), s);
+    W.gfirst.ensure(2 * pts * sizeof(unsigned long long), s);
     W.gowner.ensure(pts * sizeof(int), s);
-    OLPT_CUDA(cudaMemsetAsync(W.gfirst.p, 0xff, pts * sizeof(unsigned long long), s));
+    OLPT_CUDA(cudaMemsetAsync(W.gfirst.p, 0xff, 2 * pts * sizeof(unsigned long long), s));
     OLPT_CUDA(cudaMemsetAsync(W.gowner.p, 0xff, pts * sizeof(int), s));
     const int* a_pts = W.g_pts.as<int>();
     const uint8_t* a_cnt = W.g_cnt.as<uint8_t>();
@@ -962,7 +1018,8 @@ void prune_device(PruneWork& W, const PruneView& pv, int M, int n, int64_t total
     const double *a_pct = W.g_pct.as<double>(), *a_e = W.g_e.as<double>();
     uint8_t* a_sel = W.sel.as<uint8_t>();
     int* a_scnt = W.scnt.as<int>();
-    void* args[] = {&counts, &a_pts, &a_cnt, &n, &a_state, &a_first, &a_owner, &a_order,
+    int n_first = (int)pts;
+    void* args[] = {&counts, &a_pts, &a_cnt, &n, &a_state, &a_first, &n_first, &a_owner, &a_order,
                     &a_pct, &a_e, &a_sel, &a_scnt};
     // at most one block an SM: they have to be resident together
     int dev = 0, sms = 1;

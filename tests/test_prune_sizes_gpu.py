@@ -34,3 +34,24 @@ def test_selection_at_the_sorts_limits(M):
         ctx.close()
     assert np.array_equal(got, _prune(ids, e, counts, [1] * n_cam))
     assert np.array_equal(got, again)
+
+
+@pytest.mark.parametrize("drop", [0.0, 0.1])
+def test_selection_at_the_pools_limits(drop):
+    """Pools of a point in registers (32), in shared memory (128) and in global memory, with
+    checks that tie within the tolerance and some that are not finite."""
+    rng = np.random.default_rng(int(10 * drop))
+    sizes = [1, 2, 31, 32, 33, 34, 64, 127, 128, 129, 130, 513, 1500]
+    first = np.repeat(np.arange(len(sizes)), sizes)
+    M = len(first)
+    ids = np.c_[first, rng.integers(0, M // 3, M), rng.permutation(M)].astype(np.int32)
+    ids = ids[np.lexsort(ids.T[::-1])]
+    e = rng.integers(1, 400, M) * 1e-4 * (1.0 + rng.integers(-1, 2, M) * 2e-10)
+    e[rng.random(M) < drop] = np.nan
+    counts = [len(sizes), M, M]
+    ctx = _ffi.Context(0)
+    try:
+        got = ctx.prune_matches(ids, e, counts)
+    finally:
+        ctx.close()
+    assert np.array_equal(got, _prune(ids, e, counts, [1] * 3))
