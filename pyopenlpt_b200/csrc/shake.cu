@@ -60,10 +60,11 @@ template <typename Real>
 __global__ void __launch_bounds__(256) splat_kernel(const __grid_constant__ ShakeView v,
                                                     const double* xyz, int64_t n, double* uv,
                                                     Real* otfp, const uint8_t* flags,
-                                                    int all_cams) {
+                                                    int all_cams, int per_warp) {
   constexpr unsigned kFull = 0xffffffffu;
-  const int64_t pair = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
+  const int64_t warp = blockIdx.x * (int64_t)(blockDim.x / 32) + threadIdx.x / 32;
+  const int64_t pair = lane < per_warp ? warp * per_warp + lane : n * v.n_cam;
   double u = 0.0, w = 0.0;
   Real o[5] = {0, 0, 0, 0, 0};
   Rect r{1, 0, 1, 0};
@@ -1335,10 +1336,15 @@ static void residual_pass(olpt_ctx* ctx, ShakeView& v, const uint8_t* flags, int
   W.otfp.ensure((n * C + 1) * 5 * sizeof(Real), s);
   ensure_projection_planes(ctx, v, sizeof(Real) == 8);
   W.proj_clean = false;
+  // 32 pairs a warp where that gives the SMs 16 warps each, else so few (down to 2) that it does:
+  // a warp takes its windows one after the other (up to 9,000 objects on four cameras: 21 -> 12
+  // us a launch; above 75,000 pairs the rule gives 32 and nothing changes)
+  int per_warp = 32;
+  while (per_warp > 2 && n * C < (int64_t)per_warp * 148 * 16) per_warp /= 2;
   if (n > 0)
-    splat_kernel<Real><<<OLPT_G(nblk(n * C)), 256, 0, s>>>(v, ctx->obj.xyz.as<double>(), n,
-                                                          ctx->obj.uv.as<double>(),
-                                                          W.otfp.as<Real>(), flags, all_cams);
+    splat_kernel<Real><<<OLPT_G(nblk(n * C, 8 * per_warp)), 256, 0, s>>>(
+        v, ctx->obj.xyz.as<double>(), n, ctx->obj.uv.as<double>(), W.otfp.as<Real>(), flags,
+        all_cams, per_warp);
   OLPT_CUDA(cudaGetLastError());
   // algorithmic bytes: read the image, write the residual, for every computed camera
   double bytes = 0;
