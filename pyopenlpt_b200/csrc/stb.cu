@@ -15,7 +15,7 @@
 //    the view-volume test and the camera-visibility test;
 //  * the predictions go through the device shake and residual (shake.cu), the
 //    residual through the device IPR (ipr.cu);
-//  * repeat_kernel / link_kernel / nn_kernel: radius and nearest-neighbour queries
+//  * repeat_kernel / link_kernel (a warp a track) / nn_kernel: radius and nearest-neighbour queries
 //    over CSR hash grids (cell >= the query radius, 27 cells) that stand in for
 //    nanoflann; nearest-neighbour ties go to the lowest index;
 //  * linfit_kernel: one thread per track;
@@ -217,24 +217,109 @@ __global__ void repeat_kernel(const double* obj, int n, HashGrid g, double tol, 
 }
 
 // ---------------------------------------------------------------- linking
-// STB::linkShortTrack (STB.cpp:743-872) for every active short track.  tg: grid
+// The points in the distinct buckets of the 27 cells around q, as one list that the lanes of a
+// warp share: lane e < 27 finds its cell's bucket (one lane keeps a bucket that several cells
+// share), and a prefix sum over the buckets' sizes places them.
+struct WarpList {
+  int start[27], before[28];  // first item of every bucket, list positions before it
+};
+
+__device__ __forceinline__ int warp_list(const HashGrid& g, const double q[3], WarpList& L) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int n = 0, st = 0;
+  if (g.pts) {
+    const long long cx = (long long)floor(q[0] / g.cell), cy = (long long)floor(q[1] / g.cell),
+                    cz = (long long)floor(q[2] / g.cell);
+    const int b = lane < 27 ? hash_bucket(cx + lane % 3 - 1, cy + lane / 3 % 3 - 1,
+                                          cz + lane / 9 - 1, g.n_buckets)
+                            : -1;
+    const unsigned same = __match_any_sync(kFull, b);
+    if (b >= 0 && lane == __ffs(same) - 1) {
+      st = g.start[b];
+      n = g.start[b + 1] - st;
+    }
+  }
+  int incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += y;
+  }
+  __syncwarp();  // the list before is no longer read
+  if (lane < 27) {
+    L.start[lane] = st;
+    L.before[lane + 1] = incl;
+    if (lane == 0) L.before[0] = 0;
+  }
+  __syncwarp();
+  return __shfl_sync(kFull, incl, 31);
+}
+
+// Item at list position t; e is the position's bucket, or one before it.
+__device__ __forceinline__ int list_item(const HashGrid& g, const WarpList& L, int t, int& e) {
+  while (t >= L.before[e + 1]) ++e;
+  return g.items[L.start[e] + t - L.before[e]];
+}
+
+__device__ __forceinline__ double warp_sum(double x) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+// grid_nearest by a warp.
+__device__ int warp_nearest(const HashGrid& g, const double q[3], double r2, WarpList& L) {
+  const int total = warp_list(g, q, L);
+  int best = -1;
+  double bd = 0.0;
+  for (int t = threadIdx.x & 31, e = 0; t < total; t += 32) {
+    const int j = list_item(g, L, t, e);
+    const double d2 = l2sq(q, g.pts + 3 * (int64_t)j);
+    if (best < 0 || d2 < bd || (d2 == bd && j < best)) {
+      best = j;
+      bd = d2;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const int j = __shfl_xor_sync(0xffffffffu, best, o);
+    const double d2 = __shfl_xor_sync(0xffffffffu, bd, o);
+    if (j >= 0 && (best < 0 || d2 < bd || (d2 == bd && j < best))) {
+      best = j;
+      bd = d2;
+    }
+  }
+  best = __shfl_sync(0xffffffffu, best, 0);
+  bd = __shfl_sync(0xffffffffu, bd, 0);
+  return (best >= 0 && bd < r2) ? best : -1;
+}
+
+// STB::linkShortTrack (STB.cpp:743-872) for every active short track, a warp each.  tg: grid
 // over the long tracks' second-to-last points rounded to float (TrackCloud,
 // inc/libSTB/Track.h:49-62), disp: their last displacement; go: grid over the new
-// objects.  len: points in the short track (an empty track is UNLINKED).
-__global__ void link_kernel(const double* p_last, const int* len, int n_sa, HashGrid tg,
-                            const double* disp, HashGrid go, double base_r, int* link) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// objects.  len: points in the short track (an empty track is UNLINKED).  Bound by the neighbour
+// tracks' FP64 weights (five divisions each); a thread a track read one neighbour a lane at a
+// time from 32 places (51,000 particles: 4.3 -> 3.4 ms for the two launches of a sequence).
+constexpr int kLinkWarps = 4;
+
+__global__ void __launch_bounds__(kLinkWarps * 32) link_kernel(const double* p_last, const int* len,
+                                                               int n_sa, HashGrid tg,
+                                                               const double* disp, HashGrid go,
+                                                               double base_r, int* link) {
+  __shared__ WarpList lists[kLinkWarps];
+  WarpList& L = lists[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int i = blockIdx.x * kLinkWarps + (threadIdx.x >> 5);
   if (i >= n_sa) return;
   if (len[i] == 0 || !(base_r > 0.0)) {
-    link[i] = -1;
+    if (lane == 0) link[i] = -1;
     return;
   }
-  const double* p = p_last + 3 * (int64_t)i;
-  int bk[27];
-  const int nb = cell_buckets(tg, p, bk);
+  const double p[3] = {p_last[3 * (int64_t)i], p_last[3 * (int64_t)i + 1],
+                       p_last[3 * (int64_t)i + 2]};
   // the radius of every step (factor 1, 1.1, 1.1 * 1.1, ...); the neighbour sums of all
-  // steps are accumulated in one scan each (same neighbour order as one scan per step,
-  // so the same sums)
+  // steps are accumulated in one scan each
   double fac[kLinkIters], r2[kLinkIters];
 #pragma unroll
   for (int st = 0; st < kLinkIters; ++st) {
@@ -249,20 +334,22 @@ __global__ void link_kernel(const double* p_last, const int* len, int n_sa, Hash
     cnt[st] = 0;
     mean_d2[st] = 0.0;
   }
-  for (int e = 0; e < nb; ++e)
-    for (int s = tg.start[bk[e]]; s < tg.start[bk[e] + 1]; ++s) {
-      const double d2 = l2sq(p, tg.pts + 3 * (int64_t)tg.items[s]);
+  const int total = warp_list(tg, p, L);
+  for (int t = lane, e = 0; t < total; t += 32) {
+    const double d2 = l2sq(p, tg.pts + 3 * (int64_t)list_item(tg, L, t, e));
 #pragma unroll
-      for (int st = 0; st < kLinkIters; ++st)
-        if (d2 < r2[st]) {
-          ++cnt[st];
-          mean_d2[st] += d2;
-        }
-    }
+    for (int st = 0; st < kLinkIters; ++st)
+      if (d2 < r2[st]) {
+        ++cnt[st];
+        mean_d2[st] += d2;
+      }
+  }
   double beta2[kLinkIters];
   bool any = false;
 #pragma unroll
   for (int st = 0; st < kLinkIters; ++st) {
+    cnt[st] = __reduce_add_sync(0xffffffffu, cnt[st]);
+    mean_d2[st] = warp_sum(mean_d2[st]);
     beta2[st] = 0.0;
     if (cnt[st] > 0) {
       any = true;
@@ -279,24 +366,31 @@ __global__ void link_kernel(const double* p_last, const int* len, int n_sa, Hash
   double sum_w[kLinkIters], sx[kLinkIters], sy[kLinkIters], sz[kLinkIters];
 #pragma unroll
   for (int st = 0; st < kLinkIters; ++st) sum_w[st] = sx[st] = sy[st] = sz[st] = 0.0;
-  if (any)
-    for (int e = 0; e < nb; ++e)
-      for (int s = tg.start[bk[e]]; s < tg.start[bk[e] + 1]; ++s) {
-        const int j = tg.items[s];
-        const double d2 = l2sq(p, tg.pts + 3 * (int64_t)j);
-        if (!(d2 < r2[kLinkIters - 1])) continue;
-        const double dx = disp[3 * (int64_t)j], dy = disp[3 * (int64_t)j + 1],
-                     dz = disp[3 * (int64_t)j + 2];
+  if (any) {
+    for (int t = lane, e = 0; t < total; t += 32) {
+      const int j = list_item(tg, L, t, e);
+      const double d2 = l2sq(p, tg.pts + 3 * (int64_t)j);
+      if (!(d2 < r2[kLinkIters - 1])) continue;
+      const double dx = disp[3 * (int64_t)j], dy = disp[3 * (int64_t)j + 1],
+                   dz = disp[3 * (int64_t)j + 2];
 #pragma unroll
-        for (int st = 0; st < kLinkIters; ++st) {
-          if (cnt[st] == 0 || !(d2 < r2[st])) continue;
-          const double w = 1.0 / (1.0 + d2 * beta2[st]);
-          sum_w[st] += w;
-          sx[st] += w * dx;
-          sy[st] += w * dy;
-          sz[st] += w * dz;
-        }
+      for (int st = 0; st < kLinkIters; ++st) {
+        if (cnt[st] == 0 || !(d2 < r2[st])) continue;
+        const double w = 1.0 / (1.0 + d2 * beta2[st]);
+        sum_w[st] += w;
+        sx[st] += w * dx;
+        sy[st] += w * dy;
+        sz[st] += w * dz;
       }
+    }
+#pragma unroll
+    for (int st = 0; st < kLinkIters; ++st) {
+      sum_w[st] = warp_sum(sum_w[st]);
+      sx[st] = warp_sum(sx[st]);
+      sy[st] = warp_sum(sy[st]);
+      sz[st] = warp_sum(sz[st]);
+    }
+  }
   int obj_id = -1;
 #pragma unroll
   for (int st = 0; st < kLinkIters; ++st) {
@@ -309,14 +403,14 @@ __global__ void link_kernel(const double* p_last, const int* len, int n_sa, Hash
     }
     const double est[3] = {p[0] + vel[0], p[1] + vel[1], p[2] + vel[2]};
     const double r_obj = base_r * fac[st];
-    obj_id = grid_nearest(go, est, r_obj * r_obj);
+    obj_id = warp_nearest(go, est, r_obj * r_obj, L);
     if (obj_id >= 0) break;
     if (cnt[st] == 0) {
-      obj_id = grid_nearest(go, p, r_obj * r_obj);
+      obj_id = warp_nearest(go, p, r_obj * r_obj, L);
       if (obj_id >= 0) break;
     }
   }
-  link[i] = obj_id;
+  if (lane == 0) link[i] = obj_id;
 }
 
 // Nearest object within the radius for every query point (initial phase).
@@ -362,7 +456,9 @@ constexpr int kPfMaxNb = 4096;  // objects of one frame inside one search cube
 
 // PredField::calPredField (PredField.cpp:20-90), one grid node per CTA:
 // findNeighbor (|d| < r on every axis, :205-231), updateDispPDF (:247-283),
-// findPDFPeakID / findPDFPeakLoc / fitPeakBinLocGauss (:286-369).
+// findPDFPeakID / findPDFPeakLoc / fitPeakBinLocGauss (:286-369).  Bound by the pairs' atomics
+// on the bins in shared memory; with an exponential per bin and one thread looking for the
+// maximum 5.6 ms for three launches at 51,000 particles, now 4.2.
 __global__ void __launch_bounds__(256) pf_node_kernel(PfView pf, HashGrid gp, HashGrid gc,
                                                       double* field, int* overflow) {
   extern __shared__ __align__(16) unsigned char pf_smem[];
@@ -370,8 +466,8 @@ __global__ void __launch_bounds__(256) pf_node_kernel(PfView pf, HashGrid gp, Ha
   int* lp = reinterpret_cast<int*>(pdf + pf.nbin_tot);
   int* lc = lp + kPfMaxNb;
   __shared__ int n_nb[2];
-  __shared__ int s_peak;
-  __shared__ double s_peakv;
+  __shared__ int s_peak, s_maxi[8];
+  __shared__ double s_peakv, s_maxv[8];
   const int g = blockIdx.x;
   const int zi = g % pf.nz, yi = (g / pf.nz) % pf.ny, xi = g / (pf.ny * pf.nz);
   // myMATH::linspace nodes (myMATH.cpp:9-33)
@@ -416,25 +512,62 @@ __global__ void __launch_bounds__(256) pf_node_kernel(PfView pf, HashGrid gp, Ha
     const double yb = pf.m[1] * (a[1] - b[1]) + pf.c[1];
     const double zb = pf.m[2] * (a[2] - b[2]) + pf.c[2];
     const int xi0 = (int)round(xb), yi0 = (int)round(yb), zi0 = (int)round(zb);
-    for (int i = max(0, xi0 - 1); i <= min(pf.nbin[0] - 1, xi0 + 1); ++i) {
-      const double xx = i - xb;
-      for (int j = max(0, yi0 - 1); j <= min(pf.nbin[1] - 1, yi0 + 1); ++j) {
-        const double yy = j - yb;
-        for (int k = max(0, zi0 - 1); k <= min(pf.nbin[2] - 1, zi0 + 1); ++k) {
-          const double zz = k - zb;
-          atomicAdd(&pdf[i * nyz + j * pf.nbin[2] + k], exp(-(xx * xx + yy * yy + zz * zz)));
-        }
+    // exp(-(x^2 + y^2 + z^2)) as a product: nine exponentials for the 27 bins
+    double ex[3], ey[3], ez[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double xx = xi0 - 1 + k - xb, yy = yi0 - 1 + k - yb, zz = zi0 - 1 + k - zb;
+      ex[k] = exp(-(xx * xx));
+      ey[k] = exp(-(yy * yy));
+      ez[k] = exp(-(zz * zz));
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      if (xi0 - 1 + i < 0 || xi0 - 1 + i >= pf.nbin[0]) continue;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        if (yi0 - 1 + j < 0 || yi0 - 1 + j >= pf.nbin[1]) continue;
+        const double exy = ex[i] * ey[j];
+        double* row = pdf + (xi0 - 1 + i) * nyz + (yi0 - 1 + j) * pf.nbin[2] + zi0 - 1;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (zi0 - 1 + k >= 0 && zi0 - 1 + k < pf.nbin[2]) atomicAdd(row + k, exy * ez[k]);
       }
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {  // std::max_element: the first maximum
-    int bi = 0;
-    double bv = pdf[0];
-    for (int b = 1; b < pf.nbin_tot; ++b)
-      if (bv < pdf[b]) {
-        bv = pdf[b];
-        bi = b;
+  // std::max_element: the first maximum (a first bin that is not a number stays)
+  int bi = threadIdx.x;
+  double bv = bi < pf.nbin_tot ? pdf[bi] : -1.0;  // below every bin
+  for (int b = threadIdx.x + blockDim.x; b < pf.nbin_tot; b += blockDim.x)
+    if (bv < pdf[b] || (bv != bv && bi)) {
+      bv = pdf[b];
+      bi = b;
+    }
+  auto better = [](double v, int b, double w, int c) {  // (w, c) goes before (v, b)
+    if (b == 0 && v != v) return false;
+    if (c == 0 && w != w) return true;
+    return v < w || (v == w && c < b) || (v != v && w == w);
+  };
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const double w = __shfl_xor_sync(0xffffffffu, bv, o);
+    const int c = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (better(bv, bi, w, c)) {
+      bv = w;
+      bi = c;
+    }
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_maxv[threadIdx.x >> 5] = bv;
+    s_maxi[threadIdx.x >> 5] = bi;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)blockDim.x / 32; ++w)
+      if (better(bv, bi, s_maxv[w], s_maxi[w])) {
+        bv = s_maxv[w];
+        bi = s_maxi[w];
       }
     s_peak = bi;
     s_peakv = bv;
@@ -1171,7 +1304,7 @@ void conv_phase(olpt_ctx* ctx, int frame) {
       HashGrid tg = build_grid(W.g1, W.k1, d_key, n_la, 3.0 * r_max, s);
       HashGrid go = build_grid(W.g2, W.k2, d_obj, n_obj, r_max, s);
       W.link.ensure((n_sa + 1) * sizeof(int), s);
-      link_kernel<<<OLPT_G(nblk(n_sa, 128)), 128, 0, s>>>(d_pl, d_len, n_sa, tg, d_disp, go, base_r,
+      link_kernel<<<OLPT_G(nblk(n_sa, kLinkWarps)), kLinkWarps * 32, 0, s>>>(d_pl, d_len, n_sa, tg, d_disp, go, base_r,
                                                          W.link.as<int>());
       OLPT_CUDA(cudaGetLastError());
       link = download(ctx, W.link.as<int>(), n_sa);
