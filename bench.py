@@ -366,7 +366,7 @@ def workload_config(name, s, sc=None, seq=None, st=None):
 
 # ----------------------------------------------------------------------------- our arm
 PROF_NAMES = {0: "peak detection", 1: "stereo level expansion", 2: "residual image",
-              3: "shake (warp per particle)", 4: "predictive field"}
+              3: "shake", 4: "predictive field"}
 PHASE_NAMES = {5: "detection", 6: "stereo matching (all)", 7: "candidate sort + prune + greedy",
                8: "shake (all)", 9: "output + residual", 10: "STB track work",
                11: "sequential greedy (replacement fallback)", 12: "track work: prediction",
@@ -378,9 +378,9 @@ PHASE_NAMES = {5: "detection", 6: "stereo matching (all)", 7: "candidate sort + 
 # algorithmic bytes per object in FP32 (C x 64 ROI pixels x 4 B + 2 x (24 + C x 16 + 8) B
 # of state + C x 5 x 4 B of OTF).  4 cameras: dram__bytes_read.sum + dram__bytes_write.sum
 # of three shake_kernel launches of the 1280x800 STB convergence frames (16-19 k objects
-# each) over their objects.  6 cameras: two launches of the first IPR of a 2048^2 headline
-# frame (14,840 objects each), dram__bytes.sum.per_second x duration over the objects.
-SHAKE_TRAFFIC = {4: (7_300.0, 1_296.0), 6: (22_440.0, 1_912.0)}
+# each) over their objects, with an earlier form of the kernel (a warp an object).  6
+# cameras: four launches on 120,000 objects over 2048^2 images, 156-235 MB each.
+SHAKE_TRAFFIC = {4: (7_300.0, 1_296.0), 6: (1_700.0, 1_912.0)}
 
 
 def shake_traffic(args, prec, dom, bytes_per_launch, cams):

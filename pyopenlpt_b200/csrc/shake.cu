@@ -55,7 +55,7 @@ __device__ __forceinline__ void raise_to(double* p, double v) {
 // (a window's row is one 16-byte run of one sector for the atomics).  Replaces a pass over the
 // objects, the counting sort of the pairs by 32x32 image tile (five launches) and a kernel in
 // which four tiles each recomputed a pair's window and Gaussian per pixel: 120,000 objects on
-// six 2048^2 cameras, the whole residual took 620 us and takes 150 us.
+// six 2048^2 cameras, the whole residual took 620 us and takes 270 us (cold caches).
 template <typename Real>
 __global__ void __launch_bounds__(256) splat_kernel(const __grid_constant__ ShakeView v,
                                                     const double* xyz, int64_t n, double* uv,

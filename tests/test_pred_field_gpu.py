@@ -1,6 +1,6 @@
 """The predictive field's nodes against a numpy restatement of PredField::calPredField
-(PredField.cpp:20-90) on the same objects.  The field's file holds nine digits of values up to about 10 mm, and its sums of at most
-1e5 exponentials are equal up to 1e-11: 1e-7 mm."""
+(PredField.cpp:20-90) on the same objects.  The field's file holds nine digits of values up to
+about 10 mm, and its sums of at most 1e5 exponentials are equal up to 1e-11: 1e-7 mm."""
 import os
 
 import numpy as np
