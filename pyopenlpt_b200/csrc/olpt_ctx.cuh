@@ -195,6 +195,7 @@ struct PruneWork {
   DevBuf gstate, gfirst, gowner, sel, spos, scnt;
   Csr points;
   int n_sel = 0;  // kept candidates of the last device prune
+  int cluster = -1;  // the device runs clusters of 16 sort blocks (-1: not asked yet)
   HostBuf pin;    // pinned staging of the sequential greedy's input
   void release(cudaStream_t s) {
     for (DevBuf* b : {&key, &val, &key2, &val2, &hist, &scan_tmp, &ids_s, &e_s, &X_s, &fl,

@@ -843,7 +843,7 @@ static void radix_sort_device(PruneWork& W, int n, int bits, cudaStream_t s) {
     std::swap(W.val, W.val2);
     return;
   }
-  if (n <= kClSort) {
+  if (n <= kClSort && W.cluster != 0) {
     OLPT_CUDA(cudaFuncSetAttribute(cluster_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kClSmem));
     OLPT_CUDA(cudaFuncSetAttribute(cluster_sort_kernel,
@@ -853,19 +853,29 @@ static void radix_sort_device(PruneWork& W, int n, int bits, cudaStream_t s) {
     at.val.clusterDim.x = kClBlocks;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(OLPT_G(kClBlocks));
+    cfg.gridDim = dim3(kClBlocks);
     cfg.blockDim = dim3(kSmallThreads);
     cfg.dynamicSmemBytes = kClSmem;
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    const int per = ((n + kClBlocks - 1) / kClBlocks + 31) / 32 * 32;
-    OLPT_CUDA(cudaLaunchKernelEx(&cfg, cluster_sort_kernel, (const uint64_t*)W.key.as<uint64_t>(),
-                                 (const int*)W.val.as<int>(), n, bits, per,
-                                 W.key2.as<uint64_t>(), W.val2.as<int>()));
-    std::swap(W.key, W.key2);
-    std::swap(W.val, W.val2);
-    return;
+    if (W.cluster < 0) {  // a partition of the device may have no 16 SMs side by side
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, cluster_sort_kernel, &cfg) != cudaSuccess)
+        cudaGetLastError();
+      W.cluster = clusters > 0;
+    }
+    if (W.cluster) {
+      const int per = ((n + kClBlocks - 1) / kClBlocks + 31) / 32 * 32;
+      cfg.gridDim = dim3(OLPT_G(kClBlocks));
+      OLPT_CUDA(cudaLaunchKernelEx(&cfg, cluster_sort_kernel,
+                                   (const uint64_t*)W.key.as<uint64_t>(),
+                                   (const int*)W.val.as<int>(), n, bits, per,
+                                   W.key2.as<uint64_t>(), W.val2.as<int>()));
+      std::swap(W.key, W.key2);
+      std::swap(W.val, W.val2);
+      return;
+    }
   }
   const int n_blocks = (n + kRsTile - 1) / kRsTile;
   W.hist.ensure((size_t)256 * n_blocks * sizeof(int), s);
