@@ -61,7 +61,8 @@ struct SmView {
   const double* l2d;     // x n_cam x 6: image line on camera t (pt, unit, normalized unit)
   const float4* fl;      // x n_cam: (n, d) of that line, |n . p + d| = distance of p from it
   double tol2d, tol3d;
-  float eps;             // FP32 error bound of a distance, without the part of |d|
+  float eps;             // FP32 error bound of a distance, without the part of |d|, for points
+                         // in the image
   double tq[OLPT_MAX_CAM + 1];  // quick-gate tolerance of k lines without its angle factor
   double limit[6];
   // near-tolerance log (off when near_band == 0): 2D tests whose distance lies within
@@ -777,7 +778,10 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : 3) enum_kernel(
         const float2 p = v.fxy[id];
         const float4 L = v.fl[(int64_t)g * v.n_cam + (int)((cams >> (4 * i)) & 15u)];
         const float z = fabsf(fmaf(L.x, p.x, fmaf(L.y, p.y, L.z)));
-        const float b = v.eps + 5e-7f * fabsf(L.z);
+        float b = v.eps + 5e-7f * fabsf(L.z);
+        // eps covers coordinates inside the image: a path's first point, which comes from the
+        // list and not from the grid, may lie anywhere
+        if (i == 0) b += 5e-7f * (fabsf(p.x) + fabsf(p.y));
         ok = ok && !(z > tol + b);
         edge = edge || !(z < tol - b);
       }
