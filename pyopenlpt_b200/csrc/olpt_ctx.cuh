@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -45,6 +46,23 @@ struct ApiError {
   do {                                \
     if (!(cond)) throw ::olpt::ApiError{(code), (msg)}; \
   } while (0)
+
+// Dynamic shared memory that the current device grants Kernel, raised to at least `bytes`.  The
+// limit belongs to the kernel on the device, not to a context: one that another context's
+// thread lowered between this call and the launch would refuse the launch, so it only rises.
+template <auto Kernel>
+void allow_smem(size_t bytes) {
+  static std::mutex mu;
+  static size_t set[64] = {};
+  int dev = 0;
+  OLPT_CUDA(cudaGetDevice(&dev));
+  OLPT_REQUIRE(dev >= 0 && dev < 64, OLPT_ERR_INVALID_ARG, "device ordinal out of range");
+  std::lock_guard<std::mutex> lk(mu);
+  if (bytes <= set[dev]) return;
+  OLPT_CUDA(cudaFuncSetAttribute((const void*)Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)bytes));
+  set[dev] = bytes;
+}
 
 // Grow-only device buffer (stream-ordered allocation).
 struct DevBuf {

@@ -742,25 +742,9 @@ __global__ void __launch_bounds__(kDetThreads, 3) detect_kernel(const __grid_con
   }
 }
 
-// Dynamic shared memory of detect_kernel<T> on the current device raised to at least
-// `bytes` (the attribute is per device; set once per device and size).
-template <typename T>
-void detect_smem_attr(size_t bytes) {
-  static std::mutex mu;
-  static size_t set[64] = {};
-  int dev = 0;
-  OLPT_CUDA(cudaGetDevice(&dev));
-  OLPT_REQUIRE(dev >= 0 && dev < 64, OLPT_ERR_INVALID_ARG, "device ordinal out of range");
-  std::lock_guard<std::mutex> lk(mu);
-  if (bytes <= 48 * 1024 || bytes <= set[dev]) return;
-  OLPT_CUDA(cudaFuncSetAttribute(detect_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)bytes));
-  set[dev] = bytes;
-}
-
 template <typename T>
 void launch_detect(const DetArgs& a, int n_blocks, size_t smem, cudaStream_t s) {
-  detect_smem_attr<T>(smem);
+  allow_smem<detect_kernel<T>>(smem);
   detect_kernel<T><<<OLPT_G(n_blocks), kDetThreads, smem, s>>>(a);
   OLPT_CUDA(cudaGetLastError());
 }

@@ -1409,8 +1409,7 @@ static void launch_shake(int warps, cudaStream_t s, const ShakeView& v, int64_t 
   const size_t per_warp = v.obj_stride * (32 / LPO);
   while (warps > 1 && v.cam_bytes + per_warp * warps > kShakeSmemMax) warps /= 2;
   const size_t smem = v.cam_bytes + per_warp * warps;
-  OLPT_CUDA(cudaFuncSetAttribute(shake_kernel<Real, NC, LPO, MINB>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem<shake_kernel<Real, NC, LPO, MINB>>(smem);
   shake_kernel<Real, NC, LPO, MINB><<<OLPT_G(nblk(n, warps * (32 / LPO))), 32 * warps, smem, s>>>(
       v, n, xyz, uv, otfp, score, delta, active, resid_out);
 }
