@@ -996,8 +996,7 @@ const double* cal_pred_field(olpt_ctx* ctx, int i) {
   OLPT_CUDA(cudaMemsetAsync(W.flag.p, 0, sizeof(int), s));
   const size_t smem = pf.nbin_tot * sizeof(double) + 2 * kPfMaxNb * sizeof(int);
   OLPT_REQUIRE(smem <= 200 * 1024, OLPT_ERR_UNSUPPORTED, "predictive field: too many PDF bins");
-  OLPT_CUDA(cudaFuncSetAttribute(pf_node_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+  allow_smem<pf_node_kernel>(smem);
   const int pid = ctx->prof.begin(PROF_PF, s);
   pf_node_kernel<<<OLPT_G(n_grid), 256, smem, s>>>(pf, gp, gc, W.field.as<double>(),
                                                    W.flag.as<int>());

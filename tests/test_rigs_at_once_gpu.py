@@ -11,6 +11,7 @@ from pyopenlpt_b200 import _ffi, synth
 pytestmark = pytest.mark.gpu
 
 VOLUME = (-20.0, 20.0, -20.0, 20.0, -10.0, 10.0)
+FRAMES = 64
 
 
 def _at_once(jobs):
@@ -66,6 +67,43 @@ def test_shake_of_a_pinhole_and_a_polynomial_rig(n, precision):
         for g, w in zip(got, want):
             for name in ("xyz", "uv", "score", "flags"):
                 assert np.array_equal(g[name], w[name]), name
+    finally:
+        for c in ctxs:
+            c.close()
+
+
+def test_predictive_fields_of_different_bins():
+    """21 bins an axis take 107 KB of a block's shared memory, 11 bins 43 KB."""
+    seq = synth.make_sequence(n_particles=40, n_frames=1, n_cam=2, n_row=64, n_col=64, focal=300.0,
+                              volume=VOLUME, a=200.0, noise=0.0, bits=8, seed=1)
+    ipr = synth.IPRSettings(n_loop_ipr=1, n_shake_loop=1, match_cam_count=2)
+    stb = synth.STBSettings(pf_nx=2, pf_ny=2, pf_nz=2, n_initial_frames=FRAMES)
+    bins = [21, 11, 21, 11, 11, 11]
+    ctxs = []
+    try:
+        params = []
+        for b in bins:
+            ctx = _ffi.Context(0)
+            ctxs.append(ctx)
+            ctx.upload_cameras([_ffi.camera_desc(c) for c in seq.cams])
+            ctx.upload_otf(2, 2, 2, VOLUME, synth.otf_table_array(2, seq.otf_abc))
+            params.append(_ffi.stb_params(ipr, stb, VOLUME, 0, FRAMES - 1, 0))
+            for k in range(3):
+                params[-1].pf_nbin[k] = b
+
+        def job(ctx, p, times):
+            for _ in range(times):
+                ctx.stb_configure(p)
+                for t in range(FRAMES):  # the last one computes all fields
+                    ctx.upload_images(seq.frames[0])
+                    ctx.stb_process_frame(t)
+            return [ctx.stb_tracks(k) for k in range(4)]
+
+        want = [job(c, p, 1) for c, p in zip(ctxs, params)]
+        got = _at_once([lambda c=c, p=p: job(c, p, 60) for c, p in zip(ctxs, params)])
+        for g, w in zip(got, want):
+            for a, b in zip(g, w):
+                assert all(np.array_equal(x, y) for x, y in zip(a, b))
     finally:
         for c in ctxs:
             c.close()
