@@ -1052,16 +1052,13 @@ __device__ __forceinline__ int next_camera(const SmView& v, const PathN<N>& ch) 
 // calTriangulateTol, TriangulationCheckWithTol: StereoMatch.cpp:1072-1141), then the child path
 // (terminal, or with its next target camera).  Bound by the gathers of the lines of sight.
 template <int K>
-__global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
-    const __grid_constant__ SmView v, const void* in_v, const Pair* pairs, const int* n_ptr,
-    int pair_cap, void* out_v, int* out_count, int out_cap) {
+__device__ __forceinline__ void tri_tile(const SmView& v, const void* in_v, const Pair* pairs,
+                                         int n_pairs, int tile, void* out_v, int* out_count,
+                                         int out_cap) {
   __shared__ int s_cnt[8], s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool last = K + 1 == v.m;
-  const int n_pairs = *n_ptr;
-  if (n_pairs > pair_cap) return;  // pairs are missing: the level is repeated
-  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gi - (int)threadIdx.x >= n_pairs) return;
+  const int64_t gi = tile * (int64_t)blockDim.x + threadIdx.x;
   PathN<K + 1> ch;
   bool ok = gi < n_pairs;
   if (ok) {
@@ -1127,6 +1124,25 @@ __global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
   full.k = K + 1;
   full.target = -1;
   static_cast<Path*>(out_v)[slot] = full;
+}
+
+// LOOP: the blocks share the tiles of 256 pairs; else there is a block for each (the loop is 10%
+// slower at the largest levels).
+template <int K, bool LOOP>
+__global__ void __launch_bounds__(256, K <= 2 ? 4 : K <= 4 ? 3 : 2) tri_kernel(
+    const __grid_constant__ SmView v, const void* in_v, const Pair* pairs, const int* n_ptr,
+    int pair_cap, void* out_v, int* out_count, int out_cap) {
+  const int n_pairs = *n_ptr;
+  if (n_pairs > pair_cap) return;  // pairs are missing: the level is repeated
+  const int tiles = (int)((n_pairs + 255ll) / 256);
+  int tile = blockIdx.x;
+  if (tile >= tiles) return;
+  for (;;) {
+    tri_tile<K>(v, in_v, pairs, n_pairs, tile, out_v, out_count, out_cap);
+    tile += gridDim.x;
+    if (!LOOP || tile >= tiles) return;
+    __syncthreads();  // the tile's counts are no longer read
+  }
 }
 
 // StereoMatch::checkMatch, case "every active camera was used to build"
@@ -1374,12 +1390,19 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
   // A look at the counts after every step lets the buffers and grids follow them, but leaves
   // the device idle for about 10 us.  Up to 16,384 seeds the levels are enqueued without one
   // (buffers of 16 paths and 8 pairs a seed or what earlier calls needed; 10,000 detections on
-  // each of four cameras: 860 -> 745 us a call).  Above, the looks do not show, while grids
-  // sized by the buffers do (51,000 detections: 114 ms a track sequence with the looks, 117
-  // to 120 without).
+  // each of four cameras: 860 -> 745 us a call), over grids of those guesses or a full chip
+  // (sized by buffers that a dense frame has grown, 300 detections on six cameras take 680 us
+  // instead of the 395 on a fresh context).  Above, the looks do not show (51,000 detections:
+  // 114 ms a track sequence with the looks, 117 to 120 without).
   bool look = v.near_band > 0.0 || n_ref > 16384;
   const int64_t path_guess = std::min<int64_t>(INT32_MAX, std::max<int64_t>(16 * n_ref, 4096));
-  int pair_cap = (int)std::min<int64_t>(INT32_MAX, std::max<int64_t>(8 * n_ref, 4096));
+  const int64_t pair_guess = std::min<int64_t>(INT32_MAX, std::max<int64_t>(8 * n_ref, 4096));
+  const int64_t term_guess = std::max<int64_t>(4 * n_ref, 4096);
+  // threads of a kernel whose count is not known: for the guess or a full chip, within the buffer
+  auto at_once = [](int64_t cap, int64_t guess) {
+    return std::min(cap, std::max<int64_t>(guess, 148 * 2048));
+  };
+  int pair_cap = (int)pair_guess;
   // buffers are grow-only: their capacity from earlier calls avoids a redo
   pair_cap = (int)std::max<int64_t>(pair_cap, (int64_t)(W.pairs.bytes / sizeof(Pair)) - 1);
   DevBuf* in_buf = &W.path_a;
@@ -1397,7 +1420,7 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
     W.cand_ids.ensure((size_t)cap_c * n_cam * sizeof(int), s);
     W.cand_e.ensure((size_t)cap_c * sizeof(double), s);
     W.cand_x.ensure((size_t)cap_c * 3 * sizeof(double), s);
-    check_kernel<<<OLPT_G(std::min(nblk(cap_c, 128), 148 * 64)), 128, 0, s>>>(
+    check_kernel<<<OLPT_G(std::min(nblk(look ? cap_c : at_once(cap_c, term_guess), 128), 148 * 64)), 128, 0, s>>>(
         v, W.term.as<Path>(), cnt + 2 * last, W.cand_ids.as<int>(), W.cand_e.as<double>(),
         W.cand_x.as<double>(), cnt + kCand, cap_c);
     OLPT_CUDA(cudaGetLastError());
@@ -1424,7 +1447,7 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
       }
       // so many blocks that a warp slot gets several chunks of the larger levels, which vary
       const int64_t work =
-          level == 1 ? 32 * (int64_t)in_cap : look ? h[2 * level - 2] : in_cap;
+          level == 1 ? 32 * (int64_t)in_cap : look ? h[2 * level - 2] : at_once(in_cap, path_guess);
       const int pid = ctx->prof.begin(PROF_STEREO, s);
       kern<<<OLPT_G((int)std::min<int64_t>(nblk(work), 148 * 32)), 256, 0, s>>>(
           v, in_buf->p, cnt + 2 * level - 2, in_cap, W.pairs.as<Pair>(), cnt + 2 * level - 1,
@@ -1436,26 +1459,25 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
     // the triangulation gate and the children
     DevBuf* dst = level == last ? &W.term : out_buf;
     const int64_t guess =
-        level == last ? std::max<int64_t>(4 * n_ref, 4096)
+        level == last ? term_guess
         : !look || level == 1 ? path_guess
                               : std::max<int64_t>(4 * (int64_t)h[2 * level - 2], 4096);
     out_cap = (int)std::min<int64_t>(
         INT32_MAX, std::max<int64_t>({(int64_t)out_cap, guess,
                                       (int64_t)(dst->bytes / rec(level + 1)) - 1}));
     dst->ensure((size_t)out_cap * rec(level + 1), s);
-    auto kern = tri_kernel<1>;
+    auto kern = look ? tri_kernel<1, false> : tri_kernel<1, true>;
     switch (level) {
       case 1: break;
-      case 2: kern = tri_kernel<2>; break;
-      case 3: kern = tri_kernel<3>; break;
-      case 4: kern = tri_kernel<4>; break;
-      case 5: kern = tri_kernel<5>; break;
-      case 6: kern = tri_kernel<6>; break;
-      default: kern = tri_kernel<7>; break;
+      case 2: kern = look ? tri_kernel<2, false> : tri_kernel<2, true>; break;
+      case 3: kern = look ? tri_kernel<3, false> : tri_kernel<3, true>; break;
+      case 4: kern = look ? tri_kernel<4, false> : tri_kernel<4, true>; break;
+      case 5: kern = look ? tri_kernel<5, false> : tri_kernel<5, true>; break;
+      case 6: kern = look ? tri_kernel<6, false> : tri_kernel<6, true>; break;
+      default: kern = look ? tri_kernel<7, false> : tri_kernel<7, true>; break;
     }
     const int pid = ctx->prof.begin(PROF_STEREO, s);
-    // a block per 256 pairs; those past the count leave at once
-    const int tiles = nblk(look ? std::min(h[2 * level - 1], pair_cap) : pair_cap);
+    const int tiles = nblk(look ? std::min(h[2 * level - 1], pair_cap) : at_once(pair_cap, pair_guess));
     kern<<<OLPT_G(std::max(tiles, 1)), 256, 0, s>>>(
         v, in_buf->p, W.pairs.as<Pair>(), cnt + 2 * level - 1, pair_cap, dst->p, cnt + 2 * level,
         out_cap);
