@@ -183,11 +183,6 @@ olpt_status_t olpt_ctx_create(olpt_ctx** out, int device) {
     return OLPT_ERR_CUDA;
   }
   ctx->own_stream = true;
-  // without it the read-backs go to pageable memory
-  if (cudaMallocHost(&ctx->pinned.p, kReadBackBytes) == cudaSuccess)
-    ctx->pinned.bytes = kReadBackBytes;
-  else
-    cudaGetLastError();
   *out = ctx;
   return OLPT_OK;
 }

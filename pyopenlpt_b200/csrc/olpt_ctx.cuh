@@ -483,15 +483,17 @@ namespace olpt {
 // and from there to where they belong.  A copy to pageable memory waits for the stream by
 // itself, and goes through a staging area of the driver (a detection list of 1,700 spots in
 // three of them: 30 us, this way 12 us).  What does not fit into the block (results so large
-// that the copy itself counts) is copied directly.  One user at a time, like the context.
-constexpr size_t kReadBackBytes = 1 << 20;
+// that the copy itself counts) is copied directly.  The block starts with the first read-back
+// and grows to what they need, because pinning is paid by the page (64 KB 60 us, 1 MB 1.1 ms):
+// a context that only runs the network has none.  One user at a time, like the context.
+constexpr size_t kReadBackFirst = 64 << 10, kReadBackBytes = 1 << 20;
 
 class ReadBack {
  public:
   explicit ReadBack(olpt_ctx* c) : c_(c) {}
   void add(void* dst, const void* src, size_t bytes) {
     if (!bytes) return;
-    if (n_ < kMax && c_->pinned.p && used_ + bytes <= kReadBackBytes) {
+    if (n_ < kMax && room(bytes)) {
       char* at = c_->pinned.as<char>() + used_;
       OLPT_CUDA(cudaMemcpyAsync(at, src, bytes, cudaMemcpyDeviceToHost, c_->stream));
       part_[n_++] = {dst, at, bytes};
@@ -509,6 +511,24 @@ class ReadBack {
 
  private:
   static constexpr int kMax = 8;
+  // the block holds `bytes` more, after growing where it may
+  bool room(size_t bytes) {
+    HostBuf& b = c_->pinned;
+    if (used_ + bytes <= b.bytes) return true;
+    if (used_ + bytes > kReadBackBytes) return false;
+    size_t size = kReadBackFirst;
+    while (size < used_ + bytes) size *= 2;
+    finish();  // no copy into the block that goes is under way
+    void* p = nullptr;
+    if (cudaMallocHost(&p, size) != cudaSuccess) {
+      cudaGetLastError();
+      return bytes <= b.bytes;
+    }
+    if (b.p) cudaFreeHost(b.p);
+    b.p = p;
+    b.bytes = size;
+    return true;
+  }
   struct Part {
     void* dst;
     const void* at;
