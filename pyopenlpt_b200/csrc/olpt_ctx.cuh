@@ -204,7 +204,7 @@ struct PruneView {
 
 // Device workspace of the candidate sort and prune (prune.cu).
 struct PruneWork {
-  DevBuf key, val, key2, val2, hist, scan_tmp;
+  DevBuf key, val, key2, val2, hist, hist2, scan_tmp;
   DevBuf ids_s, e_s, X_s;
   DevBuf fl, slot_key, fcnt, slot_pct, slot_used, pct;
   DevBuf counts;  // PruneCount words (prune.cu)
@@ -216,7 +216,7 @@ struct PruneWork {
   int cluster = -1;  // the device runs clusters of 16 sort blocks (-1: not asked yet)
   HostBuf pin;    // pinned staging of the sequential greedy's input
   void release(cudaStream_t s) {
-    for (DevBuf* b : {&key, &val, &key2, &val2, &hist, &scan_tmp, &ids_s, &e_s, &X_s, &fl,
+    for (DevBuf* b : {&key, &val, &key2, &val2, &hist, &hist2, &scan_tmp, &ids_s, &e_s, &X_s, &fl,
                       &slot_key, &fcnt, &slot_pct, &slot_used, &pct, &counts, &pcls, &ecls,
                       &cstart, &tiles, &mixed, &g_pts, &g_cnt, &g_pct, &g_e, &pool_e, &pool_i,
                       &gstate, &gfirst, &gowner, &sel, &spos, &scnt})

@@ -44,12 +44,19 @@ inline int nblk(int64_t n, int t = 256) { return (int)((n + t - 1) / t); }
 // Stable LSD sort by 8-bit digits, two launches a digit: the tiles' digit counts, and the
 // scatter, whose blocks add up the counts of the tiles before theirs themselves (5 launches
 // with a device-wide scan of the counts in between; 30,000 keys of 64 bits: 72 us instead of
-// 200).  A warp owns 256 consecutive items of the tile and ranks them without block barriers.
+// 200).  Those sums grow with the square of the tiles, so above kRsSumTiles the counts lie by
+// digit and are scanned.  Counts, scan and scatter of a digit at 2, 8 and 16 million keys: 61,
+// 403 and 1,293 us with sums in every block, 40, 118 and 221 us with the scan.  A warp owns
+// 256 consecutive items of the tile and ranks them without block barriers.
 constexpr int kRsThreads = 512;
 constexpr int kRsWarps = kRsThreads / 32;
 constexpr int kRsItems = 8;
 constexpr int kRsTile = kRsThreads * kRsItems;
+// 0.5 and 1 million keys, a digit: 23 and 30 us with the sums, 25 and 29 us with the scan
+constexpr int kRsSumTiles = 256;
 
+// counts by tile, or (SCANNED) by digit
+template <bool SCANNED>
 __global__ void __launch_bounds__(kRsThreads) rs_hist_kernel(const uint64_t* key, int n, int shift,
                                                              int* hist) {
   __shared__ int h[256];
@@ -62,7 +69,9 @@ __global__ void __launch_bounds__(kRsThreads) rs_hist_kernel(const uint64_t* key
     if (i < n) atomicAdd(&h[(int)((key[i] >> shift) & 255u)], 1);
   }
   __syncthreads();
-  if (threadIdx.x < 256) hist[blockIdx.x * 256 + threadIdx.x] = h[threadIdx.x];
+  if (threadIdx.x < 256)
+    hist[SCANNED ? threadIdx.x * gridDim.x + blockIdx.x : blockIdx.x * 256 + threadIdx.x] =
+        h[threadIdx.x];
 }
 
 // Exclusive prefix sums of the first 256 threads' values.
@@ -81,6 +90,8 @@ __device__ __forceinline__ int scan256(int x, int* wsum) {
   return before + incl - x;
 }
 
+// hist: the tiles' counts, or (SCANNED) the first position of every digit and tile
+template <bool SCANNED>
 __global__ void __launch_bounds__(kRsThreads) rs_scatter_kernel(const uint64_t* key, const int* val,
                                                                 int n, int shift, const int* hist,
                                                                 int n_blocks, uint64_t* key_out,
@@ -89,25 +100,31 @@ __global__ void __launch_bounds__(kRsThreads) rs_scatter_kernel(const uint64_t* 
   __shared__ int half_all[256], half_before[256], wsum[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int d = threadIdx.x & 255, half = threadIdx.x >> 8;
-  // this digit's count in all tiles and in the tiles before, over every second tile
-  int all = 0, before = 0;
-#pragma unroll 8
-  for (int b = half; b < n_blocks; b += 2) {
-    const int x = hist[b * 256 + d];
-    all += x;
-    before += b < (int)blockIdx.x ? x : 0;
-  }
-  if (half) {
-    half_all[d] = all;
-    half_before[d] = before;
-  }
   for (int q = threadIdx.x; q < kRsWarps * 256; q += kRsThreads) (&cnt[0][0])[q] = 0;
-  __syncthreads();
-  if (!half) {
-    all += half_all[d];
-    before += half_before[d];
+  int base = 0;
+  if constexpr (SCANNED) {
+    if (!half) base = hist[d * n_blocks + blockIdx.x];
+    __syncthreads();
+  } else {
+    // this digit's count in all tiles and in the tiles before, over every second tile
+    int all = 0, before = 0;
+#pragma unroll 8
+    for (int b = half; b < n_blocks; b += 2) {
+      const int x = hist[b * 256 + d];
+      all += x;
+      before += b < (int)blockIdx.x ? x : 0;
+    }
+    if (half) {
+      half_all[d] = all;
+      half_before[d] = before;
+    }
+    __syncthreads();
+    if (!half) {
+      all += half_all[d];
+      before += half_before[d];
+    }
+    base = scan256(half ? 0 : all, wsum) + before;
   }
-  int base = scan256(half ? 0 : all, wsum) + before;
   const int i0 = blockIdx.x * kRsTile + w * (32 * kRsItems) + lane;
   uint64_t kk[kRsItems];
   int vv[kRsItems];
@@ -878,13 +895,18 @@ static void radix_sort_device(PruneWork& W, int n, int bits, cudaStream_t s) {
     }
   }
   const int n_blocks = (n + kRsTile - 1) / kRsTile;
+  const bool scanned = n_blocks > kRsSumTiles;
+  auto hist = scanned ? rs_hist_kernel<true> : rs_hist_kernel<false>;
+  auto scatter = scanned ? rs_scatter_kernel<true> : rs_scatter_kernel<false>;
   W.hist.ensure((size_t)256 * n_blocks * sizeof(int), s);
+  if (scanned) W.hist2.ensure(((size_t)256 * n_blocks + 1) * sizeof(int), s);
   for (int shift = 0; shift < bits; shift += 8) {
-    rs_hist_kernel<<<OLPT_G(n_blocks), kRsThreads, 0, s>>>(W.key.as<uint64_t>(), n, shift,
-                                                          W.hist.as<int>());
-    rs_scatter_kernel<<<OLPT_G(n_blocks), kRsThreads, 0, s>>>(
-        W.key.as<uint64_t>(), W.val.as<int>(), n, shift, W.hist.as<int>(), n_blocks,
-        W.key2.as<uint64_t>(), W.val2.as<int>());
+    hist<<<OLPT_G(n_blocks), kRsThreads, 0, s>>>(W.key.as<uint64_t>(), n, shift, W.hist.as<int>());
+    if (scanned)
+      exclusive_scan(W.hist.as<int>(), 256 * n_blocks, W.hist2.as<int>(), W.scan_tmp, s);
+    scatter<<<OLPT_G(n_blocks), kRsThreads, 0, s>>>(
+        W.key.as<uint64_t>(), W.val.as<int>(), n, shift, (scanned ? W.hist2 : W.hist).as<int>(),
+        n_blocks, W.key2.as<uint64_t>(), W.val2.as<int>());
     std::swap(W.key, W.key2);
     std::swap(W.val, W.val2);
   }
