@@ -118,7 +118,6 @@ struct OtfDev {
   int nx = 2, ny = 2, nz = 2, n_grid = 8;
   double bmin[3], bmax[3];
   double d[3];  // grid spacing
-  double* table = nullptr;  // [4][n_cam][n_grid] a,b,c,alpha (device)
   int alpha_zero = 0;       // every alpha entry is +0.0 (cos = 1, sin = +0 exactly)
 };
 

@@ -31,7 +31,6 @@ struct ShakeView {
   OtfView otf;
   double r_px, ratio;
   int roi_area;          // augmented ROI pixels (side^2)
-  int exact_sums;        // FP64 path: row-major sequential sums
   PlaneView orig[OLPT_MAX_CAM];  // current images (u8/u16/f32/f64)
   PlaneView res[OLPT_MAX_CAM];   // residual planes (Real)
   PlaneView proj[OLPT_MAX_CAM];  // projection planes (Real), 0 outside a pass

@@ -5,7 +5,7 @@
 //  1. sort by ids (lexicographic, camera 0 first; -1 < any id) with a stable LSD
 //     radix sort of packed 64-bit keys;
 //  2. every candidate's 2D points (global point index per active camera, camera
-//     order) and the point -> candidate lists (CSR, ascending candidate);
+//     order) and the point -> candidate lists (CSR, in any order);
 //  3. per 2D point (one warp): the percentile of every candidate in the point's pool.
 //     The reference stable-sorts the pool with a tolerance comparator (rtol 1e-9,
 //     atol 1e-12) and averages ranks over runs of tolerance-equal e_check.  When the

@@ -188,7 +188,8 @@ __global__ void __launch_bounds__(256) residual_kernel(const __grid_constant__ S
 // ---------------------------------------------------------------- 3. shake
 // Camera parameters of a block in shared memory, [value][camera] so that the lanes of a
 // group, each on its own camera, read neighbouring words.  Polynomial terms keep their
-// coefficients as they are and their exponents (all 0..3, CamDev::pow3) as 2-bit fields.
+// coefficients as they are and their exponents (all 0..3, CamDev::pow3) as byte offsets of the
+// factors in the point's power list (CamSmem::expo).
 constexpr int kCamVals = 28;  // R 9, T 3, fx fy cx cy, distortion 12
 
 struct Strided {
@@ -1257,7 +1258,7 @@ __global__ void score_scale_kernel(double* score, const uint8_t* act, int64_t n,
   score[i] = pow(score[i], expo);
 }
 
-static ShakeView make_view(olpt_ctx* ctx, const ShakeParams& sp, bool fp64) {
+static ShakeView make_view(olpt_ctx* ctx, const ShakeParams& sp) {
   ShakeView v{};
   v.n_cam = ctx->n_cam;
   v.cams = ctx->cams_d.as<CamDev>();
@@ -1271,7 +1272,6 @@ static ShakeView make_view(olpt_ctx* ctx, const ShakeParams& sp, bool fp64) {
   const int win = (int)std::lround(2.0 * sp.radius_obj);
   OLPT_REQUIRE(win >= 1 && win < 32, OLPT_ERR_UNSUPPORTED,
                "projection window round(2 * radius_obj) must be below 32 px");
-  v.exact_sums = fp64 ? 1 : 0;
   for (int c = 0; c < ctx->n_cam; ++c) {
     const CamDev& cm = ctx->cams_h[c];
     const ImagePlane& im = ctx->img[c];
@@ -1548,7 +1548,7 @@ template <typename Real>
 static void shake_impl(olpt_ctx* ctx, const ShakeParams& sp) {
   const bool fp64 = sizeof(Real) == 8;
   cudaStream_t s = ctx->stream;
-  ShakeView v = make_view(ctx, sp, fp64);
+  ShakeView v = make_view(ctx, sp);
   ensure_residual_planes(ctx, v, fp64);
   const int64_t n = ctx->obj.n;
   ctx->obj.ensure(std::max<int64_t>(n, 1), ctx->n_cam, s);
@@ -1563,7 +1563,7 @@ static void learned_impl(olpt_ctx* ctx, const ShakeParams& sp) {
   cudaStream_t s = ctx->stream;
   MlpWork& M = ctx->mlp;
   const LearnedParams& lp = M.lp;
-  ShakeView v = make_view(ctx, sp, fp64);
+  ShakeView v = make_view(ctx, sp);
   ensure_residual_planes(ctx, v, fp64);
   int64_t n = ctx->obj.n;
   const int C = ctx->n_cam;
@@ -1635,7 +1635,7 @@ static void learned_impl(olpt_ctx* ctx, const ShakeParams& sp) {
 
 void residual_all_device(olpt_ctx* ctx, const ShakeParams& sp) {
   const bool fp64 = sp.precision == 1;
-  ShakeView v = make_view(ctx, sp, fp64);
+  ShakeView v = make_view(ctx, sp);
   ensure_residual_planes(ctx, v, fp64);
   if (fp64)
     residual_pass<double>(ctx, v, nullptr, 0, 0);
@@ -1667,7 +1667,7 @@ void shake_device(olpt_ctx* ctx, const ShakeParams& sp) {
 // images when make_current.
 void residual_device(olpt_ctx* ctx, const ShakeParams& sp, bool use_flags, bool make_current) {
   const bool fp64 = sp.precision == 1;
-  ShakeView v = make_view(ctx, sp, fp64);
+  ShakeView v = make_view(ctx, sp);
   ensure_residual_planes(ctx, v, fp64);
   const uint8_t* fl = use_flags ? ctx->obj.flags.as<uint8_t>() : nullptr;
   if (fp64)
