@@ -278,10 +278,10 @@ typedef struct olpt_ipr_params {
  * tolerance growing x1.5 per loop.  The current images end as the final residual.
  * n_objects receives the number of reconstructed objects. */
 olpt_status_t olpt_ipr_run(olpt_ctx* ctx, const olpt_ipr_params* p, int64_t* n_objects);
-/* Launch shapes of the shake (warps per block: 1, 2 or 4; shake_regs 64: the kernel built
- * for 4 resident blocks per SM, 128 registers a thread; 128: for 5 blocks, 102 registers)
- * and of the residual image (threads per block: 128 or 256).  They change only
- * the speed: every result is the same for every choice.  Default {4, 256, 64}. */
+/* Launch shapes of the shake (warps per block: 1, 2 or 4) and of the residual image (threads
+ * per block: 128 or 256).  They change only the speed: every result is the same for every
+ * choice.  shake_regs (64 or 128) chose between two builds of the shake; there is one, and both
+ * values run it.  Default {4, 256, 64}. */
 typedef struct olpt_tuning {
   int shake_warps_per_block;
   int residual_threads;

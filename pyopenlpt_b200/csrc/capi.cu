@@ -1005,15 +1005,16 @@ olpt_status_t olpt_tuning_set(olpt_ctx* ctx, const olpt_tuning* t) {
   });
 }
 
-static const olpt_tuning kTuneCand[OLPT_TUNING_CANDIDATES] = {
-    {4, 256, 64},  {2, 256, 64},  {1, 256, 64},  {4, 256, 128},
-    {2, 256, 128}, {4, 128, 64},  {2, 128, 64},  {4, 128, 128}};
+static const olpt_tuning kTuneCand[] = {
+    {4, 256, 64}, {2, 256, 64}, {1, 256, 64}, {4, 128, 64}, {2, 128, 64}};
+constexpr int kTuneCands = (int)(sizeof(kTuneCand) / sizeof(kTuneCand[0]));
+static_assert(kTuneCands <= OLPT_TUNING_CANDIDATES, "callers' arrays");
 
 olpt_status_t olpt_tuning_candidates(olpt_tuning* out, int* n) {
   if (!n) return OLPT_ERR_INVALID_ARG;
-  *n = OLPT_TUNING_CANDIDATES;
+  *n = kTuneCands;
   if (out)
-    for (int i = 0; i < OLPT_TUNING_CANDIDATES; ++i) out[i] = kTuneCand[i];
+    for (int i = 0; i < kTuneCands; ++i) out[i] = kTuneCand[i];
   return OLPT_OK;
 }
 
@@ -1065,7 +1066,7 @@ olpt_status_t olpt_autotune_ipr(olpt_ctx* ctx, const olpt_ipr_params* p, int rep
     double best_t = 0;
     olpt_tuning pick = start;
     try {
-      for (int k = 0; k < OLPT_TUNING_CANDIDATES; ++k) {
+      for (int k = 0; k < kTuneCands; ++k) {
         ctx->tune = cand[k];
         restore();
         run(&got);  // untimed: warms the launch shape, and its objects are checked

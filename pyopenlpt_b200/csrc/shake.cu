@@ -645,8 +645,10 @@ __device__ __forceinline__ double group_median(double x, bool has) {
 // copy of the evaluation serves every step, entered by the block's warps together.
 // 120,000 objects on six polynomial cameras: 2.3 ms a launch, 52% of the issue slots (9.0 ms
 // and 50% with one warp per object); every sum keeps its order, so results are unchanged.
-template <typename Real, int NC, int LPO, int MINB>
-__global__ void __launch_bounds__(128, MINB) shake_kernel(const __grid_constant__ ShakeView v,
+// Four resident blocks an SM (128 registers a thread); built for five (102 registers), 8,000
+// objects take 126 us instead of 115, 32,000 of six cameras 767 instead of 694.
+template <typename Real, int NC, int LPO>
+__global__ void __launch_bounds__(128, 4) shake_kernel(const __grid_constant__ ShakeView v,
                                                        int64_t n, double* xyz, double* uv,
                                                        const Real* otfp, double* score,
                                                        double delta, const uint8_t* active,
@@ -1402,15 +1404,15 @@ static void shake_layout(ShakeView& v, int lpo, bool fp64) {
   v.obj_stride = off;
 }
 
-template <typename Real, int NC, int LPO, int MINB>
+template <typename Real, int NC, int LPO>
 static void launch_shake(int warps, cudaStream_t s, const ShakeView& v, int64_t n, double* xyz,
                          double* uv, const Real* otfp, double* score, double delta,
                          const uint8_t* active, double* resid_out) {
   const size_t per_warp = v.obj_stride * (32 / LPO);
   while (warps > 1 && v.cam_bytes + per_warp * warps > kShakeSmemMax) warps /= 2;
   const size_t smem = v.cam_bytes + per_warp * warps;
-  allow_smem<shake_kernel<Real, NC, LPO, MINB>>(smem);
-  shake_kernel<Real, NC, LPO, MINB><<<OLPT_G(nblk(n, warps * (32 / LPO))), 32 * warps, smem, s>>>(
+  allow_smem<shake_kernel<Real, NC, LPO>>(smem);
+  shake_kernel<Real, NC, LPO><<<OLPT_G(nblk(n, warps * (32 / LPO))), 32 * warps, smem, s>>>(
       v, n, xyz, uv, otfp, score, delta, active, resid_out);
 }
 
@@ -1422,35 +1424,35 @@ static void launch_shake(int warps, cudaStream_t s, const ShakeView& v, int64_t 
 // shared memory holds too few 8-lane groups (32,000 objects: 1,879 us with 8, 1,382 with 32).
 constexpr int64_t kWaveObjects = 148 * 16;
 
-template <typename Real, int NC, int MINB>
+template <typename Real, int NC>
 static void launch_shake_nc(int warps, cudaStream_t s, ShakeView& v, int64_t n, double* xyz,
                             double* uv, const Real* otfp, double* score, double delta,
                             const uint8_t* active, double* resid_out) {
   if constexpr (sizeof(Real) == 4) {
     shake_layout(v, 8, false);
     if (n > kWaveObjects && v.cam_bytes + 4 * v.obj_stride <= kShakeSmemMax) {
-      launch_shake<Real, NC, 8, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active,
+      launch_shake<Real, NC, 8>(warps, s, v, n, xyz, uv, otfp, score, delta, active,
                                       resid_out);
       return;
     }
   }
   shake_layout(v, 32, sizeof(Real) == 8);
-  launch_shake<Real, NC, 32, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active,
+  launch_shake<Real, NC, 32>(warps, s, v, n, xyz, uv, otfp, score, delta, active,
                                    resid_out);
 }
 
-template <typename Real, int MINB>
+template <typename Real>
 static void launch_shake_cams(int warps, cudaStream_t s, ShakeView& v, int64_t n, double* xyz,
                               double* uv, const Real* otfp, double* score, double delta,
                               const uint8_t* active, double* resid_out) {
   switch (v.n_cam) {
-    case 2: launch_shake_nc<Real, 2, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
-    case 3: launch_shake_nc<Real, 3, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
-    case 4: launch_shake_nc<Real, 4, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
-    case 5: launch_shake_nc<Real, 5, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
-    case 6: launch_shake_nc<Real, 6, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
-    case 7: launch_shake_nc<Real, 7, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
-    default: launch_shake_nc<Real, 8, MINB>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
+    case 2: launch_shake_nc<Real, 2>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
+    case 3: launch_shake_nc<Real, 3>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
+    case 4: launch_shake_nc<Real, 4>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
+    case 5: launch_shake_nc<Real, 5>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
+    case 6: launch_shake_nc<Real, 6>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
+    case 7: launch_shake_nc<Real, 7>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
+    default: launch_shake_nc<Real, 8>(warps, s, v, n, xyz, uv, otfp, score, delta, active, resid_out); break;
   }
 }
 
@@ -1481,15 +1483,10 @@ static void shake_iterations(olpt_ctx* ctx, const ShakeParams& sp, ShakeView& v,
     parabola_matrix(x3, 3, B);
     for (int r = 0; r < 2; ++r)
       for (int i = 0; i < 3; ++i) v.fit3[r][i] = B[r + 1][i];
-    if (n > 0) {
-      // the build for four resident blocks per SM (128 registers a thread) is the default; for
-      // five (102 registers) 8,000 objects take 126 us instead of 115, 32,000 of six cameras
-      // 767 instead of 694
-      auto launch = ctx->tune.shake_regs >= 128 ? launch_shake_cams<Real, 5>
-                                                : launch_shake_cams<Real, 4>;
-      launch(warps_per_blk, s, v, n, ctx->obj.xyz.as<double>(), ctx->obj.uv.as<double>(),
-             W.otfp.as<Real>(), ctx->obj.score.as<double>(), delta, active, resid_out);
-    }
+    if (n > 0)
+      launch_shake_cams<Real>(warps_per_blk, s, v, n, ctx->obj.xyz.as<double>(),
+                              ctx->obj.uv.as<double>(), W.otfp.as<Real>(),
+                              ctx->obj.score.as<double>(), delta, active, resid_out);
     ctx->prof.end(PROF_SHAKE, pid, s, bytes);
     OLPT_CUDA(cudaGetLastError());
     delta *= 0.5;
