@@ -249,6 +249,15 @@ def reference_ipr_time(sc, s, threads: int, images=None):
     return len(out["xyz"]), dt
 
 
+def reference_missing():
+    """Why the reference arm and the CPU baseline cannot run here, or None."""
+    from oracle import ref
+    if os.path.exists(ref.REF_SO):
+        return None
+    return ("oracle/_ref/liboref.so is not built (it is compiled from the reference's sources, "
+            "which are not here)")
+
+
 REF_STB_BUDGET_S = 420.0  # convergence frames of the reference arm stop after this
 
 
@@ -284,6 +293,10 @@ def reference_stb(name, threads, warmup, steps, budget_s, converge=None):
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return 0
+    why = reference_missing()
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
         return 0
     threads = os.cpu_count() or 1
     kind = WORKLOADS[args.workload]["kind"]
@@ -1269,6 +1282,10 @@ def detection_roofline(args, o: Ours):
 
 
 def run_ours(args):
+    why = None if args.no_cpu_baseline else reference_missing()
+    if why:
+        args.no_cpu_baseline = True
+        print(f"no CPU baseline: {why}", file=sys.stderr)
     o = Ours(args)
     learned = None
     if o.world == 1 and args.learn_ipr_frames > 0:
