@@ -152,9 +152,11 @@ __device__ __forceinline__ bool fit_at(const PeakCam& c, const double* lut, int 
   return fit3(l, m, h, col, x) && fit3(u, m, d, r, y);
 }
 
-// Evaluate one chunk; returns a bitmask of detections (bit j = pixel c0 + j).
+// Evaluate one chunk; returns a bitmask of detections (bit j = pixel c0 + j).  Of floating-point
+// levels it takes the fits to decide: they go to xy, in order (4-neighbour maxima: N / 2).
 template <typename T, int N>
-__device__ __forceinline__ unsigned eval_chunk(const PeakCam& c, const PeakArgs& a, int r, int c0) {
+__device__ __forceinline__ unsigned eval_chunk(const PeakCam& c, const PeakArgs& a, int r, int c0,
+                                               double2 (&xy)[N / 2]) {
   if (r < 1 || r > c.H - 2) return 0u;
   T cen[N];
   load_chunk<T, N>(c, r, c0, cen);
@@ -185,11 +187,17 @@ __device__ __forceinline__ unsigned eval_chunk(const PeakCam& c, const PeakArgs&
   // integer levels: a local maximum always has a finite centre (see mask_staged)
   if constexpr (std::is_integral<T>::value) return cand;
   unsigned mask = 0u;
+  int n = 0;
   while (cand) {
     const int j = __ffs(cand) - 1;
     cand &= cand - 1;
     double x, y;
-    if (fit_at<T>(c, a.lut, r, c0 + j, x, y)) mask |= 1u << j;
+    if (!fit_at<T>(c, a.lut, r, c0 + j, x, y)) continue;
+    mask |= 1u << j;
+#pragma unroll
+    for (int q = 0; q < N / 2; ++q)
+      if (q == n) xy[q] = make_double2(x, y);
+    ++n;
   }
   return mask;
 }
@@ -205,8 +213,12 @@ __device__ __forceinline__ int find_cam(const PeakArgs& a, int blk) {
 // memory (256 chunks at a time), fits them one per thread and stores coalesced.  Bands of 512
 // chunks: 2048^2 u16 makes 1,024 blocks where bands of 2,048 made 256, fewer than two a SM,
 // and the fits ran on the few lanes of a warp that held a detection, for each of the chunk's
-// pixels in turn (400,000 spots: 84 us a call before, 27 us with these bands).
-template <typename T, bool EMIT>
+// pixels in turn (400,000 spots: 84 us a call before, 27 us with these bands).  KEEP, for
+// floating-point levels: the fits that decided are listed too, not repeated (launch_peaks).  A
+// wide row is a band of dozens of rounds, each a chain of its barriers: one where no spot is
+// found, two else (100 x 16,384 with 819 spots, EMIT: f64 73 -> 53 us, f32 48 -> 33 us against
+// three barriers and the fits repeated).
+template <typename T, bool EMIT, bool KEEP>
 __global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
   constexpr int N = 16 / sizeof(T);
   const int cam = find_cam(a, blockIdx.x);
@@ -218,20 +230,22 @@ __global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
   const int rows = min(c.band_rows, c.H - r0);
   const int total = rows * cpr;
 
-  __shared__ int warp_sums[kPeakThreads / 32];
+  __shared__ int warp_sums[2][kPeakThreads / 32];  // of this round and the one before
   // 4-neighbour maxima: at most half the pixels of 256 chunks
   __shared__ uint32_t list[EMIT ? kPeakThreads * N / 2 : 1];
+  __shared__ double2 fits[EMIT && KEEP ? kPeakThreads * N / 2 : 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int64_t base = EMIT ? a.band_offsets[blockIdx.x] : 0;
   int count = 0;
-  for (int start = 0; start < total; start += kPeakThreads) {
+  for (int start = 0, round = 0; start < total; start += kPeakThreads, round ^= 1) {
     const int i = start + threadIdx.x;
     unsigned mask = 0u;
     int lr = 0, c0 = 0;
+    double2 xy[N / 2];
     if (i < total) {
       lr = i / cpr;
       c0 = (i - lr * cpr) * N;
-      mask = eval_chunk<T, N>(c, a, r0 + lr, c0);
+      mask = eval_chunk<T, N>(c, a, r0 + lr, c0, xy);
     }
     const int n = __popc(mask);
     if (!EMIT) {
@@ -245,15 +259,21 @@ __global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
       int t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
-    if (lane == 31) warp_sums[wid] = incl;
-    __syncthreads();
+    if (lane == 31) warp_sums[round][wid] = incl;
+    __syncthreads();  // also: the list of the round before is no longer read
     int before = 0, all = 0;
 #pragma unroll
     for (int w = 0; w < kPeakThreads / 32; ++w) {
-      before += w < wid ? warp_sums[w] : 0;
-      all += warp_sums[w];
+      before += w < wid ? warp_sums[round][w] : 0;
+      all += warp_sums[round][w];
     }
+    if (all == 0) continue;
     int pos = before + incl - n;
+    if constexpr (KEEP) {
+#pragma unroll
+      for (int q = 0; q < N / 2; ++q)
+        if (q < n) fits[pos + q] = xy[q];
+    }
     while (mask) {
       const int j = __ffs(mask) - 1;
       mask &= mask - 1;
@@ -263,22 +283,24 @@ __global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
     for (int k = threadIdx.x; k < all; k += kPeakThreads) {
       const int p = (int)list[k], lrow = p / (cpr * N);
       const int r = r0 + lrow, col = p - lrow * cpr * N;
-      double x, y;
-      fit_at<T>(c, a.lut, r, col, x, y);
-      c.x[base + k] = x;
-      c.y[base + k] = y;
+      double2 at;
+      if constexpr (KEEP)
+        at = fits[k];
+      else
+        fit_at<T>(c, a.lut, r, col, at.x, at.y);
+      c.x[base + k] = at.x;
+      c.y[base + k] = at.y;
       c.rc[base + k] = make_int2(r, col);
     }
     base += all;
-    __syncthreads();
   }
   if (!EMIT) {
     count = __reduce_add_sync(0xffffffffu, count);
-    if (lane == 0) warp_sums[wid] = count;
+    if (lane == 0) warp_sums[0][wid] = count;
     __syncthreads();
     if (threadIdx.x == 0) {
       int acc = 0;
-      for (int w = 0; w < kPeakThreads / 32; ++w) acc += warp_sums[w];
+      for (int w = 0; w < kPeakThreads / 32; ++w) acc += warp_sums[0][w];
       a.band_counts[blockIdx.x] = acc;
     }
   }
@@ -319,19 +341,26 @@ __global__ void __launch_bounds__(1024) band_scan_kernel(const PeakArgs a, int64
   if (threadIdx.x == 0) totals[cam] = run;
 }
 
+// Whether EMIT keeps the fits: of f64 always (2048^2, 200,000 spots: 83 -> 67 us), of f32 where a
+// row is more than a band's chunks, so that few blocks run long chains (16 x 20,000: 57 -> 40
+// us; elsewhere the larger shared memory costs more, 2048^2: 53 -> 65 us); integers have none.
 template <typename T>
 void launch_peaks(const PeakArgs& a, int n_blocks, int64_t* band_offsets, int64_t* totals,
                   cudaStream_t s) {
-  peaks_kernel<T, false><<<OLPT_G(n_blocks), kPeakThreads, 0, s>>>(a);
+  peaks_kernel<T, false, false><<<OLPT_G(n_blocks), kPeakThreads, 0, s>>>(a);
   OLPT_CUDA(cudaGetLastError());
   band_scan_kernel<<<OLPT_G(a.n_cam), 1024, 0, s>>>(a, band_offsets, totals);
   OLPT_CUDA(cudaGetLastError());
   PeakArgs b = a;
   b.band_offsets = band_offsets;
-  peaks_kernel<T, true><<<OLPT_G(n_blocks), kPeakThreads, 0, s>>>(b);
+  auto emit = peaks_kernel<T, true, std::is_same<T, double>::value>;
+  if constexpr (std::is_same<T, float>::value) {
+    for (int c = 0; c < a.n_cam; ++c)
+      if (a.cam[c].W > kBandChunks * (int)(16 / sizeof(T))) emit = peaks_kernel<T, true, true>;
+  }
+  emit<<<OLPT_G(n_blocks), kPeakThreads, 0, s>>>(b);
   OLPT_CUDA(cudaGetLastError());
 }
-
 
 // ---------------------------------------------------------------------------
 // Staged single-read detector.
