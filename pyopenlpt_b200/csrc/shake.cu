@@ -326,7 +326,7 @@ struct Obj {
   double* dd;      // n_cam x (roi_area + 1): squared differences (FP64 ordered sums)
   double2* uv;     // [j][c] projection
   Real* otf;       // [j][c][5]
-  uint32_t* win;   // [j][c] rows (bits 0..7) and columns (8..15) of the ROI in the window
+  uint32_t* win;   // [j][c] rows (bits 0..15) and columns (16..31) of the ROI in the window
   int4* roi;       // [c] rmin, rmax, cmin, cmax
   Real* ey;        // [8] row factors of the camera and point at work
   double* pw;      // [j][3][4] powers of the points' coordinates (polynomial cameras)
@@ -346,9 +346,9 @@ __device__ __forceinline__ Obj<Real> obj_smem(const ShakeView& v, unsigned char*
   return s;
 }
 
-// The projection window's rows / columns [lo, hi) within 8 ROI rows / columns from r0.
-__device__ __forceinline__ uint32_t span8(int lo, int hi, int r0) {
-  const int a = max(0, min(8, lo - r0)), b = max(0, min(8, hi - r0));
+// The projection window's rows / columns [lo, hi) within 16 ROI rows / columns from r0.
+__device__ __forceinline__ uint32_t span16(int lo, int hi, int r0) {
+  const int a = max(0, min(16, lo - r0)), b = max(0, min(16, hi - r0));
   return b > a ? ((1u << b) - 1u) & ~((1u << a) - 1u) : 0u;
 }
 
@@ -367,9 +367,9 @@ __device__ __forceinline__ void eval_slot(const ShakeView& v, const CamSmem& cs,
   const int4 R = S.roi[c];
   // TracerShakeStrategy::calShakeResidue's window (Shake.cpp:951-1045)
   const uint32_t rows =
-      span8((int)floor(w - v.r_px), min(R.y, (int)ceil(w + v.r_px + 1)), R.x);
-  const uint32_t cols = span8((int)floor(u - v.r_px), (int)ceil(u + v.r_px + 1), R.z);
-  S.win[j * NC + c] = rows | (cols << 8);
+      span16((int)floor(w - v.r_px), min(R.y, (int)ceil(w + v.r_px + 1)), R.x);
+  const uint32_t cols = span16((int)floor(u - v.r_px), (int)ceil(u + v.r_px + 1), R.z);
+  S.win[j * NC + c] = rows | (cols << 16);
 }
 
 template <typename Real>
@@ -440,28 +440,39 @@ __device__ __forceinline__ void residue(const ShakeView& v, Obj<Real>& S, int nj
     const int h = R.y - R.x, w = R.w - R.z;
     const bool some = h > 0 && w > 0;
     used += some ? 1 : 0;
-    const bool fast = area == 64 && __all_sync(kFull, w == 8 || !some);
-    const int col = g & 7;
-    Real m[64 / LPO];
-    if (fast) {
+    // the lanes' sums for point j -> the camera's mean
+    auto add = [&](int j, Real s) {
+#pragma unroll
+      for (int o = LPO / 2; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+      if (some) {
+        const double t = w * h == 64 ? (double)s * 0.015625 : (double)s / (double)(w * h);
+        if (j == 0)
+          cost[0] += t;
+        else if (j == 1)
+          cost[1] += t;
+        else
+          cost[2] += t;
+      }
+    };
+    if (area == 64 && __all_sync(kFull, w == 8 || !some)) {
       // an ROI of 8 columns: the lane's pixels lie in one column, rows g / 8 + LPO / 8 i
+      const int col = g & 7;
+      Real m[64 / LPO];
 #pragma unroll
       for (int i = 0; i < 64 / LPO; ++i)
         m[i] = (g >> 3) + (LPO / 8) * i < h ? S.aug[c * area + LPO * i + g] : (Real)0;
-    }
 #pragma unroll 1
-    for (int j = 0; j < nj; ++j) {
-      const int e = j * NC + c;
-      Real part[NA];
+      for (int j = 0; j < nj; ++j) {
+        const int e = j * NC + c;
+        Real part[NA];
 #pragma unroll
-      for (int k = 0; k < NA; ++k) part[k] = (Real)0;
-      const double2 uw = S.uv[e];
-      if (fast) {
+        for (int k = 0; k < NA; ++k) part[k] = (Real)0;
+        const double2 uw = S.uv[e];
         Real o[5], fy[64 / LPO];
 #pragma unroll
         for (int k = 0; k < 5; ++k) o[k] = S.otf[5 * e + k];
         const uint32_t win = S.win[e];
-        const Real fx = axis_factor<Real>(sep, R.z + col, uw.x, o[1], (win >> (8 + col)) & 1u);
+        const Real fx = axis_factor<Real>(sep, R.z + col, uw.x, o[1], (win >> (16 + col)) & 1u);
         if (g < 8)
           S.ey[g] = axis_factor<Real>(sep, R.x + g, uw.y, o[2], (win >> g) & 1u);
         __syncwarp();
@@ -482,50 +493,66 @@ __device__ __forceinline__ void residue(const ShakeView& v, Obj<Real>& S, int nj
         else
           pixels(std::false_type{});
         __syncwarp();
-      } else if (some) {
-        int first = g;
         if (sizeof(Real) == 4) {
-          first = (g - c * area) % LPO;
-          if (first < 0) first += LPO;
+#pragma unroll
+          for (int o = NA / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < o; ++k) part[k] += part[k + o];
+          add(j, part[0]);
         }
-        const int r0 = (int)floor(uw.y - v.r_px), r1 = (int)ceil(uw.y + v.r_px + 1);
-        const int c0 = (int)floor(uw.x - v.r_px), c1 = (int)ceil(uw.x + v.r_px + 1);
-        const int n = w * h;
-        int k = 0;
+      }
+      continue;
+    }
+    // an ROI of another size: a pixel's place and value serve the points together (20,000 objects
+    // on four cameras, 32 lanes, ROIs of 256 pixels: 1,297 -> 1,199 us against one point after
+    // the other)
+    Real part[3][NA];
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int k = 0; k < NA; ++k) part[j][k] = (Real)0;
+    if (some) {
+      int first = g;
+      if (sizeof(Real) == 4) {
+        first = (g - c * area) % LPO;
+        if (first < 0) first += LPO;
+      }
+      const int n = w * h;
+      int k = 0;
 #pragma unroll 1
-        for (int p = first; p < n; p += LPO, k = (k + 1) % NA) {
-          const int row = R.x + p / w, cc = R.z + p % w;
+      for (int p = first; p < n; p += LPO, k = (k + 1) % NA) {
+        const int pr = p / w, pc = p - pr * w;
+        const Real m = S.aug[c * area + p];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          if (j >= nj) break;
+          const int e = j * NC + c;
+          const uint32_t win = S.win[e];
           Real pred = (Real)0;
-          if (row >= r0 && row < r1 && cc >= c0 && cc < c1)
-            pred = gauss<Real>(cc, row, uw.x, uw.y, S.otf + 5 * e);
-          const Real d = S.aug[c * area + p] - pred;
+          if ((win >> pr) & (win >> (16 + pc)) & 1u) {
+            const double2 uw = S.uv[e];
+            pred = gauss<Real>(R.z + pc, R.x + pr, uw.x, uw.y, S.otf + 5 * e);
+          }
+          const Real d = m - pred;
           if (sizeof(Real) == 8) {
             S.dd[e * (area + 1) + p] = d * d;
           } else {
 #pragma unroll
             for (int q = 0; q < NA; ++q)
-              if (q == k) part[q] += d * d;
+              if (q == k) part[j][q] += d * d;
           }
         }
       }
-      if (sizeof(Real) == 4) {
+    }
+    if (sizeof(Real) == 4) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
 #pragma unroll
         for (int o = NA / 2; o > 0; o >>= 1)
 #pragma unroll
-          for (int k = 0; k < o; ++k) part[k] += part[k + o];
-        Real s = part[0];
-#pragma unroll
-        for (int o = LPO / 2; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        if (some) {
-          const double t = w * h == 64 ? (double)s * 0.015625 : (double)s / (double)(w * h);
-          if (j == 0)
-            cost[0] += t;
-          else if (j == 1)
-            cost[1] += t;
-          else
-            cost[2] += t;
-        }
-      }
+          for (int k = 0; k < o; ++k) part[j][k] += part[j][k + o];
+#pragma unroll 1
+      for (int j = 0; j < nj; ++j) add(j, j == 0 ? part[0][0] : j == 1 ? part[1][0] : part[2][0]);
     }
   }
   if (sizeof(Real) == 8) {
@@ -682,7 +709,7 @@ __global__ void __launch_bounds__(128, 4) shake_kernel(const __grid_constant__ S
       const double u = uvo[2 * g], w = uvo[2 * g + 1];
       R = roi_bound(m.n_row, m.n_col, u, w, v.r_px * v.ratio, v.r_px * v.ratio);
       const Rect pr = roi_bound(m.n_row, m.n_col, u, w, v.r_px, v.r_px);
-      win = span8(pr.rmin, pr.rmax, R.rmin) | (span8(pr.cmin, pr.cmax, R.cmin) << 8);
+      win = span16(pr.rmin, pr.rmax, R.rmin) | (span16(pr.cmin, pr.cmax, R.cmin) << 16);
       if (rect_empty(R)) R = Rect{1, 0, 1, 0};
     }
     S.roi[g] = make_int4(R.rmin, R.rmax, R.cmin, R.cmax);
@@ -704,7 +731,7 @@ __global__ void __launch_bounds__(128, 4) shake_kernel(const __grid_constant__ S
       Real q[5], a[64 / LPO], fy[64 / LPO];
 #pragma unroll
       for (int k = 0; k < 5; ++k) q[k] = q5[k];
-      const Real fx = axis_factor<Real>(sep, R.z + col, u, q[1], (win >> (8 + col)) & 1u);
+      const Real fx = axis_factor<Real>(sep, R.z + col, u, q[1], (win >> (16 + col)) & 1u);
       if (g < 8) S.ey[g] = axis_factor<Real>(sep, R.x + g, vv, q[2], (win >> g) & 1u);
 #pragma unroll
       for (int i = 0; i < 64 / LPO; ++i) {
@@ -1416,13 +1443,17 @@ static void launch_shake(int warps, cudaStream_t s, const ShakeView& v, int64_t 
       v, n, xyz, uv, otfp, score, delta, active, resid_out);
 }
 
-// Lanes per object.  FP32: 8 once a wave of one-object warps (148 SMs x 16) no longer holds
-// the objects, else 32 -- a lone object finishes sooner with more lanes.  Measured per launch
-// (4 pinhole cameras, 1024^2): 2,000 objects 77 us with 8 lanes, 75 us with 32; 3,000: 87 and
-// 120 us; 32,000: 428 and 992 us (one warp per object with everything on every lane: 128, 160
-// and 1,917 us).  FP64: 32 always; its squared differences take 3 x 8 B per ROI pixel, so
-// shared memory holds too few 8-lane groups (32,000 objects: 1,879 us with 8, 1,382 with 32).
+// Lanes per object.  FP32, ROIs of up to 64 pixels: 8 once a wave of one-object warps (148 SMs x
+// 16) no longer holds the objects, else 32 -- a lone object finishes sooner with more lanes.
+// Measured per launch (4 pinhole cameras): 2,000 objects 77 us with 8 lanes, 75 us with 32;
+// 3,500: 84 and 148 us; 20,000: 257 and 544 us.  Larger ROIs take their lanes through the pixels
+// either way, so 8 lanes pay from the third wave on, and only where four blocks (what the
+// registers allow) also find their ROIs' shared memory: 20,000 objects, ROIs of 100 pixels 759 and
+// 827 us, of 196 (three blocks) 1,277 and 1,097, of 256 on eight cameras (one block) 7,139 and
+// 1,989.  FP64: 32 always; its squared differences take 3 x 8 B per ROI pixel, so shared memory
+// holds too few 8-lane groups (32,000 objects: 1,879 us with 8, 1,382 with 32).
 constexpr int64_t kWaveObjects = 148 * 16;
+constexpr size_t kSmSmem = 228 * 1024;  // of an SM, 1 KB a block reserved
 
 template <typename Real, int NC>
 static void launch_shake_nc(int warps, cudaStream_t s, ShakeView& v, int64_t n, double* xyz,
@@ -1430,7 +1461,11 @@ static void launch_shake_nc(int warps, cudaStream_t s, ShakeView& v, int64_t n, 
                             const uint8_t* active, double* resid_out) {
   if constexpr (sizeof(Real) == 4) {
     shake_layout(v, 8, false);
-    if (n > kWaveObjects && v.cam_bytes + 4 * v.obj_stride <= kShakeSmemMax) {
+    const bool eight = v.roi_area <= 64
+                           ? n > kWaveObjects && v.cam_bytes + 4 * v.obj_stride <= kShakeSmemMax
+                           : n > 2 * kWaveObjects &&
+                                 4 * (v.cam_bytes + 16 * v.obj_stride + 1024) <= kSmSmem;
+    if (eight) {
       launch_shake<Real, NC, 8>(warps, s, v, n, xyz, uv, otfp, score, delta, active,
                                       resid_out);
       return;
