@@ -956,6 +956,8 @@ bool sort_candidates_device(PruneWork& W, const int* ids, const double* e, const
 // Steps 2-6 on the sorted candidates (W.ids_s, W.e_s).
 void prune_device(PruneWork& W, const PruneView& pv, int M, int n, int64_t total_points,
                   cudaStream_t s) {
+  require_scan(M);
+  if (M > 0) require_scan(total_points);
   W.counts.ensure(PC_N * sizeof(int), s);
   W.sel.ensure((size_t)M + 16, s);
   W.scnt.ensure((size_t)(M + 1) * sizeof(int), s);

@@ -81,7 +81,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(const int* in,
 
 }  // namespace
 
-void exclusive_scan(const int* in, int n, int* out, DevBuf& tmp, cudaStream_t s) {
+void exclusive_scan(const int* in, int n, int* out, DevBuf& tmp, cudaStream_t s, int most) {
+  if (n > most) require_scan(n);
   if (n <= 0) {
     OLPT_CUDA(cudaMemsetAsync(out, 0, sizeof(int), s));
     return;

@@ -1309,6 +1309,7 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
     v.cols[c] = std::max(1, cm.n_col / v.cell + (cm.n_col % v.cell ? 1 : 0));
     max_side = std::max(max_side, (float)(v.rows[c] + v.cols[c]) * v.cell);
     cells += (int64_t)v.rows[c] * v.cols[c];
+    if (v.active[c]) require_scan((int64_t)v.rows[c] * v.cols[c]);
   }
   OLPT_REQUIRE(total < (1ll << 30), OLPT_ERR_UNSUPPORTED, "stereo: too many detections");
   v.raw_off[n_cam] = (int)total;
@@ -1347,7 +1348,8 @@ void stereo_match_device(olpt_ctx* ctx, const SmParams& prm, StereoResult& res) 
   OLPT_CUDA(cudaMemsetAsync(W.cell_cnt.p, 0, (size_t)n_cells * sizeof(int), s));
   if (n > 0)
     bin_kernel<<<OLPT_G(nblk(n)), 256, 0, s>>>(v, n, W.cell_of.as<int>(), W.cell_cnt.as<int>());
-  exclusive_scan(W.cell_cnt.as<int>(), (int)n_cells, W.cell_start.as<int>(), W.scan_tmp, s);
+  exclusive_scan(W.cell_cnt.as<int>(), (int)n_cells, W.cell_start.as<int>(), W.scan_tmp, s,
+                 INT32_MAX);
   if (n > 0) {
     place_kernel<<<OLPT_G(nblk(n)), 256, 0, s>>>(v, n, W.cell_of.as<int>(), W.cell_cnt.as<int>(),
                                                  W.pid.as<int>(), W.xy.as<double2>(),
