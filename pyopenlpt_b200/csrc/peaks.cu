@@ -218,8 +218,10 @@ __device__ __forceinline__ int find_cam(const PeakArgs& a, int blk) {
 // wide row is a band of dozens of rounds, each a chain of its barriers: one where no spot is
 // found, two else (100 x 16,384 with 819 spots, EMIT: f64 73 -> 53 us, f32 48 -> 33 us against
 // three barriers and the fits repeated).
+// 16-bit levels: compiled for four blocks an SM (2048^2: 30.8 -> 27 to 29 us a call; 8 bits need
+// the registers, 512^2 18.6 -> 29 us); the others as the compiler chooses (0).
 template <typename T, bool EMIT, bool KEEP>
-__global__ void __launch_bounds__(kPeakThreads) peaks_kernel(const PeakArgs a) {
+__global__ void __launch_bounds__(kPeakThreads, sizeof(T) == 2 ? 4 : 0) peaks_kernel(const PeakArgs a) {
   constexpr int N = 16 / sizeof(T);
   const int cam = find_cam(a, blockIdx.x);
   const PeakCam& c = a.cam[cam];
