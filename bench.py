@@ -391,8 +391,8 @@ PHASE_NAMES = {5: "detection", 6: "stereo matching (all)", 7: "candidate sort + 
 # algorithmic bytes per object in FP32 (C x 64 ROI pixels x 4 B + 2 x (24 + C x 16 + 8) B
 # of state + C x 5 x 4 B of OTF).  dram__bytes_read.sum + dram__bytes_write.sum of four
 # shake_kernel launches over their objects.  4 cameras: 18,000 objects over 1280x800 images,
-# 9.1-9.8 MB each.  6 cameras: 120,000 objects over 2048^2 images, 156-235 MB each.
-SHAKE_TRAFFIC = {4: (527.0, 1_296.0), 6: (1_700.0, 1_912.0)}
+# 9.0-9.1 MB each.  6 cameras: 120,000 objects over 2048^2 images, 135-145 MB each.
+SHAKE_TRAFFIC = {4: (501.0, 1_296.0), 6: (1_174.0, 1_912.0)}
 
 
 def shake_traffic(args, prec, dom, bytes_per_launch, cams):

@@ -213,7 +213,7 @@ __device__ __forceinline__ int find_cam(const PeakArgs& a, int blk) {
 // memory (256 chunks at a time), fits them one per thread and stores coalesced.  Bands of 512
 // chunks: 2048^2 u16 makes 1,024 blocks where bands of 2,048 made 256, fewer than two a SM,
 // and the fits ran on the few lanes of a warp that held a detection, for each of the chunk's
-// pixels in turn (400,000 spots: 84 us a call before, 27 us with these bands).  KEEP, for
+// pixels in turn (400,000 spots: 84 us a call before, 25 us with these bands).  KEEP, for
 // floating-point levels: the fits that decided are listed too, not repeated (launch_peaks).  A
 // wide row is a band of dozens of rounds, each a chain of its barriers: one where no spot is
 // found, two else (100 x 16,384 with 819 spots, EMIT: f64 73 -> 53 us, f32 48 -> 33 us against

@@ -670,8 +670,8 @@ __device__ __forceinline__ double group_median(double x, bool has) {
 // evaluation per use (7.6 of 11.6 cycles between issues went to instruction fetch).  Here
 // four objects share the scalar code, the conversions run per ROI row and column, and one
 // copy of the evaluation serves every step, entered by the block's warps together.
-// 120,000 objects on six polynomial cameras: 2.3 ms a launch, 52% of the issue slots (9.0 ms
-// and 50% with one warp per object); every sum keeps its order, so results are unchanged.
+// 120,000 objects on six polynomial cameras: 1.9 ms a launch, 49 to 59% of the issue slots (9.0
+// ms and 50% with one warp per object); every sum keeps its order, so results are unchanged.
 // Four resident blocks an SM (128 registers a thread); built for five (102 registers), 8,000
 // objects take 126 us instead of 115, 32,000 of six cameras 767 instead of 694.
 template <typename Real, int NC, int LPO>

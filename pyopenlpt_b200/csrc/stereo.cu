@@ -1050,7 +1050,9 @@ __device__ __forceinline__ int next_camera(const SmView& v, const PathN<N>& ch) 
 // Expand one level, second half: one thread per (path, candidate) pair.  All 2D tests in FP64
 // for the pairs that FP32 could not decide, the quick triangulation gate (computeMinParallaxDeg,
 // calTriangulateTol, TriangulationCheckWithTol: StereoMatch.cpp:1072-1141), then the child path
-// (terminal, or with its next target camera).  Bound by the gathers of the lines of sight.
+// (terminal, or with its next target camera).  Bound by the gathers of the lines of sight and by
+// L1 (70% busy at K = 1): the exact branches take rays and paths by address, so these lie in
+// local memory, 336 to 624 B a thread.
 template <int K>
 __device__ __forceinline__ void tri_tile(const SmView& v, const void* in_v, const Pair* pairs,
                                          int n_pairs, int tile, void* out_v, int* out_count,
